@@ -7,6 +7,7 @@
 #include <cmath>
 #include <string>
 #include "mks_internal.cuh"
+#include "mks_fixed.cuh"
 
 namespace mks {
 
@@ -212,49 +213,57 @@ __global__ void k_links_soa_to_aos(const double2 *__restrict__ soa, double *__re
 #pragma unroll
   for (int k = 0; k < 9; k++) { double2 v = s[(size_t)k * Vh]; d[2 * k] = v.x; d[2 * k + 1] = v.y; }
 }
-__global__ void k_links_to_f32(const double2 *__restrict__ src, float4 *__restrict__ a, float2 *__restrict__ b, int Vh) {
+// out[0]: bits of the largest |component|; out[1]: non-zero when one is not finite
+__global__ void k_links_maxabs(const double2 *__restrict__ src, size_t n, unsigned long long *out) {
+  double m = 0;
+  bool bad = false;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    double2 v = src[i];
+    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+    bad = bad || !isfinite(v.x) || !isfinite(v.y);
+  }
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  bad = __any_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(out, (unsigned long long)__double_as_longlong(m));
+    if (bad) atomicMax(out + 1, 1ull);
+  }
+}
+// the FP32, FP16 and integer forms of a link field in one pass over its
+// FP64 entries (a pass each read them three times; HBM-bound: 144 B read and
+// 252 B written per link)
+__global__ void k_links_lowprec(const double2 *__restrict__ src, float4 *__restrict__ a32, float2 *__restrict__ b32,
+                                uint4 *__restrict__ a16, __half2 *__restrict__ b16, int4 *__restrict__ fx, float inv,
+                                int fx_exp, int Vh) {
   int h = blockIdx.x * blockDim.x + threadIdx.x;
   int pd = blockIdx.y;  // par*4+dir
   if (h >= Vh) return;
   const double2 *s = src + ((size_t)pd * 9) * Vh + h;
+  float2 f[9];
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    double2 u = s[(size_t)(2 * k) * Vh], v = s[(size_t)(2 * k + 1) * Vh];
-    a[((size_t)pd * 4 + k) * Vh + h] = make_float4((float)u.x, (float)u.y, (float)v.x, (float)v.y);
+  for (int k = 0; k < 9; k++) {
+    const double2 u = s[(size_t)k * Vh];
+    f[k] = make_float2((float)u.x, (float)u.y);
+    int4 w;
+    fx_split(fx_scale(u.x, fx_exp) + 8, w.x, w.y);  // + 8: rounds the cut at 16
+    fx_split(fx_scale(u.y, fx_exp) + 8, w.z, w.w);
+    fx[((size_t)pd * 9 + k) * Vh + h] = w;
   }
-  double2 w = s[(size_t)8 * Vh];
-  b[(size_t)pd * Vh + h] = make_float2((float)w.x, (float)w.y);
-}
-__global__ void k_links_maxabs(const double2 *__restrict__ src, size_t n, unsigned long long *out) {
-  double m = 0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double2 v = src[i];
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-  }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
-}
-__global__ void k_links_to_f16(const double2 *__restrict__ src, uint4 *__restrict__ a, __half2 *__restrict__ b,
-                               const unsigned long long *maxbits, int Vh) {
-  int h = blockIdx.x * blockDim.x + threadIdx.x;
-  int pd = blockIdx.y;
-  if (h >= Vh) return;
-  double mx = __longlong_as_double((long long)*maxbits);
-  float inv = mx > 0 ? (float)(1.0 / mx) : 0.f;
-  const double2 *s = src + ((size_t)pd * 9) * Vh + h;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    a32[((size_t)pd * 4 + k) * Vh + h] = make_float4(f[2 * k].x, f[2 * k].y, f[2 * k + 1].x, f[2 * k + 1].y);
+  b32[(size_t)pd * Vh + h] = f[8];
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     unsigned w[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      double2 u = s[(size_t)(4 * k + j) * Vh];
-      __half2 hv = __floats2half2_rn((float)u.x * inv, (float)u.y * inv);
+      __half2 hv = __floats2half2_rn(f[4 * k + j].x * inv, f[4 * k + j].y * inv);
       w[j] = *reinterpret_cast<unsigned *>(&hv);
     }
-    a[((size_t)pd * 2 + k) * Vh + h] = make_uint4(w[0], w[1], w[2], w[3]);
+    a16[((size_t)pd * 2 + k) * Vh + h] = make_uint4(w[0], w[1], w[2], w[3]);
   }
-  double2 u = s[(size_t)8 * Vh];
-  b[(size_t)pd * Vh + h] = __floats2half2_rn((float)u.x * inv, (float)u.y * inv);
+  b16[(size_t)pd * Vh + h] = __floats2half2_rn(f[8].x * inv, f[8].y * inv);
 }
 
 int vec_aos_to_soa64(const double *aos_dev, double2 *soa, int par) {
@@ -310,50 +319,54 @@ static void free_slot(LinkSlot &s) {
   dev_free(s.fat64); dev_free(s.lng64);
   dev_free(s.fat32a); dev_free(s.lng32a); dev_free(s.fat32b); dev_free(s.lng32b);
   dev_free(s.fat16a); dev_free(s.lng16a); dev_free(s.fat16b); dev_free(s.lng16b);
+  dev_free(s.fat_fx); dev_free(s.lng_fx);
   s = LinkSlot();
-}
-
-static int make_f16(const double2 *src, uint4 **a, __half2 **b, float *scale) {
-  Context &c = g_ctx;
-  int Vh = (int)c.Vh;
-  size_t n = (size_t)8 * 9 * Vh;
-  unsigned long long *mx;
-  MKS_TRY(dev_alloc((void **)&mx, sizeof(unsigned long long)));
-  MKS_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned long long), c.stream));
-  k_links_maxabs<<<c.sm_count * 4, 256, 0, c.stream>>>(src, n, mx);
-  k_links_to_f16<<<dim3(grid_for(Vh, 256), 8), 256, 0, c.stream>>>(src, *a, *b, mx, Vh);
-  c.launches += 2;
-  unsigned long long bits = 0;
-  MKS_CUDA(cudaMemcpyAsync(&bits, mx, sizeof bits, cudaMemcpyDeviceToHost, c.stream));
-  MKS_CUDA(cudaStreamSynchronize(c.stream));
-  dev_free(mx);
-  double m;
-  memcpy(&m, &bits, sizeof m);
-  *scale = (float)m;
-  MKS_CUDA(cudaGetLastError());
-  return MKS_OK;
 }
 
 int links_make_lowprec(LinkSlot &s) {
   Context &c = g_ctx;
   int Vh = (int)c.Vh;
-  size_t n32a = (size_t)8 * 4 * Vh, n32b = (size_t)8 * Vh;
-  if (!s.fat32a) {
-    MKS_TRY(dev_alloc((void **)&s.fat32a, n32a * sizeof(float4)));
-    MKS_TRY(dev_alloc((void **)&s.lng32a, n32a * sizeof(float4)));
-    MKS_TRY(dev_alloc((void **)&s.fat32b, n32b * sizeof(float2)));
-    MKS_TRY(dev_alloc((void **)&s.lng32b, n32b * sizeof(float2)));
-    MKS_TRY(dev_alloc((void **)&s.fat16a, (size_t)8 * 2 * Vh * sizeof(uint4)));
-    MKS_TRY(dev_alloc((void **)&s.lng16a, (size_t)8 * 2 * Vh * sizeof(uint4)));
-    MKS_TRY(dev_alloc((void **)&s.fat16b, n32b * sizeof(__half2)));
-    MKS_TRY(dev_alloc((void **)&s.lng16b, n32b * sizeof(__half2)));
+  size_t n32a = (size_t)8 * 4 * Vh, n32b = (size_t)8 * Vh, nfx = (size_t)8 * 9 * Vh;
+  auto need = [](auto *&q, size_t n) { return q ? (int)MKS_OK : dev_alloc((void **)&q, n * sizeof *q); };
+  MKS_TRY(need(s.fat32a, n32a));
+  MKS_TRY(need(s.lng32a, n32a));
+  MKS_TRY(need(s.fat32b, n32b));
+  MKS_TRY(need(s.lng32b, n32b));
+  MKS_TRY(need(s.fat16a, n32a / 2));
+  MKS_TRY(need(s.lng16a, n32a / 2));
+  MKS_TRY(need(s.fat16b, n32b));
+  MKS_TRY(need(s.lng16b, n32b));
+  MKS_TRY(need(s.fat_fx, nfx));
+  MKS_TRY(need(s.lng_fx, nfx));
+  // largest component of either field: the FP16 scales and the integers' exponent
+  unsigned long long *mx, bits[4];
+  MKS_TRY(dev_alloc((void **)&mx, sizeof bits));
+  MKS_CUDA(cudaMemsetAsync(mx, 0, sizeof bits, c.stream));
+  k_links_maxabs<<<c.sm_count * 4, 256, 0, c.stream>>>(s.fat64, nfx, mx);
+  k_links_maxabs<<<c.sm_count * 4, 256, 0, c.stream>>>(s.lng64, nfx, mx + 2);
+  MKS_CUDA(cudaMemcpyAsync(bits, mx, sizeof bits, cudaMemcpyDeviceToHost, c.stream));
+  MKS_CUDA(cudaStreamSynchronize(c.stream));
+  dev_free(mx);
+  double m[2];
+  memcpy(&m[0], &bits[0], 8);
+  memcpy(&m[1], &bits[2], 8);
+  s.fat16scale = (float)m[0];
+  s.lng16scale = (float)m[1];
+  s.fx_special = bits[1] || bits[3];
+  int ex = -1021;
+  if (!s.fx_special) {
+    const double top = m[0] > m[1] ? m[0] : m[1];
+    int k = 0;
+    frexp(top, &k);
+    if (top > 0 && k > ex) ex = k;
   }
-  k_links_to_f32<<<dim3(grid_for(Vh, 256), 8), 256, 0, c.stream>>>(s.fat64, s.fat32a, s.fat32b, Vh);
-  k_links_to_f32<<<dim3(grid_for(Vh, 256), 8), 256, 0, c.stream>>>(s.lng64, s.lng32a, s.lng32b, Vh);
-  c.launches += 2;
+  s.fx_exp = ex;
+  const float inv[2] = {m[0] > 0 ? (float)(1.0 / m[0]) : 0.f, m[1] > 0 ? (float)(1.0 / m[1]) : 0.f};
+  const dim3 grid(grid_for(Vh, 256), 8);
+  k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.fat64, s.fat32a, s.fat32b, s.fat16a, s.fat16b, s.fat_fx, inv[0], ex, Vh);
+  k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.lng64, s.lng32a, s.lng32b, s.lng16a, s.lng16b, s.lng_fx, inv[1], ex, Vh);
+  c.launches += 4;
   MKS_CUDA(cudaGetLastError());
-  MKS_TRY(make_f16(s.fat64, &s.fat16a, &s.fat16b, &s.fat16scale));
-  MKS_TRY(make_f16(s.lng64, &s.lng16a, &s.lng16b, &s.lng16scale));
   return MKS_OK;
 }
 

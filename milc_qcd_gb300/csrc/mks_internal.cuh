@@ -13,6 +13,7 @@
 //       FP32  float4  [4][Vh] (entries 0..7) + float2 [Vh] (entry 8)
 //       FP16  uint4   [2][Vh] (entries 0..7 as 16 halves) + __half2 [Vh],
 //             scaled by one global factor per link type
+//       FP64 D_eo: int4 [9][Vh], each entry's integer halves (mks_fixed.cuh)
 //     stored [parity][dir][...], so D_eo streams forward links at h and
 //     backward links of the other parity at the neighbour index: every link
 //     is read exactly once per application, without back-link copies.
@@ -357,6 +358,10 @@ struct LinkSlot {
   uint4 *fat16a = nullptr, *lng16a = nullptr;            // [2][4][2][Vh]
   __half2 *fat16b = nullptr, *lng16b = nullptr;          // [2][4][Vh]
   float fat16scale = 1.f, lng16scale = 1.f;
+  // the links as integers (mks_fixed.cuh), one exponent for fat and long;
+  // fx_special: one of them is not finite and D_eo works in plain FP64
+  int4 *fat_fx = nullptr, *lng_fx = nullptr;             // [2][4][9][Vh]
+  int fx_exp = 0, fx_special = 0;
 };
 
 struct Context {

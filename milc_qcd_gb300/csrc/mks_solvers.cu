@@ -22,6 +22,7 @@
 #include <vector>
 #include "mks_internal.cuh"
 #include "mks_dslash.cuh"
+#include "mks_dslash_fx.cuh"
 #include "mks_blas.cuh"
 
 namespace mks {
@@ -156,6 +157,32 @@ struct PtrSet64 { double2 *p[BLAS_MAXSRC]; };
 struct PtrSet32 { float2 *p[BLAS_MAXSRC]; };
 struct PtrSet16 { __half2 *p[BLAS_MAXSRC]; float *n[BLAS_MAXSRC]; };
 
+// a site's FP64 components stored as a block of integers (mks_fixed.cuh), the
+// form that the FP64 D_eo reads
+__device__ __forceinline__ void fx_put(const FxVec &d, int h, int Vh, const double (&v)[6]) {
+  s64 q[6];
+  int e;
+  fx_encode(v, q, e);
+  fx_store(d, h, Vh, q, e);
+}
+
+// FP64 SoA vectors as blocks
+struct OpToBlocks {
+  const double2 *v[BLAS_MAXSRC];
+  FxVec q[BLAS_MAXSRC];
+  int Vh;
+  __device__ void operator()(int h, int s, double *) const {
+    double w[6];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double2 a = v[s][(size_t)c * Vh + h];
+      w[2 * c] = a.x;
+      w[2 * c + 1] = a.y;
+    }
+    fx_put(q[s], h, Vh, w);
+  }
+};
+
 // |v|^2
 template <typename T2> struct OpNorm {
   T2 *v[2 * BLAS_MAXSRC];
@@ -178,13 +205,14 @@ template <typename T2> struct OpNorm {
 // source's x is known to be zero and D D x is not computed (ttt taken as 0).
 struct OpResid64 {
   double2 *ttt[BLAS_MAXSRC], *x[BLAS_MAXSRC], *src[BLAS_MAXSRC], *r[BLAS_MAXSRC], *p[BLAS_MAXSRC];
+  FxVec pq[BLAS_MAXSRC];  // p as blocks
   const CgState *st;
   double msq4[BLAS_MAXSRC];
   int map[BLAS_MAXSRC], tzero[BLAS_MAXSRC];
-  int Vh, setp;
+  int Vh, setp;           // setp: p <- r (FP64 solve)
   __device__ void operator()(int h, int s, double *out) const {
     if (st && st[map[s]].status != ST_HOST) { out[0] = 0; out[1] = 0; return; }
-    double a = 0, xx = 0;
+    double a = 0, xx = 0, pv[6];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       size_t i = (size_t)c * Vh + h;
@@ -192,9 +220,12 @@ struct OpResid64 {
       double2 rv = make_double2(sv.x + (t.x + (-msq4[s]) * xv.x), sv.y + (t.y + (-msq4[s]) * xv.y));
       r[s][i] = rv;
       if (setp) p[s][i] = rv;
+      pv[2 * c] = rv.x;
+      pv[2 * c + 1] = rv.y;
       a += rv.x * rv.x + rv.y * rv.y;
       xx += xv.x * xv.x + xv.y * xv.y;
     }
+    if (setp) fx_put(pq[s], h, Vh, pv);
     out[0] = a;
     out[1] = (xx == 0) ? 1.0 : a / xx;
   }
@@ -226,6 +257,7 @@ template <typename R> struct OpUpdate {
   T2 *x[BLAS_MAXSRC], *p[BLAS_MAXSRC], *r[BLAS_MAXSRC], *ttt[BLAS_MAXSRC];
   __half2 *p16[BLAS_MAXSRC];
   float *p16n[BLAS_MAXSRC];
+  FxVec pq[BLAS_MAXSRC];  // FP64: p as blocks
   const CgState *st;
   int Vh, relres;
   // split epilogue: ttt holds D D p only and the update forms
@@ -251,7 +283,10 @@ template <typename R> struct OpUpdate {
       x[s][i] = xv; r[s][i] = rv; p[s][i] = pv;
       pn.c[k] = {(R)pv.x, (R)pv.y};
     }
-    if (p16[s]) {
+    if constexpr (sizeof(R) == 8) {
+      const double w[6] = {pn.c[0].re, pn.c[0].im, pn.c[1].re, pn.c[1].im, pn.c[2].re, pn.c[2].im};
+      fx_put(pq[s], h, Vh, w);
+    } else if (p16[s]) {
       float m = 0.f;
 #pragma unroll
       for (int k = 0; k < 3; k++) m = fmaxf(m, fmaxf(fabsf((float)pn.c[k].re), fabsf((float)pn.c[k].im)));
@@ -383,11 +418,9 @@ static int launch_site(int family, const Op &op, const Fin &fin, const int *skip
 
 // ------------------------------------------------------------------
 // D_eo launchers
-struct LinkSet64 { LinkF64 fat, lng; };
 struct LinkSet32 { LinkF32 fat, lng; };
 struct LinkSet16 { LinkF16 fat, lng; };
 
-static LinkSet64 links64(const LinkSlot &s) { return {{s.fat64}, {s.lng64}}; }
 static LinkSet32 links32(const LinkSlot &s) { return {{s.fat32a, s.fat32b}, {s.lng32a, s.lng32b}}; }
 static LinkSet16 links16(const LinkSlot &s) {
   return {{s.fat16a, s.fat16b, s.fat16scale}, {s.lng16a, s.lng16b, s.lng16scale}};
@@ -478,7 +511,6 @@ static bool tma_tile(const Geom &g, int G, int *T, int *R) {
 }
 
 template <class LinkT> struct PrecOf;
-template <> struct PrecOf<LinkF64> { enum { v = MKS_PREC_DOUBLE }; typedef VecF64 In; typedef VecF64 Out; typedef double R; };
 template <> struct PrecOf<LinkF32> { enum { v = MKS_PREC_SINGLE }; typedef VecF32 In; typedef VecF32 Out; typedef float R; };
 template <> struct PrecOf<LinkF16> { enum { v = MKS_PREC_HALF }; typedef VecF16 In; typedef VecF32 Out; typedef float R; };
 
@@ -724,7 +756,6 @@ static bool ms_shift64(double resid, bool batched) {
   return v < 0 ? (!batched && resid < 1e-7) : v != 0;
 }
 
-static void set_vec(VecF64 &v, float *p, float *) { v.p = (double2 *)p; }
 static void set_vec(VecF32 &v, float *p, float *) { v.p = (float2 *)p; }
 static void set_vec(VecF16 &v, float *p, float *n) { v.p = (__half2 *)p; v.norm = n; }
 
@@ -913,19 +944,91 @@ static int launch_dslash(int family, const LinkT &fat, const LinkT &lng,
     }
     sh = t;
   }
-  if (a.nsrc > 1 && family != MKS_K_DSLASH_F64) family = MKS_K_DSLASH_MRHS;
+  if (a.nsrc > 1) family = MKS_K_DSLASH_MRHS;
   return launch_shape<R, LinkT, InT, OutT, EPI, NSUM, Fin>(family, fat, lng, a, fin, sh);
 }
 
-// plain D on FP64 SoA fields, nsrc sources
-static int dslash64(const LinkSlot &sl, int out_par, int nsrc, double2 *const *in, double2 *const *out,
-                    const int *skip = nullptr) {
-  DslashArgs<VecF64, VecF64, VecF64> a;
+// ------------------------------------------------------------------
+// FP64 D_eo (mks_dslash_fx.cuh)
+
+// Four threads per site (one direction each) while one would leave the SMs
+// with under FX_SPLIT_THREADS threads each: the chain of 16 terms is then
+// the launch's time.
+constexpr int FX_SPLIT_THREADS = 512;
+
+// mult: how many sets of 32 / SPLIT sites a block takes (G warps each)
+template <int SPLIT, int NB, int OUT, int EPI, class Fin>
+static int launch_fx_as(FxArgs &a, const Fin &fin, int mult, int rows) {
+  Context &c = ctx();
+  a.G = (a.nsrc + NB - 1) / NB;
+  const int block = 32 * a.G * mult, grid = grid_for(c.Vh, 32 / SPLIT * mult);
+  if (EPI == EPI_AXPY) {
+    MKS_TRY(ensure_red(3 * a.G * NB, grid));
+    a.red = c.red;
+  }
+  (EPI == EPI_AXPY ? g_shape_epi : g_shape)[MKS_PREC_DOUBLE][a.nsrc] = {a.G * SPLIT, NB, block, 0, 0, 0, 0};
+  timing_begin(MKS_K_DSLASH_F64);
+  k_dslash_fx<SPLIT, NB, OUT, EPI, Fin><<<dim3(grid, rows), block, 0, c.stream>>>(a, fin);
+  timing_end(MKS_K_DSLASH_F64);
+  MKS_CUDA(cudaGetLastError());
+  return MKS_OK;
+}
+
+// rows = 2: both parities of one source in one launch (in[y], out[y] of
+// output parity y).  One source per thread up to 8 (blocks of one warp per
+// source share their sites' links in L1), two beyond.
+template <int OUT, int EPI, class Fin>
+static int launch_fx(const LinkSlot &sl, FxArgs &a, const Fin &fin, int rows = 1) {
+  Context &c = ctx();
+  a.g = c.geom;
+  a.fat = {sl.fat_fx};
+  a.lng = {sl.lng_fx};
+  a.fat64 = sl.fat64;
+  a.lng64 = sl.lng64;
+  a.EL = sl.fx_exp;
+  a.special = sl.fx_special;
+  const int mult = a.nsrc == 1 ? 4 : a.nsrc == 2 ? 2 : 1;
+  if (a.nsrc <= 8 && c.Vh * a.nsrc * rows < (size_t)c.sm_count * FX_SPLIT_THREADS)
+    return launch_fx_as<4, 1, OUT, EPI>(a, fin, mult > 2 ? 2 : mult, rows);
+  if constexpr (OUT != FX_OUT_AOS) {
+    if (a.nsrc > 8) return launch_fx_as<1, 2, OUT, EPI>(a, fin, 1, rows);
+  }
+  return launch_fx_as<1, 1, OUT, EPI>(a, fin, mult, rows);
+}
+
+// D on blocks: outq (blocks) or out (FP64 SoA)
+static int dslash_blocks(const LinkSlot &sl, int out_par, int nsrc, const FxVec *in, const FxVec *outq,
+                         double2 *const *out, int rev, const int *skip = nullptr) {
+  FxArgs a;
   memset(&a, 0, sizeof a);
-  a.out_par = out_par; a.nsrc = nsrc; a.skip = skip;
-  for (int s = 0; s < nsrc; s++) { a.in[s].p = in[s]; a.out[s].p = out[s]; }
-  LinkSet64 L = links64(sl);
-  return launch_dslash<double, LinkF64, VecF64, VecF64, EPI_PLAIN, 0>(MKS_K_DSLASH_F64, L.fat, L.lng, a, FinNone());
+  a.out_par = out_par; a.nsrc = nsrc; a.rev = rev; a.skip = skip;
+  for (int s = 0; s < nsrc; s++) {
+    a.in[s] = in[s];
+    if (outq) a.outq[s] = outq[s];
+    else a.out[s] = out[s];
+  }
+  return outq ? launch_fx<FX_OUT_BLOCK, EPI_PLAIN>(sl, a, FinNone()) : launch_fx<FX_OUT_F64, EPI_PLAIN>(sl, a, FinNone());
+}
+
+static int to_blocks(int nsrc, const double2 *const *v, const FxVec *q) {
+  OpToBlocks op;
+  memset(&op, 0, sizeof op);
+  for (int s = 0; s < nsrc; s++) { op.v[s] = v[s]; op.q[s] = q[s]; }
+  op.Vh = (int)ctx().Vh;
+  return launch_site<OpToBlocks, 0, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, nsrc);
+}
+
+static int ws_blocks(const std::string &name, FxVec *v) {
+  MKS_TRY(wsv(name + "_q", 3 * ctx().Vh, &v->q));
+  return wsv(name + "_e", ctx().Vh, &v->e);
+}
+
+// plain D on FP64 SoA fields, nsrc sources
+static int dslash64(const LinkSlot &sl, int out_par, int nsrc, double2 *const *in, double2 *const *out) {
+  FxVec q[MAXSRC];
+  for (int s = 0; s < nsrc; s++) MKS_TRY(ws_blocks("fx_in" + std::to_string(s), &q[s]));
+  MKS_TRY(to_blocks(nsrc, in, q));
+  return dslash_blocks(sl, out_par, nsrc, q, nullptr, out, 1);
 }
 
 // ------------------------------------------------------------------
@@ -948,26 +1051,45 @@ static int slot_ok(int slot) {
 
 // ------------------------------------------------------------------
 // public D
+
+// MILC AoS field (rows: one parity, or both from par0 on) to blocks
+__global__ void __launch_bounds__(128) k_aos_to_blocks(const double *__restrict__ aos, FxVec q0, FxVec q1, int par0, int Vh) {
+  const int h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= Vh) return;
+  const int par = par0 ^ (int)blockIdx.y;
+  const double *b = aos + ((size_t)par * Vh + h) * 6;
+  double v[6];
+#pragma unroll
+  for (int k = 0; k < 6; k++) v[k] = b[k];
+  fx_put(blockIdx.y ? q1 : q0, h, Vh, v);
+}
+static int aos_to_blocks(const double *aos, FxVec q0, FxVec q1, int par0, int rows) {
+  Context &c = ctx();
+  const int block = c.Vh < (size_t)c.sm_count * 128 ? 32 : 128;
+  k_aos_to_blocks<<<dim3(grid_for(c.Vh, block), rows), block, 0, c.stream>>>(aos, q0, q1, par0, (int)c.Vh);
+  c.launches++;
+  MKS_CUDA(cudaGetLastError());
+  return MKS_OK;
+}
+
+// MILC field -> blocks of the parities that D reads -> D straight into the
+// caller's field: two launches for any parity.
 static int dslash_dev_impl(const double *src_dev, double *dst_dev, int parity, int slot) {
   Context &c = ctx();
-  double2 *in, *out;
-  MKS_TRY(wsv("ds_in", 6 * c.Vh, &in));
-  MKS_TRY(wsv("ds_out", 6 * c.Vh, &out));
-  const LinkSlot &sl = c.slots[slot];
-  for (int op = 0; op < 2; op++) {
-    int out_par = op;
-    bool want = (parity == MKS_EVENANDODD) || (parity == MKS_EVEN && op == 0) || (parity == MKS_ODD && op == 1);
-    if (!want) continue;
-    MKS_TRY(vec_aos_to_soa64(src_dev, par64(in, 1 - out_par), 1 - out_par));
+  FxVec in[2];
+  for (int k = 0; k < 2; k++) MKS_TRY(ws_blocks("ds_in" + std::to_string(k), &in[k]));
+  FxArgs a;
+  memset(&a, 0, sizeof a);
+  a.nsrc = 1;
+  a.out_par = parity == MKS_ODD ? 1 : 0;
+  const int rows = parity == MKS_EVENANDODD ? 2 : 1;
+  for (int y = 0; y < rows; y++) {
+    const int op = a.out_par + y;
+    a.in[y] = in[1 - op];
+    a.out[y] = (double2 *)dst_dev;
   }
-  for (int op = 0; op < 2; op++) {
-    bool want = (parity == MKS_EVENANDODD) || (parity == MKS_EVEN && op == 0) || (parity == MKS_ODD && op == 1);
-    if (!want) continue;
-    double2 *pin = par64(in, 1 - op), *pout = par64(out, op);
-    MKS_TRY(dslash64(sl, op, 1, &pin, &pout));
-    MKS_TRY(vec_soa64_to_aos(pout, dst_dev, op));
-  }
-  return MKS_OK;
+  MKS_TRY(aos_to_blocks(src_dev, in[1 - a.out_par], in[a.out_par], 1 - a.out_par, rows));
+  return launch_fx<FX_OUT_AOS, EPI_PLAIN>(c.slots[slot], a, FinNone(), rows);
 }
 
 }  // namespace mks
@@ -1006,7 +1128,8 @@ namespace mks {
 // block CG driver (nsrc = 1 is the single-source solver)
 struct CgFields {
   // FP64, one parity [3][Vh] per source
-  double2 *src[MAXSRC], *x[MAXSRC], *r[MAXSRC], *p[MAXSRC], *ttt[MAXSRC], *t[MAXSRC];  // t: other parity
+  double2 *src[MAXSRC], *x[MAXSRC], *r[MAXSRC], *p[MAXSRC], *ttt[MAXSRC];
+  FxVec pq[MAXSRC], tq[MAXSRC];  // D input (p, or x for a residual) and D of it (other parity), as blocks
   // sloppy
   float2 *x32[MAXSRC], *r32[MAXSRC], *p32[MAXSRC], *ttt32[MAXSRC], *t32[MAXSRC];
   __half2 *p16[MAXSRC], *t16[MAXSRC];
@@ -1023,7 +1146,8 @@ static int alloc_cg_fields(CgFields &f, int nsrc, int prec) {
     MKS_TRY(wsv("cg_r" + k, n, &f.r[s]));
     MKS_TRY(wsv("cg_p" + k, n, &f.p[s]));
     MKS_TRY(wsv("cg_ttt" + k, n, &f.ttt[s]));
-    MKS_TRY(wsv("cg_t" + k, n, &f.t[s]));
+    MKS_TRY(ws_blocks("cg_p" + k, &f.pq[s]));
+    MKS_TRY(ws_blocks("cg_t" + k, &f.tq[s]));
     if (prec != MKS_PREC_DOUBLE) {
       MKS_TRY(wsv("cg_x32" + k, n, &f.x32[s]));
       MKS_TRY(wsv("cg_r32" + k, n, &f.r32[s]));
@@ -1060,12 +1184,12 @@ int dslash32_multi(int slot, int out_par, int nsrc, float2 *const *in, float2 *c
   return MKS_OK;
 }
 
-// ttt <- D_par D_opar x  (FP64) for the sources listed
-static int apply_DD64(const LinkSlot &sl, int par, int nsrc, double2 *const *x, double2 *const *t,
+// ttt <- D_par D_opar x  (FP64) for the sources listed; xq, tq scratch
+static int apply_DD64(const LinkSlot &sl, int par, int nsrc, double2 *const *x, const FxVec *xq, const FxVec *tq,
                       double2 *const *ttt) {
-  MKS_TRY(dslash64(sl, 1 - par, nsrc, x, t));
-  MKS_TRY(dslash64(sl, par, nsrc, t, ttt));
-  return MKS_OK;
+  MKS_TRY(to_blocks(nsrc, x, xq));
+  MKS_TRY(dslash_blocks(sl, 1 - par, nsrc, xq, tq, nullptr, 1));
+  return dslash_blocks(sl, par, nsrc, tq, nullptr, ttt, 0);
 }
 
 static int read_states(Solver &S, int nsrc, CgState *h) {
@@ -1085,25 +1209,18 @@ static int write_states(Solver &S, int nsrc, const CgState *h, int skip) {
 // one sloppy or FP64 CG iteration for all running sources (3 launches)
 static int cg_iteration(const LinkSlot &sl, int par, int nsrc, int prec, const double *msq4, CgFields &f, Solver &S) {
   if (prec == MKS_PREC_DOUBLE) {
-    DslashArgs<VecF64, VecF64, VecF64> a1;
-    memset(&a1, 0, sizeof a1);
-    a1.out_par = 1 - par; a1.nsrc = nsrc; a1.skip = S.skip;
-    for (int s = 0; s < nsrc; s++) { a1.in[s].p = f.p[s]; a1.out[s].p = f.t[s]; }
-    LinkSet64 L = links64(sl);
-    MKS_TRY((launch_dslash<double, LinkF64, VecF64, VecF64, EPI_PLAIN, 0>(MKS_K_DSLASH_F64, L.fat, L.lng, a1, FinNone())));
-    DslashArgs<VecF64, VecF64, VecF64> a2;
-    memset(&a2, 0, sizeof a2);
-    a2.out_par = par; a2.nsrc = nsrc; a2.skip = S.skip;
+    MKS_TRY(dslash_blocks(sl, 1 - par, nsrc, f.pq, f.tq, nullptr, 1, S.skip));
+    FxArgs a;
+    memset(&a, 0, sizeof a);
+    a.out_par = par; a.nsrc = nsrc; a.skip = S.skip;
     for (int s = 0; s < nsrc; s++) {
-      a2.in[s].p = f.t[s]; a2.out[s].p = f.ttt[s]; a2.p[s].p = f.p[s]; a2.r[s].p = f.r[s]; a2.coef[s] = -msq4[s];
+      a.in[s] = f.tq[s]; a.out[s] = f.ttt[s]; a.p[s] = f.p[s]; a.r[s] = f.r[s]; a.coef[s] = -msq4[s];
     }
-    double *tot;
-    MKS_TRY(wsv("cg_tot", 3 * MAXSRC, &tot));
-    a2.totals = tot;
-    MKS_TRY((launch_dslash<double, LinkF64, VecF64, VecF64, EPI_AXPY, 3>(MKS_K_DSLASH_F64, L.fat, L.lng, a2, FinCgAlpha{S.st})));
+    MKS_TRY(wsv("cg_tot", 3 * MAXSRC, &a.totals));
+    MKS_TRY((launch_fx<FX_OUT_F64, EPI_AXPY>(sl, a, FinCgAlpha{S.st})));
     OpUpdate<double> up;
     memset(&up, 0, sizeof up);
-    for (int s = 0; s < nsrc; s++) { up.x[s] = f.x[s]; up.p[s] = f.p[s]; up.r[s] = f.r[s]; up.ttt[s] = f.ttt[s]; }
+    for (int s = 0; s < nsrc; s++) { up.x[s] = f.x[s]; up.p[s] = f.p[s]; up.r[s] = f.r[s]; up.ttt[s] = f.ttt[s]; up.pq[s] = f.pq[s]; }
     up.st = S.st; up.Vh = (int)ctx().Vh; up.relres = 0;
     MKS_TRY((launch_site<OpUpdate<double>, 1, FinCgUpdate>(MKS_K_BLAS, up, FinCgUpdate{S.st, S.skip}, S.skip, nsrc)));
     return MKS_OK;
@@ -1294,10 +1411,12 @@ static int run_batch(const LinkSlot &sl, int par, int nsrc, int prec, const doub
   key_push(key, sl.fat64); key_push(key, sl.lng64); key_push(key, sl.fat32a); key_push(key, sl.lng32a);
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
+  key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fx_exp); key_push(key, sl.fx_special);
   key_push(key, S.st); key_push(key, S.skip); key_push(key, c.red.partials); key_push(key, c.red.count);
   for (int s = 0; s < nsrc; s++) {
     key_push(key, msq4[s]);
-    key_push(key, f.x[s]); key_push(key, f.p[s]); key_push(key, f.r[s]); key_push(key, f.ttt[s]); key_push(key, f.t[s]);
+    key_push(key, f.x[s]); key_push(key, f.p[s]); key_push(key, f.r[s]); key_push(key, f.ttt[s]);
+    key_push(key, f.pq[s].q); key_push(key, f.pq[s].e); key_push(key, f.tq[s].q); key_push(key, f.tq[s].e);
     key_push(key, f.x32[s]); key_push(key, f.p32[s]); key_push(key, f.r32[s]); key_push(key, f.ttt32[s]);
     key_push(key, f.t32[s]); key_push(key, f.p16[s]); key_push(key, f.t16[s]); key_push(key, f.p16n[s]);
     key_push(key, f.t16n[s]);
@@ -1310,21 +1429,22 @@ static int run_batch(const LinkSlot &sl, int par, int nsrc, int prec, const doub
 static int true_residual(const LinkSlot &sl, int par, int nsrc, const double *msq4, CgFields &f, Solver &S, int setp,
                          const std::vector<int> &need, const std::vector<int> &xzero, std::vector<double> *relrsq) {
   int idx[MAXSRC], nd = 0, ndd = 0;
-  double2 *xs[MAXSRC], *ts[MAXSRC], *tts[MAXSRC];
+  double2 *xs[MAXSRC], *tts[MAXSRC];
+  FxVec xq[MAXSRC], tq[MAXSRC];
   for (int s = 0; s < nsrc; s++) {
     if (!need[s]) continue;
     idx[nd++] = s;
-    if (!xzero[s]) { xs[ndd] = f.x[s]; ts[ndd] = f.t[s]; tts[ndd] = f.ttt[s]; ndd++; }
+    if (!xzero[s]) { xs[ndd] = f.x[s]; xq[ndd] = f.pq[s]; tq[ndd] = f.tq[s]; tts[ndd] = f.ttt[s]; ndd++; }
   }
   if (nd == 0) return MKS_OK;
-  if (ndd > 0) MKS_TRY(apply_DD64(sl, par, ndd, xs, ts, tts));
+  if (ndd > 0) MKS_TRY(apply_DD64(sl, par, ndd, xs, xq, tq, tts));
   OpResid64 op;
   memset(&op, 0, sizeof op);
   FinResid fin;
   memset(&fin, 0, sizeof fin);
   for (int k = 0; k < nd; k++) {
     int s = idx[k];
-    op.ttt[k] = f.ttt[s]; op.x[k] = f.x[s]; op.src[k] = f.src[s]; op.r[k] = f.r[s]; op.p[k] = f.p[s];
+    op.ttt[k] = f.ttt[s]; op.x[k] = f.x[s]; op.src[k] = f.src[s]; op.r[k] = f.r[s]; op.p[k] = f.p[s]; op.pq[k] = f.pq[s];
     op.msq4[k] = msq4[s]; op.map[k] = s; op.tzero[k] = xzero[s];
     fin.map[k] = s;
   }
@@ -1444,7 +1564,8 @@ static int block_cg_shifted(int slot, int par, int nsrc, const double *msq4, con
     memset(&g, 0, sizeof g);
     for (int k = 0; k < (int)act.size(); k++) {
       const int s = act[k];
-      g.src[k] = f.src[s]; g.x[k] = f.x[s]; g.r[k] = f.r[s]; g.p[k] = f.p[s]; g.ttt[k] = f.ttt[s]; g.t[k] = f.t[s];
+      g.src[k] = f.src[s]; g.x[k] = f.x[s]; g.r[k] = f.r[s]; g.p[k] = f.p[s]; g.ttt[k] = f.ttt[s];
+      g.pq[k] = f.pq[s]; g.tq[k] = f.tq[s];
       g.x32[k] = f.x32[s]; g.r32[k] = f.r32[s]; g.p32[k] = f.p32[s]; g.ttt32[k] = f.ttt32[s]; g.t32[k] = f.t32[s];
       g.p16[k] = f.p16[s]; g.t16[k] = f.t16[s]; g.p16n[k] = f.p16n[s]; g.t16n[k] = f.t16n[s];
       sig[k] = msq4[s];
@@ -1498,7 +1619,7 @@ static int block_cg_shifted(int slot, int par, int nsrc, const double *msq4, con
       std::vector<double> relrsq;
       std::vector<int> need(nact);
       for (int k = 0; k < nact; k++) need[k] = hs[k].status == ST_HOST;
-      MKS_TRY(true_residual(sl, par, nact, sig, g, S, mixed ? (first ? 1 : 0) : 1, need,
+      MKS_TRY(true_residual(sl, par, nact, sig, g, S, mixed ? 0 : 1, need,
                             first ? xzero : std::vector<int>(nact, 0), arg->relresid > 0 ? &relrsq : nullptr));
       if (mixed) {
         OpDemote dm;
@@ -2093,7 +2214,8 @@ template <typename R, typename RS = R>
 __device__ __forceinline__ void ms_site_update(const MsState &m, typename VT<RS>::v2 *const *psim,
                                                typename VT<RS>::v2 *const *pm, typename VT<R>::v2 *r,
                                                const typename VT<R>::v2 *ttt, typename VT<R>::v2 *cgp,
-                                               __half2 *p16, float *p16n, int h, int Vh, double *out) {
+                                               const FxVec &cgq, __half2 *p16, float *p16n, int h, int Vh,
+                                               double *out) {
     typedef typename VT<R>::v2 T2;
     typedef typename VT<RS>::v2 S2;
     const int n = m.num_now, jl = m.j_low;
@@ -2112,6 +2234,7 @@ __device__ __forceinline__ void ms_site_update(const MsState &m, typename VT<RS>
     for (int j = 0; j < n; j++) {
       if (m.retired[j]) continue;
       const RS bj = (RS)m.beta_i[j], zj = (RS)m.zeta_ip1[j], aj = (RS)m.alpha[j];
+      double w[6];
 #pragma unroll
       for (int k = 0; k < 3; k++) {
         size_t i = (size_t)k * Vh + h;
@@ -2121,8 +2244,10 @@ __device__ __forceinline__ void ms_site_update(const MsState &m, typename VT<RS>
         psim[j][i] = xv;
         pm[j][i] = pv;
         if (j == jl) { T2 cv; cv.x = (R)pv.x; cv.y = (R)pv.y; cgp[i] = cv; }
+        if (sizeof(R) == 8) { w[2 * k] = pv.x; w[2 * k + 1] = pv.y; }
       }
-      if (j == jl && p16) {
+      if (sizeof(R) == 8 && j == jl) fx_put(cgq, h, Vh, w);
+      if (sizeof(R) == 4 && j == jl && p16) {
         float mx = 0.f;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -2146,12 +2271,13 @@ template <typename R, typename RS = R> struct OpShiftUpdate {
   typedef typename VT<RS>::v2 S2;
   S2 *psim[MAXSH], *pm[MAXSH];
   T2 *r, *ttt, *cgp;
+  FxVec cgq;  // FP64: cgp as blocks
   __half2 *p16;
   float *p16n;
   const MsState *st;
   int Vh;
   __device__ void operator()(int h, int, double *out) const {
-    ms_site_update<R, RS>(*st, psim, pm, r, ttt, cgp, p16, p16n, h, Vh, out);
+    ms_site_update<R, RS>(*st, psim, pm, r, ttt, cgp, cgq, p16, p16n, h, Vh, out);
   }
 };
 
@@ -2166,7 +2292,7 @@ template <typename R, typename RS = R> struct OpShiftUpdateM {
   int Vh;
   __device__ void operator()(int h, int k, double *out) const {
     const int f = map[k];
-    ms_site_update<R, RS>(st[f], psim[f], pm[f], r[f], ttt[f], cgp[f], nullptr, nullptr, h, Vh, out);
+    ms_site_update<R, RS>(st[f], psim[f], pm[f], r[f], ttt[f], cgp[f], FxVec{nullptr, nullptr}, nullptr, nullptr, h, Vh, out);
   }
 };
 
@@ -2176,6 +2302,7 @@ template <typename R, typename RS = R> struct OpShiftInit {
   typedef typename VT<RS>::v2 S2;
   S2 *psim[MAXSH], *pm[MAXSH];
   T2 *r, *cgp;
+  FxVec cgq;  // FP64: cgp as blocks
   const double2 *src;
   __half2 *p16;
   float *p16n;
@@ -2184,10 +2311,13 @@ template <typename R, typename RS = R> struct OpShiftInit {
     double a = 0;
     float mx = 0.f;
     T2 v[3];
+    double w[6];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       size_t i = (size_t)k * Vh + h;
       double2 sv = src[i];
+      w[2 * k] = sv.x;
+      w[2 * k + 1] = sv.y;
       v[k].x = (R)sv.x; v[k].y = (R)sv.y;
       r[i] = v[k]; cgp[i] = v[k];
       a += sv.x * sv.x + sv.y * sv.y;
@@ -2199,6 +2329,7 @@ template <typename R, typename RS = R> struct OpShiftInit {
         psim[j][i] = z;
       }
     }
+    if (sizeof(R) == 8) fx_put(cgq, h, Vh, w);
     if (p16) {
       float inv = mx > 0.f ? 1.f / mx : 0.f;
       p16n[h] = mx;
@@ -2283,14 +2414,20 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
   Context &c = ctx();
   const int Vh = (int)c.Vh;
   size_t n = 3 * c.Vh;
-  T2 *r, *cgp, *ttt, *t;
+  T2 *r, *cgp, *ttt, *t = nullptr;
+  FxVec cgq = {nullptr, nullptr}, tq = {nullptr, nullptr};
   S2 *pm[MAXSH], *psim[MAXSH];
   const char *tag = sizeof(R) == 8 ? "64" : "32";
   const char *stag = sizeof(RS) == 8 ? "64" : "32";
   MKS_TRY(wsv(std::string("ms_r") + tag, n, &r));
   MKS_TRY(wsv(std::string("ms_p") + tag, n, &cgp));
   MKS_TRY(wsv(std::string("ms_ttt") + tag, n, &ttt));
-  MKS_TRY(wsv(std::string("ms_t") + tag, n, &t));
+  if (sizeof(R) == 8) {
+    MKS_TRY(ws_blocks("ms_p", &cgq));
+    MKS_TRY(ws_blocks("ms_t", &tq));
+  } else {
+    MKS_TRY(wsv(std::string("ms_t") + tag, n, &t));
+  }
   for (int j = 0; j < nsh; j++) {
     MKS_TRY(wsv(std::string("ms_pm") + stag + "_" + std::to_string(j), n, &pm[j]));
     if (wide && x64) psim[j] = (S2 *)x64[j];
@@ -2325,7 +2462,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
     OpShiftInit<R, RS> op;
     memset(&op, 0, sizeof op);
     for (int j = 0; j < nsh; j++) { op.psim[j] = psim[j]; op.pm[j] = pm[j]; }
-    op.r = r; op.cgp = cgp; op.src = src64; op.p16 = p16; op.p16n = p16n; op.Vh = Vh; op.n = nsh;
+    op.r = r; op.cgp = cgp; op.cgq = cgq; op.src = src64; op.p16 = p16; op.p16n = p16n; op.Vh = Vh; op.n = nsh;
     double *tot;
     MKS_TRY(wsv("ms_tot", 4, &tot));
     MKS_TRY((launch_site<OpShiftInit<R, RS>, 1, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, 1, tot)));
@@ -2357,18 +2494,13 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
   auto issue = [&]() -> int {
     for (int k = 0; k < np; k++) {
       if (prec == MKS_PREC_DOUBLE) {
-        LinkSet64 L = links64(sl);
-        DslashArgs<VecF64, VecF64, VecF64> a1;
-        memset(&a1, 0, sizeof a1);
-        a1.out_par = 1 - par; a1.nsrc = 1; a1.skip = skip;
-        a1.in[0].p = (double2 *)cgp; a1.out[0].p = (double2 *)t;
-        MKS_TRY((launch_dslash<double, LinkF64, VecF64, VecF64, EPI_PLAIN, 0>(MKS_K_DSLASH_F64, L.fat, L.lng, a1, FinNone())));
-        DslashArgs<VecF64, VecF64, VecF64> a2;
-        memset(&a2, 0, sizeof a2);
-        a2.out_par = par; a2.nsrc = 1; a2.skip = skip; a2.totals = tot;
-        a2.in[0].p = (double2 *)t; a2.out[0].p = (double2 *)ttt; a2.p[0].p = (double2 *)cgp; a2.r[0].p = (double2 *)r;
-        a2.coef[0] = h.shift0;
-        MKS_TRY((launch_dslash<double, LinkF64, VecF64, VecF64, EPI_AXPY, 3>(MKS_K_DSLASH_F64, L.fat, L.lng, a2, FinMsAlpha{st})));
+        MKS_TRY(dslash_blocks(sl, 1 - par, 1, &cgq, &tq, nullptr, 1, skip));
+        FxArgs a;
+        memset(&a, 0, sizeof a);
+        a.out_par = par; a.nsrc = 1; a.skip = skip; a.totals = tot;
+        a.in[0] = tq; a.out[0] = (double2 *)ttt; a.p[0] = (double2 *)cgp; a.r[0] = (double2 *)r;
+        a.coef[0] = h.shift0;
+        MKS_TRY((launch_fx<FX_OUT_F64, EPI_AXPY>(sl, a, FinMsAlpha{st})));
       } else if (prec == MKS_PREC_SINGLE) {
         LinkSet32 L = links32(sl);
         DslashArgs<VecF32, VecF32, VecF32> a1;
@@ -2399,7 +2531,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
       OpShiftUpdate<R, RS> up;
       memset(&up, 0, sizeof up);
       for (int j = 0; j < nsh; j++) { up.psim[j] = psim[j]; up.pm[j] = pm[j]; }
-      up.r = r; up.ttt = ttt; up.cgp = cgp; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh;
+      up.r = r; up.ttt = ttt; up.cgp = cgp; up.cgq = cgq; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh;
       MKS_TRY((launch_site<OpShiftUpdate<R, RS>, 1, FinMsUpdate>(MKS_K_SHIFT, up, FinMsUpdate{st, skip}, skip, 1)));
     }
     return MKS_OK;
@@ -2411,9 +2543,11 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
   key_push(key, sl.fat64); key_push(key, sl.lng64); key_push(key, sl.fat32a); key_push(key, sl.lng32a);
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
+  key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fx_exp); key_push(key, sl.fx_special);
   key_push(key, st); key_push(key, skip); key_push(key, tot); key_push(key, c.red.partials); key_push(key, c.red.count);
   key_push(key, h.shift0); key_push(key, nsh); key_push(key, r); key_push(key, cgp); key_push(key, ttt);
-  key_push(key, t); key_push(key, p16); key_push(key, t16); key_push(key, p16n); key_push(key, t16n);
+  key_push(key, t); key_push(key, cgq.q); key_push(key, cgq.e); key_push(key, tq.q); key_push(key, tq.e);
+  key_push(key, p16); key_push(key, t16); key_push(key, p16n); key_push(key, t16n);
   for (int j = 0; j < nsh; j++) { key_push(key, psim[j]); key_push(key, pm[j]); }
   while (h.status == ST_RUN) {
     MKS_TRY(graph_batch(key, issue));
@@ -2423,11 +2557,13 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
     if (h.status == ST_HOST && h.want_reliable) {
       // reliable update: fold, FP64 residual of the lowest shift, continue
       if (!wide) MKS_TRY(ms_fold(nsh, x64, psim_out));
-      double2 *t64, *dd64;
-      MKS_TRY(wsv("ms_rel_t64", n, &t64));
+      FxVec xq, dq;
+      double2 *dd64;
+      MKS_TRY(ws_blocks("ms_rel_x", &xq));
+      MKS_TRY(ws_blocks("ms_rel_t", &dq));
       MKS_TRY(wsv("ms_rel_dd64", n, &dd64));
       double2 *xl = x64[h.j_low];
-      MKS_TRY(apply_DD64(sl, par, 1, &xl, &t64, &dd64));
+      MKS_TRY(apply_DD64(sl, par, 1, &xl, &xq, &dq, &dd64));
       OpMsResid op;
       op.src = src64; op.ddx = dd64; op.x = xl; op.r32 = (float2 *)r; op.sigma = offsets[h.j_low]; op.Vh = Vh;
       MKS_TRY((launch_site<OpMsResid, 1, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, 1, tot)));
@@ -2594,11 +2730,13 @@ static int multishift_multi_core(const LinkSlot &sl, int par, int nf, const doub
       if (h.status != ST_HOST || !h.want_reliable) continue;   // stopped fields leave the launches
       // reliable update of field f: fold, FP64 residual of its lowest shift
       if (!wide) MKS_TRY(ms_fold(nsh[f], x64[f], (void *const *)psim[f]));
-      double2 *t64, *dd64;
-      MKS_TRY(wsv("ms_rel_t64", n, &t64));
+      FxVec xq, dq;
+      double2 *dd64;
+      MKS_TRY(ws_blocks("ms_rel_x", &xq));
+      MKS_TRY(ws_blocks("ms_rel_t", &dq));
       MKS_TRY(wsv("ms_rel_dd64", n, &dd64));
       double2 *xl = x64[f][h.j_low];
-      MKS_TRY(apply_DD64(sl, par, 1, &xl, &t64, &dd64));
+      MKS_TRY(apply_DD64(sl, par, 1, &xl, &xq, &dq, &dd64));
       OpMsResid op;
       op.src = src64[f]; op.ddx = dd64; op.x = xl; op.r32 = r[f]; op.sigma = offsets[f][h.j_low]; op.Vh = Vh;
       MKS_TRY((launch_site<OpMsResid, 1, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, 1, tot1)));
