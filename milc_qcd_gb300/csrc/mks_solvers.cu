@@ -396,8 +396,8 @@ static int launch_site(int family, const Op &op, const Fin &fin, const int *skip
   // row.  Every block ends with a block reduction and a row of partial sums,
   // so for many sources fewer, longer blocks win (8 sources on 32^3x64: the
   // CG's update and dot kernels 111 ms per solve of 8 with 2 per row, 117
-  // with 4, 129 with 8), while the one-row multi-shift update needs the 4
-  // (100 ms against 116 with 2).  MKS_SITE_BLOCKS fixes the count per row.
+  // with 4, 129 with 8), while one row needs the 4 to fill the chip.
+  // MKS_SITE_BLOCKS fixes the count per row.
   static int forced = -1;
   if (forced < 0) {
     const char *e = getenv("MKS_SITE_BLOCKS");
@@ -2092,104 +2092,126 @@ struct MsState {
   long long shift_updates;  // sum over iterations of the shifts the update kernel advanced
 };
 
-// the zeta / beta / alpha recurrences of one field after K2 (t: its three sums)
+// The zeta / beta / alpha recurrences of one field after K2 (t: its three
+// sums), one lane per shift: every shift needs the lowest one's beta and
+// alpha and its own history only.  (One thread for all of them took two
+// divisions a shift one after the other, 570 clocks each: on 12^3x24 with 16
+// shifts the launch took 64 us against 19 us of the plain D.)  Called by the
+// 32 lanes of a warp.
+static_assert(MAXSH == 32, "one lane per shift");
 __device__ __forceinline__ void ms_alpha(MsState &m, const double *t) {
-    if (m.status != ST_RUN) return;
-    if (m.need_scroll) {
-      for (int j = 0; j < m.num_now; j++) {
-        m.beta_im1[j] = m.beta_i[j];
-        m.zeta_im1[j] = m.zeta_i[j];
-        m.zeta_i[j] = m.zeta_ip1[j];
-      }
-      m.need_scroll = 0;
+  const int j = threadIdx.x & 31;
+  if (m.status != ST_RUN) return;
+  const int jl = m.j_low, now0 = m.num_now;
+  const bool mine = j < now0;
+  double zi = 0, zm = 0, bm = 0, sh = 0;
+  if (mine) {
+    const bool scroll = m.need_scroll;
+    zi = scroll ? m.zeta_ip1[j] : m.zeta_i[j];
+    zm = scroll ? m.zeta_i[j] : m.zeta_im1[j];
+    bm = scroll ? m.beta_i[j] : m.beta_im1[j];
+    sh = m.shifts[j];
+  }
+  const double alpha_l = m.alpha[jl], rsq = m.rsq, pkp = t[0], c_tr = t[1], c_tt = t[2];
+  const double bml = __shfl_sync(0xffffffffu, bm, jl);
+  const double bl = -rsq / pkp;
+  // |r + beta ttt|^2 from the K2 sums
+  const double rsq_new = rsq + 2.0 * bl * c_tr + bl * bl * c_tt;
+  const double al = rsq_new / rsq;
+  __syncwarp();
+  double zp = 1.0, bi = bl;
+  bool drop = false;
+  if (mine && j != jl) {
+    const double c1 = bl * alpha_l * (zm - zi);
+    const double c2 = zm * bml * (1.0 + sh * bl);
+    zp = c1 + c2 != 0.0 ? zi * zm * bml / (c1 + c2) : 0.0;
+    if (zi != 0.0) {
+      bi = bl * zp / zi;
+    } else {
+      zp = 0.0;
+      bi = 0.0;
+      drop = j > jl;
     }
-    const int jl = m.j_low;
-    double pkp = t[0], c_tr = t[1], c_tt = t[2];
+  }
+  // shifts whose zeta vanished leave from the end, as long as each is the
+  // last one when its turn comes (in the order of j, as MILC's loop does)
+  int now = now0;
+  const unsigned dm = __ballot_sync(0xffffffffu, drop);
+  for (int k = 0; k < now0; k++)
+    if ((dm >> k & 1) && k == now - 1) now--;
+  double aj = al;
+  if (mine && j != jl && j < now) aj = zi * bl != 0.0 ? al * zp * bi / (zi * bl) : 0.0;
+  if (mine) {
+    m.zeta_im1[j] = zm;
+    m.zeta_i[j] = zi;
+    m.beta_im1[j] = bm;
+    m.zeta_ip1[j] = zp;
+    m.beta_i[j] = bi;
+    if (j < now) m.alpha[j] = aj;
+  }
+  // the update kernel of this iteration advances every shift not retired
+  const unsigned adv = __ballot_sync(0xffffffffu, mine && j < now && !m.retired[j]);
+  if (j == 0) {
+    m.need_scroll = 0;
     m.pkp = pkp;
     m.iter++;
-    m.beta_i[jl] = -m.rsq / pkp;
-    m.zeta_ip1[jl] = 1.0;
-    for (int j = 0; j < m.num_now; j++) {
-      if (j == jl) continue;
-      m.zeta_ip1[j] = m.zeta_i[j] * m.zeta_im1[j] * m.beta_im1[jl];
-      double c1 = m.beta_i[jl] * m.alpha[jl] * (m.zeta_im1[j] - m.zeta_i[j]);
-      double c2 = m.zeta_im1[j] * m.beta_im1[jl] * (1.0 + m.shifts[j] * m.beta_i[jl]);
-      if (c1 + c2 != 0.0) m.zeta_ip1[j] /= c1 + c2;
-      else m.zeta_ip1[j] = 0.0;
-      if (m.zeta_i[j] != 0.0) {
-        m.beta_i[j] = m.beta_i[jl] * m.zeta_ip1[j] / m.zeta_i[j];
-      } else {
-        m.zeta_ip1[j] = 0.0;
-        m.beta_i[j] = 0.0;
-        if (j == m.num_now - 1 && j > jl) m.num_now--;
-      }
-    }
-    // |r + beta ttt|^2 from the K2 sums
-    double b = m.beta_i[jl];
-    double rsq_new = m.rsq + 2.0 * b * c_tr + b * b * c_tt;
-    m.alpha[jl] = rsq_new / m.rsq;
-    for (int j = 0; j < m.num_now; j++) {
-      if (j == jl) continue;
-      if (m.zeta_i[j] * m.beta_i[jl] != 0.0)
-        m.alpha[j] = m.alpha[jl] * m.zeta_ip1[j] * m.beta_i[j] / (m.zeta_i[j] * m.beta_i[jl]);
-      else
-        m.alpha[j] = 0.0;
-    }
-    if (!isfinite(m.beta_i[jl])) m.status = ST_HOST;
-    // the update kernel of this iteration advances every shift not retired
-    for (int j = 0; j < m.num_now; j++) m.shift_updates += m.retired[j] ? 0 : 1;
+    m.num_now = now;
+    m.shift_updates += __popc(adv);
+    if (!isfinite(bl)) m.status = ST_HOST;
+  }
 }
 
 struct FinMsAlpha {
   MsState *st;
   __device__ void operator()(const double *t, int) const {
-    if (threadIdx.x != 0) return;
-    ms_alpha(*st, t);
+    if (threadIdx.x < 32) ms_alpha(*st, t);
   }
 };
 
 // the state of one field after K3 (rsq: the new |r|^2): retirement of
-// converged shifts, stop, reliable-update request
+// converged shifts (one lane per shift), stop, reliable-update request
 __device__ __forceinline__ void ms_update(MsState &m, double rsq) {
-    if (m.status == ST_RUN) {
-      m.rsq = rsq;
-      m.need_scroll = 1;
-      if (m.rsqretire > 0)
-        for (int j = 0; j < m.num_now; j++)
-          if (j != m.j_low && m.zeta_ip1[j] * m.zeta_ip1[j] * m.rsq < m.rsqretire) m.retired[j] = 1;
-      if ((m.rsqstop > 0 && m.rsq <= m.rsqstop) || m.iter >= m.niter || !isfinite(m.rsq)) {
-        m.status = ST_HOST;
-        // the sloppy recursion met the target: the host recomputes the
-        // lowest shift's residual in FP64 and goes on unless that meets it
-        if (m.check_true && m.delta > 0 && m.iter < m.niter && isfinite(m.rsq)) m.want_reliable = 1;
-      } else if (m.delta > 0) {
-        // sloppy solve: ask for a reliable update when |r| fell below
-        // delta * max|r| since the last one
-        double rn = sqrt(m.rsq);
-        if (rn > m.maxrr) m.maxrr = rn;
-        if (rn < m.delta * m.maxrr) { m.status = ST_HOST; m.want_reliable = 1; }
-      }
-    }
+  const int j = threadIdx.x & 31;
+  if (m.status != ST_RUN) return;
+  if (m.rsqretire > 0 && j < m.num_now && j != m.j_low && m.zeta_ip1[j] * m.zeta_ip1[j] * rsq < m.rsqretire)
+    m.retired[j] = 1;
+  __syncwarp();
+  if (j != 0) return;
+  m.rsq = rsq;
+  m.need_scroll = 1;
+  if ((m.rsqstop > 0 && m.rsq <= m.rsqstop) || m.iter >= m.niter || !isfinite(m.rsq)) {
+    m.status = ST_HOST;
+    // the sloppy recursion met the target: the host recomputes the
+    // lowest shift's residual in FP64 and goes on unless that meets it
+    if (m.check_true && m.delta > 0 && m.iter < m.niter && isfinite(m.rsq)) m.want_reliable = 1;
+  } else if (m.delta > 0) {
+    // sloppy solve: ask for a reliable update when |r| fell below
+    // delta * max|r| since the last one
+    double rn = sqrt(m.rsq);
+    if (rn > m.maxrr) m.maxrr = rn;
+    if (rn < m.delta * m.maxrr) { m.status = ST_HOST; m.want_reliable = 1; }
+  }
 }
 
 struct FinMsUpdate {
   MsState *st;
   int *skip;
   __device__ void operator()(const double *t, int) const {
-    if (threadIdx.x != 0) return;
+    if (threadIdx.x >= 32) return;
     ms_update(*st, t[0]);
-    *skip = (st->status != ST_RUN);
+    __syncwarp();
+    if (threadIdx.x == 0) *skip = (st->status != ST_RUN);
   }
 };
 
-// several fields in one multi-shift (one per row k, field map[k])
+// several fields in one multi-shift (one per row k, field map[k]), one warp
+// after the other
 constexpr int MSF = 4;
 struct FinMsAlphaM {
   MsState *st;
   int map[MSF];
   __device__ void operator()(const double *t, int n) const {
-    const int k = threadIdx.x;
-    if (k < n) ms_alpha(st[map[k]], t + 3 * k);
+    for (int k = threadIdx.x >> 5; k < n; k += blockDim.x >> 5) ms_alpha(st[map[k]], t + 3 * k);
   }
 };
 struct FinMsUpdateM {
@@ -2197,8 +2219,7 @@ struct FinMsUpdateM {
   int *skip;
   int map[MSF];
   __device__ void operator()(const double *t, int n) const {
-    const int k = threadIdx.x;
-    if (k < n) ms_update(st[map[k]], t[k]);
+    for (int k = threadIdx.x >> 5; k < n; k += blockDim.x >> 5) ms_update(st[map[k]], t[k]);
     __syncthreads();
     if (threadIdx.x == 0) {
       int any = 0;
@@ -2208,93 +2229,170 @@ struct FinMsUpdateM {
   }
 };
 
-// K3 at one site for one field: r += beta ttt, every shift's psim and pm,
-// the lowest shift's p (and its FP16 shadow); out[0] = |r|^2 at the site
-template <typename R, typename RS = R>
-__device__ __forceinline__ void ms_site_update(const MsState &m, typename VT<RS>::v2 *const *psim,
-                                               typename VT<RS>::v2 *const *pm, typename VT<R>::v2 *r,
-                                               const typename VT<R>::v2 *ttt, typename VT<R>::v2 *cgp,
-                                               const FxVec &cgq, __half2 *p16, float *p16n, int h, int Vh,
-                                               double *out) {
-    typedef typename VT<R>::v2 T2;
-    typedef typename VT<RS>::v2 S2;
-    const int n = m.num_now, jl = m.j_low;
-    const R bl = (R)m.beta_i[jl];
-    T2 rn[3];
-    R rr = 0;  // per-site sum in the storage precision
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      size_t i = (size_t)k * Vh + h;
-      T2 rv = r[i], tv = ttt[i];
-      rv.x = rv.x + bl * tv.x; rv.y = rv.y + bl * tv.y;
-      rn[k] = rv;
-      r[i] = rv;
-      rr += rv.x * rv.x + rv.y * rv.y;
-    }
-    for (int j = 0; j < n; j++) {
-      if (m.retired[j]) continue;
-      const RS bj = (RS)m.beta_i[j], zj = (RS)m.zeta_ip1[j], aj = (RS)m.alpha[j];
-      double w[6];
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        size_t i = (size_t)k * Vh + h;
-        S2 pv = pm[j][i], xv = psim[j][i];
-        xv.x = xv.x + bj * pv.x; xv.y = xv.y + bj * pv.y;
-        pv.x = zj * (RS)rn[k].x + aj * pv.x; pv.y = zj * (RS)rn[k].y + aj * pv.y;
-        psim[j][i] = xv;
-        pm[j][i] = pv;
-        if (j == jl) { T2 cv; cv.x = (R)pv.x; cv.y = (R)pv.y; cgp[i] = cv; }
-        if (sizeof(R) == 8) { w[2 * k] = pv.x; w[2 * k + 1] = pv.y; }
-      }
-      if (sizeof(R) == 8 && j == jl) fx_put(cgq, h, Vh, w);
-      if (sizeof(R) == 4 && j == jl && p16) {
-        float mx = 0.f;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          S2 pv = pm[j][(size_t)k * Vh + h];
-          mx = fmaxf(mx, fmaxf(fabsf((float)pv.x), fabsf((float)pv.y)));
-        }
-        float inv = mx > 0.f ? 1.f / mx : 0.f;
-        p16n[h] = mx;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          S2 pv = pm[j][(size_t)k * Vh + h];
-          p16[(size_t)k * Vh + h] = __floats2half2_rn((float)pv.x * inv, (float)pv.y * inv);
-        }
-      }
-    }
-    out[0] = rr;
-}
-
-template <typename R, typename RS = R> struct OpShiftUpdate {
+// K3: r += beta ttt; every shift not retired psim_j += beta_j pm_j, pm_j =
+// zeta_j r + alpha_j pm_j; the lowest shift's p also as D_eo's input (cgp in
+// R, and its FP16 or integer shadow); |r|^2.  NF fields, one per grid row.
+template <typename R, typename RS, int NF> struct MsUpdate {
   typedef typename VT<R>::v2 T2;
   typedef typename VT<RS>::v2 S2;
-  S2 *psim[MAXSH], *pm[MAXSH];
-  T2 *r, *ttt, *cgp;
-  FxVec cgq;  // FP64: cgp as blocks
+  S2 *psim[NF][MAXSH], *pm[NF][MAXSH];
+  T2 *r[NF], *ttt[NF], *cgp[NF];
+  FxVec cgq;          // FP64: cgp as blocks
   __half2 *p16;
   float *p16n;
   const MsState *st;
+  int map[NF];        // field of a grid row
   int Vh;
-  __device__ void operator()(int h, int, double *out) const {
-    ms_site_update<R, RS>(*st, psim, pm, r, ttt, cgp, cgq, p16, p16n, h, Vh, out);
-  }
 };
 
-// the same for several fields, one per row k (field map[k])
-template <typename R, typename RS = R> struct OpShiftUpdateM {
+// The update is elementwise but for |r|^2 and the shadows, so a thread takes
+// one complex component (a warp one component of 32 sites), and on small
+// lattices NG groups of warps share a tile's shifts: the shifts one after the
+// other in one thread per site held 81 blocks on 12^3x24 for 16 serial
+// rounds of loads.  Launches of a solve on average, before and now: 12^3x24
+// FP64 50 and 33 us (with the tree of sum_rows), 16^3x32 FP32 34 and 23 us,
+// 24^3x48 11 shifts in FP64 storage 133 and 121 us.  Bound: HBM (L2 where
+// the fields fit), in FP64 also the FP64 rate (6 operations per component
+// and shift).
+template <typename R, typename RS, int NF, int NG, class Fin>
+__global__ void __launch_bounds__(96 * NG) k_ms_update(const MsUpdate<R, RS, NF> a, const Fin fin, const int *skip,
+                                                      const RedScratch red, double *totals) {
   typedef typename VT<R>::v2 T2;
   typedef typename VT<RS>::v2 S2;
-  S2 *psim[MSF][MAXSH], *pm[MSF][MAXSH];
-  T2 *r[MSF], *ttt[MSF], *cgp[MSF];
-  const MsState *st;
-  int map[MSF];
-  int Vh;
-  __device__ void operator()(int h, int k, double *out) const {
-    const int f = map[k];
-    ms_site_update<R, RS>(st[f], psim[f], pm[f], r[f], ttt[f], cgp[f], FxVec{nullptr, nullptr}, nullptr, nullptr, h, Vh, out);
+  constexpr int U = 4;
+  if (skip && *skip) return;
+  __shared__ struct { S2 *x, *p; RS b, z, a; int low; } act[MAXSH];
+  __shared__ int s_nact;
+  __shared__ R s_low[6][32];
+  const int f = a.map[blockIdx.y], Vh = a.Vh;
+  const MsState &m = a.st[f];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, comp = warp % 3, grp = warp / 3;
+  if (warp == 0) {
+    const bool on = lane < m.num_now && !m.retired[lane];
+    const unsigned mask = __ballot_sync(0xffffffffu, on);
+    if (on) {
+      auto &q = act[__popc(mask & ((1u << lane) - 1))];
+      q.x = a.psim[f][lane];
+      q.p = a.pm[f][lane];
+      q.b = (RS)m.beta_i[lane];
+      q.z = (RS)m.zeta_ip1[lane];
+      q.a = (RS)m.alpha[lane];
+      q.low = lane == m.j_low;
+    }
+    if (lane == 0) s_nact = __popc(mask);
   }
-};
+  __syncthreads();
+  const int nact = s_nact;
+  const R bl = (R)m.beta_i[m.j_low];
+  T2 *r = a.r[f];
+  const T2 *ttt = a.ttt[f];
+  const bool shadow = sizeof(R) == 8 || a.p16 != nullptr;
+  double acc = 0;
+  const int ntiles = (Vh + 31) / 32;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int h = tile * 32 + lane;
+    const bool live = h < Vh;
+    const size_t i = (size_t)comp * Vh + (live ? h : 0);
+    T2 rv = r[i];
+    const T2 tv = ttt[i];
+    rv.x = rv.x + bl * tv.x;
+    rv.y = rv.y + bl * tv.y;
+    if (NG > 1) __syncthreads();   // every group has read r
+    if (grp == 0 && live) {
+      r[i] = rv;
+      acc += (double)(rv.x * rv.x + rv.y * rv.y);
+    }
+    if (live) {
+      for (int k0 = grp; k0 < nact; k0 += U * NG) {
+        // U shifts' loads in flight before the first store
+        S2 xv[U], pv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int k = k0 + u * NG;
+          if (k < nact) { xv[u] = act[k].x[i]; pv[u] = act[k].p[i]; }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int k = k0 + u * NG;
+          if (k >= nact) break;
+          const RS bj = act[k].b, zj = act[k].z, aj = act[k].a;
+          xv[u].x = xv[u].x + bj * pv[u].x;
+          xv[u].y = xv[u].y + bj * pv[u].y;
+          pv[u].x = zj * (RS)rv.x + aj * pv[u].x;
+          pv[u].y = zj * (RS)rv.y + aj * pv[u].y;
+          act[k].x[i] = xv[u];
+          act[k].p[i] = pv[u];
+          if (act[k].low) {
+            T2 cv;
+            cv.x = (R)pv[u].x;
+            cv.y = (R)pv[u].y;
+            a.cgp[f][i] = cv;
+            if (shadow) {
+              s_low[2 * comp][lane] = cv.x;
+              s_low[2 * comp + 1][lane] = cv.y;
+            }
+          }
+        }
+      }
+    }
+    if (shadow) {
+      __syncthreads();
+      if (warp == 0 && live) {
+        if constexpr (sizeof(R) == 8) {
+          double w[6];
+#pragma unroll
+          for (int k = 0; k < 6; k++) w[k] = s_low[k][lane];
+          fx_put(a.cgq, h, Vh, w);
+        } else {
+          float mx = 0.f;
+#pragma unroll
+          for (int k = 0; k < 6; k++) mx = fmaxf(mx, fabsf(s_low[k][lane]));
+          const float inv = mx > 0.f ? 1.f / mx : 0.f;
+          a.p16n[h] = mx;
+#pragma unroll
+          for (int k = 0; k < 3; k++)
+            a.p16[(size_t)k * Vh + h] = __floats2half2_rn(s_low[2 * k][lane] * inv, s_low[2 * k + 1][lane] * inv);
+        }
+      }
+      __syncthreads();
+    }
+  }
+  __shared__ double wsum[3];
+  __shared__ double row[NF], tot[NF];
+  __shared__ double scratch[96 * NG];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0 && grp == 0) wsum[comp] = acc;
+  if (threadIdx.x < NF) row[threadIdx.x] = 0.0;
+  __syncthreads();
+  if (threadIdx.x == 0) row[blockIdx.y] = wsum[0] + wsum[1] + wsum[2];
+  __syncthreads();
+  const int n = gridDim.y;
+  if (!grid_reduce_last(row, n, red, tot, scratch)) return;
+  if (threadIdx.x == 0 && totals)
+    for (int k = 0; k < n; k++) totals[k] = tot[k];
+  __syncthreads();
+  fin(tot, n);
+}
+
+template <typename R, typename RS, int NF, class Fin>
+static int launch_ms_update(const MsUpdate<R, RS, NF> &a, const Fin &fin, const int *skip, int rows, int nsh) {
+  Context &c = ctx();
+  const int ntiles = grid_for(c.Vh, 32);
+  // groups of shifts: while one group leaves under 32 warps per SM
+  const size_t warps = (size_t)ntiles * 3 * rows, full = (size_t)c.sm_count * 32;
+  const int ng = nsh >= 8 && warps * 2 < full ? 4 : nsh >= 4 && warps < full ? 2 : 1;
+  const int cap = c.sm_count * 16 / (ng * rows) > c.sm_count ? c.sm_count * 16 / (ng * rows) : c.sm_count;
+  const int gx = ntiles < cap ? ntiles : cap;
+  MKS_TRY(ensure_red(rows, gx * rows));
+  timing_begin(MKS_K_SHIFT);
+  const dim3 grid(gx, rows);
+  if (ng == 4) k_ms_update<R, RS, NF, 4, Fin><<<grid, 384, 0, c.stream>>>(a, fin, skip, c.red, nullptr);
+  else if (ng == 2) k_ms_update<R, RS, NF, 2, Fin><<<grid, 192, 0, c.stream>>>(a, fin, skip, c.red, nullptr);
+  else k_ms_update<R, RS, NF, 1, Fin><<<grid, 96, 0, c.stream>>>(a, fin, skip, c.red, nullptr);
+  timing_end(MKS_K_SHIFT);
+  MKS_CUDA(cudaGetLastError());
+  return MKS_OK;
+}
 
 // initial fields: r = p = pm_j = src (converted), psim_j = 0
 template <typename R, typename RS = R> struct OpShiftInit {
@@ -2528,11 +2626,11 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
         a2.r[0].p = (float2 *)r; a2.coef[0] = h.shift0;
         MKS_TRY((launch_dslash<float, LinkF16, VecF16, VecF32, EPI_AXPY, 3>(MKS_K_DSLASH_F16, L.fat, L.lng, a2, FinMsAlpha{st})));
       }
-      OpShiftUpdate<R, RS> up;
+      MsUpdate<R, RS, 1> up;
       memset(&up, 0, sizeof up);
-      for (int j = 0; j < nsh; j++) { up.psim[j] = psim[j]; up.pm[j] = pm[j]; }
-      up.r = r; up.ttt = ttt; up.cgp = cgp; up.cgq = cgq; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh;
-      MKS_TRY((launch_site<OpShiftUpdate<R, RS>, 1, FinMsUpdate>(MKS_K_SHIFT, up, FinMsUpdate{st, skip}, skip, 1)));
+      for (int j = 0; j < nsh; j++) { up.psim[0][j] = psim[j]; up.pm[0][j] = pm[j]; }
+      up.r[0] = r; up.ttt[0] = ttt; up.cgp[0] = cgp; up.cgq = cgq; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh;
+      MKS_TRY(launch_ms_update(up, FinMsUpdate{st, skip}, skip, 1, nsh));
     }
     return MKS_OK;
   };
@@ -2687,17 +2785,19 @@ static int multishift_multi_core(const LinkSlot &sl, int par, int nf, const doub
           fa.map[q] = f;
         }
         MKS_TRY((launch_dslash<float, LinkF32, VecF32, VecF32, EPI_AXPY, 3>(MKS_K_DSLASH_F32, L.fat, L.lng, a2, fa)));
-        OpShiftUpdateM<float, RS> up;
+        MsUpdate<float, RS, MSF> up;
         memset(&up, 0, sizeof up);
+        int nshmax = 0;
         FinMsUpdateM fu;
         fu.st = st; fu.skip = skip;
         for (int f = 0; f < nf; f++) {
           for (int j = 0; j < nsh[f]; j++) { up.psim[f][j] = psim[f][j]; up.pm[f][j] = pm[f][j]; }
+          nshmax = nsh[f] > nshmax ? nsh[f] : nshmax;
           up.r[f] = r[f]; up.ttt[f] = ttt[f]; up.cgp[f] = cgp[f];
         }
         for (int q = 0; q < nact; q++) { up.map[q] = act[q]; fu.map[q] = act[q]; }
         up.st = st; up.Vh = Vh;
-        MKS_TRY((launch_site<OpShiftUpdateM<float, RS>, 1, FinMsUpdateM>(MKS_K_SHIFT, up, fu, skip, nact)));
+        MKS_TRY(launch_ms_update(up, fu, skip, nact, nshmax));
       }
       return MKS_OK;
     };
