@@ -26,6 +26,7 @@
 #include <vector>
 #include "mks_internal.cuh"
 #include "mks_su3.cuh"
+#include "mks_fixed_mat.cuh"
 
 namespace mks {
 
@@ -332,6 +333,74 @@ struct ForceRun {
     return MKS_OK;
   }
 
+  // FP64 fields: the staples and their reverse in integer arithmetic
+  static int staple_fwd_fx(int mu, int nu, const FxMat &U, const FxMat &A, const FxMat &S) {
+    Context &c = ctx();
+    const MatF none = {nullptr, 0};
+    timing_begin(MKS_K_FORCE);
+    k_staple_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2), FXM_BLOCK, 0, c.stream>>>(c.geom, mu, nu, U, A, none, 0.0, S);
+    timing_end(MKS_K_FORCE);
+    g_force_flops += 4.0 * 198 * c.V;
+    MKS_CUDA(cudaGetLastError());
+    return MKS_OK;
+  }
+  static int staple_adj_fx(int mu, int nu, const FxMat &U, const FxMat &A, const FxMat &K, double f, MatF init,
+                           double cinit, MatF KA, const FxMat &kout, MatF KU) {
+    Context &c = ctx();
+    timing_begin(MKS_K_FORCE);
+    k_staple_adj_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2), FXM_BLOCK, 0, c.stream>>>(c.geom, mu, nu, U, A, K, f, init,
+                                                                                 cinit, KA, kout, KU);
+    timing_end(MKS_K_FORCE);
+    g_force_flops += 12.0 * 198 * c.V;
+    MKS_CUDA(cudaGetLastError());
+    return MKS_OK;
+  }
+  // fat_adj on integers: links, Kfat and the staple fields once as integers;
+  // K2 leaves its kernel as integers, K1 with its last contribution
+  static int fat_adj_fx(double2 *links, const ForceCoeffs &cf, double2 *Kfat, double2 *KU, double2 *S1, double2 *S2,
+                        double2 *K1, double2 *K2) {
+    const size_t Vh = ctx().Vh;
+    FxMat L, K, fS1, fS2, fK1, fK2;
+    const FxMat off = {nullptr, nullptr, 0, 0};
+    const MatF none = {nullptr, 0}, mK1 = mat_field(K1, Vh);
+    MKS_TRY(ws_links_fxm("fxm_links", MKS_K_FORCE, links, &L));
+    MKS_TRY(ws_links_fxm("fxm_kfat", MKS_K_FORCE, Kfat, &K));
+    MKS_TRY(ws_fxm("fxm_s", 1, &fS1, S1));
+    MKS_TRY(ws_fxm("fxm_t", 1, &fS2, S2));
+    MKS_TRY(ws_fxm("fxm_k1", 1, &fK1));
+    MKS_TRY(ws_fxm("fxm_k2", 1, &fK2, K2));
+    for (int mu = 0; mu < 4; mu++) {
+      const MatF Kd = link_dir(Kfat, mu, Vh), KUm = link_dir(KU, mu, Vh);
+      const FxMat Km = fx_link_dir(K, mu, Vh), Um = fx_link_dir(L, mu, Vh);
+      for (int nu = 0; nu < 4; nu++) {
+        if (nu == mu) continue;
+        const FxMat Un = fx_link_dir(L, nu, Vh);
+        const MatF KUn = link_dir(KU, nu, Vh);
+        MKS_TRY(staple_fwd_fx(mu, nu, Un, Um, fS1));
+        bool first = true;   // K1's first contribution starts from c3 Kfat_mu
+        if (cf.lepage != 0.0) {
+          MKS_TRY(staple_adj_fx(mu, nu, Un, fS1, Km, cf.lepage, Kd, cf.three_staple, mK1, off, KUn));
+          first = false;
+        }
+        int left = 2;
+        for (int rho = 0; rho < 4; rho++) {
+          if (rho == mu || rho == nu) continue;
+          const int sig = 6 - mu - nu - rho;
+          const FxMat Ur = fx_link_dir(L, rho, Vh), Us = fx_link_dir(L, sig, Vh);
+          MKS_TRY(staple_fwd_fx(mu, rho, Ur, fS1, fS2));
+          // K2 = c5 Kfat_mu + c7 (reverse of the sigma staple)
+          MKS_TRY(staple_adj_fx(mu, sig, Us, fS2, Km, cf.seven_staple, Kd, cf.five_staple, none, fK2,
+                                link_dir(KU, sig, Vh)));
+          MKS_TRY(staple_adj_fx(mu, rho, Ur, fS1, fK2, 1.0, first ? Kd : none, cf.three_staple, mK1,
+                                --left == 0 ? fK1 : off, link_dir(KU, rho, Vh)));
+          first = false;
+        }
+        MKS_TRY(staple_adj_fx(mu, nu, Un, Um, fK1, 1.0, none, 1.0, KUm, off, KUn));
+      }
+    }
+    return MKS_OK;
+  }
+
   static int axpby(const T2 *x, T2 *y, double a, double b, size_t n) {
     Context &c = ctx();
     timing_begin(MKS_K_FORCE);
@@ -344,11 +413,15 @@ struct ForceRun {
   // reverse of the fat-link staple recursion (load_fatlinks_cpu, ASQ_OPTIMIZED_FATTENING):
   // KU += d fat(links) / d links contracted with Kfat
   static int fat_adj(T2 *links, const ForceCoeffs &cf, T2 *Kfat, T2 *KU, T2 *S1, T2 *S2, T2 *K1, T2 *K2) {
+    const double one_link = cf.one_link - 6.0 * cf.lepage;
+    MKS_TRY(axpby(Kfat, KU, one_link, 1.0, 8 * 9 * ctx().Vh));
+    if (cf.three_staple == 0.0 && cf.lepage == 0.0 && cf.five_staple == 0.0) return MKS_OK;
+    if constexpr (sizeof(R) == 8) return fat_adj_fx(links, cf, Kfat, KU, S1, S2, K1, K2);
+    else return fat_adj_direct(links, cf, Kfat, KU, S1, S2, K1, K2);
+  }
+  static int fat_adj_direct(T2 *links, const ForceCoeffs &cf, T2 *Kfat, T2 *KU, T2 *S1, T2 *S2, T2 *K1, T2 *K2) {
     Context &c = ctx();
     const size_t Vh = c.Vh, nm = 2 * 9 * Vh;
-    const double one_link = cf.one_link - 6.0 * cf.lepage;
-    MKS_TRY(axpby(Kfat, KU, one_link, 1.0, 8 * 9 * Vh));
-    if (cf.three_staple == 0.0 && cf.lepage == 0.0 && cf.five_staple == 0.0) return MKS_OK;
     const MatT<R> mS1 = mat_field(S1, Vh), mS2 = mat_field(S2, Vh), mK1 = mat_field(K1, Vh), mK2 = mat_field(K2, Vh);
     for (int mu = 0; mu < 4; mu++) {
       const MatT<R> Kd = link_dir(Kfat, mu, Vh), Um = link_dir(links, mu, Vh), KUm = link_dir(KU, mu, Vh);

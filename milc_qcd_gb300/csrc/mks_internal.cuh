@@ -22,6 +22,7 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <string>
 #include <vector>
 #include "milc_ks_gb300.h"
 
@@ -422,7 +423,8 @@ int timing_flush();
 int dev_alloc(void **p, size_t bytes);
 void dev_free(void *p);
 
-// named workspace buffers of the solvers (mks_solvers.cu)
+// named workspace buffers kept across calls, until the lattice changes (mks_solvers.cu)
+int ws(const std::string &name, size_t bytes, void **out);
 void ws_free_all();
 
 // reduction scratch sized for `nsum` sums and `blocks` blocks

@@ -25,6 +25,7 @@
 #include <vector>
 #include "mks_internal.cuh"
 #include "mks_su3.cuh"
+#include "mks_fixed_mat.cuh"
 
 namespace mks {
 
@@ -157,6 +158,17 @@ struct Smear {
     return MKS_OK;
   }
 
+  // the staples in integer arithmetic (FP64 fields): the links and the staple
+  // fields S, T as integers, fat links accumulated in FP64
+  static int staple_fx(int mu, int nu, const FxMat &U, const FxMat &A, MatF fat, double coef, const FxMat &sout) {
+    Context &c = ctx();
+    timing_begin(MKS_K_LINKS);
+    k_staple_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2), FXM_BLOCK, 0, c.stream>>>(c.geom, mu, nu, U, A, fat, coef, sout);
+    timing_end(MKS_K_LINKS);
+    MKS_CUDA(cudaGetLastError());
+    return MKS_OK;
+  }
+
   // load_fatlinks_cpu, ASQ_OPTIMIZED_FATTENING (fermion_links_fn_load_milc.c:207-253)
   static int fatten(T2 *links, const FatCoeffs &cf, T2 *fat, T2 *staple, T2 *tmp) {
     Context &c = ctx();
@@ -167,26 +179,52 @@ struct Smear {
     timing_end(MKS_K_LINKS);
     MKS_CUDA(cudaGetLastError());
     if (cf.three_staple == 0.0 && cf.lepage == 0.0 && cf.five_staple == 0.0) return MKS_OK;
-    MatT<R> none = {nullptr, 0};
-    for (int mu = 0; mu < 4; mu++) {
-      MatT<R> Fm = link_dir(fat, mu, Vh), Um = link_dir(links, mu, Vh);
-      for (int nu = 0; nu < 4; nu++) {
-        if (nu == mu) continue;
-        MatT<R> Un = link_dir(links, nu, Vh);
-        MatT<R> S = mat_field(staple, Vh), T = mat_field(tmp, Vh);
-        MKS_TRY(launch_staple(mu, nu, Un, Um, Fm, cf.three_staple, S));
-        if (cf.lepage != 0.0) MKS_TRY(launch_staple(mu, nu, Un, S, Fm, cf.lepage, none));
-        for (int rho = 0; rho < 4; rho++) {
-          if (rho == mu || rho == nu) continue;
-          MatT<R> Ur = link_dir(links, rho, Vh);
-          MKS_TRY(launch_staple(mu, rho, Ur, S, Fm, cf.five_staple, T));
-          for (int sig = 0; sig < 4; sig++) {
-            if (sig == mu || sig == nu || sig == rho) continue;
-            MatT<R> Us = link_dir(links, sig, Vh);
-            MKS_TRY(launch_staple(mu, sig, Us, T, Fm, cf.seven_staple, none));
+    if constexpr (sizeof(R) == 8) {
+      FxMat L, S, T;
+      const FxMat off = {nullptr, nullptr, 0, 0};
+      MKS_TRY(ws_links_fxm("fxm_links", MKS_K_LINKS, links, &L));
+      MKS_TRY(ws_fxm("fxm_s", 1, &S, staple));
+      MKS_TRY(ws_fxm("fxm_t", 1, &T, tmp));
+      for (int mu = 0; mu < 4; mu++) {
+        const MatF Fm = link_dir(fat, mu, Vh);
+        const FxMat Um = fx_link_dir(L, mu, Vh);
+        for (int nu = 0; nu < 4; nu++) {
+          if (nu == mu) continue;
+          const FxMat Un = fx_link_dir(L, nu, Vh);
+          MKS_TRY(staple_fx(mu, nu, Un, Um, Fm, cf.three_staple, S));
+          if (cf.lepage != 0.0) MKS_TRY(staple_fx(mu, nu, Un, S, Fm, cf.lepage, off));
+          for (int rho = 0; rho < 4; rho++) {
+            if (rho == mu || rho == nu) continue;
+            MKS_TRY(staple_fx(mu, rho, fx_link_dir(L, rho, Vh), S, Fm, cf.five_staple, T));
+            for (int sig = 0; sig < 4; sig++) {
+              if (sig == mu || sig == nu || sig == rho) continue;
+              MKS_TRY(staple_fx(mu, sig, fx_link_dir(L, sig, Vh), T, Fm, cf.seven_staple, off));
+            }
           }
         }
       }
+    } else {
+      MatT<R> none = {nullptr, 0};
+      for (int mu = 0; mu < 4; mu++) {
+        MatT<R> Fm = link_dir(fat, mu, Vh), Um = link_dir(links, mu, Vh);
+        for (int nu = 0; nu < 4; nu++) {
+          if (nu == mu) continue;
+          MatT<R> Un = link_dir(links, nu, Vh);
+          MatT<R> S = mat_field(staple, Vh), T = mat_field(tmp, Vh);
+          MKS_TRY(launch_staple(mu, nu, Un, Um, Fm, cf.three_staple, S));
+          if (cf.lepage != 0.0) MKS_TRY(launch_staple(mu, nu, Un, S, Fm, cf.lepage, none));
+          for (int rho = 0; rho < 4; rho++) {
+            if (rho == mu || rho == nu) continue;
+            MatT<R> Ur = link_dir(links, rho, Vh);
+            MKS_TRY(launch_staple(mu, rho, Ur, S, Fm, cf.five_staple, T));
+            for (int sig = 0; sig < 4; sig++) {
+              if (sig == mu || sig == nu || sig == rho) continue;
+              MatT<R> Us = link_dir(links, sig, Vh);
+              MKS_TRY(launch_staple(mu, sig, Us, T, Fm, cf.seven_staple, none));
+            }
+          }
+        }
+    }
     }
     return MKS_OK;
   }

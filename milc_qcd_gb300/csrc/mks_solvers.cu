@@ -32,7 +32,7 @@ namespace mks {
 struct WsBuf { void *p = nullptr; size_t bytes = 0; };
 static std::map<std::string, WsBuf> g_ws;
 
-static int ws(const std::string &name, size_t bytes, void **out) {
+int ws(const std::string &name, size_t bytes, void **out) {
   WsBuf &b = g_ws[name];
   if (b.bytes < bytes) {
     dev_free(b.p);
