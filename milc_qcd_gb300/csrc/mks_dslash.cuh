@@ -481,18 +481,48 @@ __device__ __forceinline__ void dslash_body(const LinkT &fat, const LinkT &lng,
   }
 }
 
-// the multi-source shapes (G threads per site x NB sources per thread);
-// the FP32/FP16 plain D with up to 4 sources per thread is held to 64
-// registers (4 resident 256-thread blocks per SM), which it needs without
-// spilling
-#ifndef MKS_DSLASH_MINB
-#define MKS_DSLASH_MINB 4
-#endif
+// the multi-source shapes with the fused epilogue (G threads per site x NB
+// sources per thread, the G threads of a site side by side)
 template <typename R, class LinkT, class InT, class OutT, int NB, int EPI, int NSUM, class Fin>
-__global__ void __launch_bounds__(256, (sizeof(R) == 4 && NB <= 4 && EPI == EPI_PLAIN && !LinkT::scaled) ? MKS_DSLASH_MINB : 0)
+__global__ void __launch_bounds__(256)
 k_dslash(const LinkT fat, const LinkT lng, const DslashArgs<InT, OutT, typename EpiLoad<R>::type> a,
          const Fin fin) {
   dslash_body<R, LinkT, InT, OutT, NB, EPI, NSUM, Fin>(fat, lng, a, fin);
+}
+
+// The multi-source plain D: the G threads of a site sit in G warps of a block
+// at the same lane (the block holds a multiple of G warps) and lanes are
+// consecutive sites.  A vector load is then one contiguous row of one array,
+// and a link load brings 32 sites' entries in the four wavefronts that 32 / G
+// sites' took with the G threads side by side (their copies do not make a
+// 16-byte load narrower); the other groups' copies hit in L1.  Bound: the
+// latency of L2 round trips that 32 warps per SM leave uncovered.  FP32 on
+// 32^3x64, side by side and by warps: 8 sources (G = 2, NB = 4) 0.420 and
+// 0.388 ms of a floor of 0.238 (HBM), 16 sources (G = 4) 1.035 and 0.752 ms of
+// 0.297.  The FP32 plain D with up to 4 sources per thread is held to 64
+// registers (1024 threads per SM), which it needs without spilling.
+template <typename R, class LinkT, class InT, class OutT, int NB>
+__global__ void __launch_bounds__(512, (sizeof(R) == 4 && NB <= 4 && !LinkT::scaled) ? 2 : 1)
+k_dslash_w(const LinkT fat, const LinkT lng, const DslashArgs<InT, OutT, typename EpiLoad<R>::type> a) {
+  if (a.skip && *a.skip) return;
+  const Geom &g = a.g;
+  const int G = a.groups, Vh = g.Vh, par = a.out_par;
+  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nwarps = (int)blockDim.x >> 5;
+  const int grp = warp % G, bid = a.rev ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+  const int h = (bid * (nwarps / G) + warp / G) * 32 + lane;
+  if (h >= Vh) return;
+  int x, y, z, t;
+  site_coords(g, par, h, x, y, z, t);
+  const int c0[4] = {x, y, z, t};
+  V3<R> acc[NB];
+#pragma unroll
+  for (int s = 0; s < NB; s++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) acc[s].c[c] = {R(0), R(0)};
+  site_terms<R, LinkT, InT, NB, false>(fat, lng, a.in, a.nsrc, grp, g, par, h, c0, acc);
+#pragma unroll
+  for (int s = 0; s < NB; s++)
+    if (grp * NB + s < a.nsrc) a.out[grp * NB + s].store(h, Vh, acc[s]);
 }
 
 // the multi-source shapes on a persistent grid: as many CTAs as fit on the

@@ -567,13 +567,24 @@ static int launch_dslash_nb(int family, const LinkT &fat, const LinkT &lng,
     }
   }
   auto k1 = k_dslash1<R, LinkT, InT, OutT, EPI, NSUM, Fin>;
-  auto kd = k_dslash<R, LinkT, InT, OutT, NB, EPI, NSUM, Fin>;
   if constexpr (!has_variants<LinkT, EPI>()) {
     pipe = false;
     persist = false;
   }
   if (persist) pipe = false;  // the persistent kernel loads directly
   const bool one = !pipe && !persist && NB == 1 && a.groups == 1 && block == 256;
+  if constexpr (EPI == EPI_PLAIN) {
+    if (!one && !pipe && !persist) {
+      // blocks of a multiple of G warps
+      if (block % (32 * a.groups)) block = 32 * a.groups;
+      timing_begin(family);
+      k_dslash_w<R, LinkT, InT, OutT, NB>
+          <<<(int)((threads + block - 1) / block), block, 0, c.stream>>>(fat, lng, a);
+      timing_end(family);
+      MKS_CUDA(cudaGetLastError());
+      return MKS_OK;
+    }
+  }
   int grid = nvb;
   a.nvb = 0;
   if constexpr (has_variants<LinkT, EPI>()) {
@@ -593,15 +604,15 @@ static int launch_dslash_nb(int family, const LinkT &fat, const LinkT &lng,
       k_dslash_g<R, LinkT, InT, OutT, NB, EPI, NSUM, Fin><<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
     else if (pipe)
       k_dslash_p<R, LinkT, InT, OutT, NB, EPI, NSUM, Fin><<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
-    else if (one)
-      k1<<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
     else
-      kd<<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
+      k1<<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
+  } else if constexpr (EPI == EPI_PLAIN) {
+    k1<<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
   } else {
     if (one)
       k1<<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
     else
-      kd<<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
+      k_dslash<R, LinkT, InT, OutT, NB, EPI, NSUM, Fin><<<grid, block, 0, c.stream>>>(fat, lng, a, fin);
   }
   timing_end(family);
   MKS_CUDA(cudaGetLastError());
