@@ -114,6 +114,11 @@ __device__ __forceinline__ void fx_mad(u64 &s, int x, int y) {
   // (8 sources, 24^3x48: 1.33 against 0.83 ms)
   asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(s) : "r"(x), "r"(y));
 }
+__device__ __forceinline__ u64 fx_mul(int x, int y) {
+  u64 s;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(s) : "r"(x), "r"(y));
+  return s;
+}
 __device__ __forceinline__ void fx_mac(FxSum &s, int xh, int xl, int yh, int yl) {
   fx_mad(s.H, xh, yh);
   fx_mad(s.M, xh, yl);

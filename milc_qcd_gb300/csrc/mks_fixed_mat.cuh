@@ -3,40 +3,54 @@
 // them (see mks_fixed.cuh for why: an fma.f64 costs 30 integer multiply-adds).
 //
 // A matrix is nine complex entries as integers with one exponent: component =
-// q 2^(e-60), |q| <= 2^60, cut as q = 4 (h 2^30 + l), |h| <= 2^28, l signed,
-// stored as int4 {re h, re l, im h, im l} (the 16 bytes of a double2).  A
-// product is K = H 2^60 + M 2^30 by three multiply-adds per real product (the
-// low halves' product, 2^-58 of the operands' bounds, is left out) and three
-// real products per complex one; six terms of 2^56 leave room in 64 bits, and
-// partial sums may wrap around.  q_out = 2 H + M 2^-29 keeps 60 bits of the
-// bound 6 * 2^56, e_out = e_a + e_b + 3.  A matrix of zeros has e = FX_ZERO,
-// one that holds an infinity or a NaN e = FX_SPECIAL and the doubles' bits; a
-// site that meets one is done in plain FP64.
+// q 2^(e-60), |q| <= 2^60, cut as q = h 2^32 + l, |h| <= 2^28, |l| < 2^31, stored
+// as int4 {re h, re l, im h, im l} (the 16 bytes of a double2) in tiles of 32
+// sites, so that an entry is a constant distance from the last.  A product is
+// K = H 2^64 + M 2^32 by three multiply-adds per real product (the low halves'
+// product, 2^-58 of the operands' bounds, is left out); six terms of 2^56 and
+// twelve of 2^59 leave room in 64 bits.  Complex products take four real ones:
+// with the three of D_eo the sums of halves, and the narrower l that they
+// need, cost more instructions than the multiply-adds they save (the integer
+// ALU, half as fast as a multiply-add's issue rate would have it, is what
+// bounds these kernels).  The first product of a chain keeps K 2^-64, one add
+// of M's high word; the last K 2^-61.  A matrix of zeros has e = FX_ZERO, one
+// that holds an infinity or a NaN e = FX_SPECIAL and the doubles' bits; a site
+// that meets one is done in plain FP64.
 //
 // A staple term is a chain L (M R) of three matrices, its adjoint six chains;
 // the chains run in a loop whose operands are fetched three ahead into shared
 // memory by cp.async (a fetch in flight holds no registers, of which the
-// products take about 200).
+// products take up to 200); the FP64 fields that the result is added to come
+// the same way behind the last chain.
 #pragma once
 #include "mks_fixed.cuh"
 #include "mks_su3.cuh"
 
 namespace mks {
 
-// one direction of a link field, or a single matrix field
+// a field of nd = 4 matrices per site (a direction each) or nd = 1 (every
+// direction uses it), or one direction of it: entry k of site h at
+// p[par ps + (9 (h / 32) + k) 32 + h % 32]
 struct FxMat {
-  int4 *p;     // [par ps + k Vh + h]
+  int4 *p;
   int *e;      // [par es + h]
   size_t ps, es;
+  int nd;
+  __host__ __device__ static size_t sites(size_t Vh) { return (Vh + 31) / 32 * 32; }
+  __device__ __forceinline__ int4 *at(int par, int h) const {
+    return p + par * ps + (size_t)(h >> 5) * 288 + (h & 31);
+  }
 };
-__host__ __device__ inline FxMat fx_link_dir(const FxMat &f, int dir, size_t Vh) {
-  return {f.p + (size_t)dir * 9 * Vh, f.e + (size_t)dir * Vh, 36 * Vh, 4 * Vh};
+__device__ __forceinline__ FxMat fx_link_dir(const FxMat &f, int dir, size_t Vh) {
+  const size_t d = f.nd == 4 ? dir : 0;
+  return {f.p + d * 9 * FxMat::sites(Vh), f.e + d * Vh, f.ps, f.es, 1};
 }
 
+// l never is -2^31, which has no negative (one unit of 2^-60 off instead)
 __device__ __forceinline__ void fxm_split(s64 q, int &h, int &l) {
   const int lo = (int)q;
   h = (int)(q >> 32) + (int)((unsigned)lo >> 31);
-  l = lo >> 2;
+  l = max(lo, -0x7fffffff);
 }
 
 // a matrix of doubles as integers
@@ -59,8 +73,8 @@ __device__ __forceinline__ void fxm_encode(const double2 (&v)[9], int4 (&u)[9], 
   e = max(ex, 1) - 1022;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    fxm_split(fx_scale(v[k].x, e) + 2, u[k].x, u[k].y);   // + 2: rounds the cut at 4
-    fxm_split(fx_scale(v[k].y, e) + 2, u[k].z, u[k].w);
+    fxm_split(fx_scale(v[k].x, e), u[k].x, u[k].y);
+    fxm_split(fx_scale(v[k].y, e), u[k].z, u[k].w);
   }
   if (!any) e = FX_ZERO;
 }
@@ -76,19 +90,19 @@ static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__re
 #pragma unroll
   for (int k = 0; k < 9; k++) v[k] = s[(size_t)k * Vh];
   fxm_encode(v, u, e);
+  int4 *d = fx_link_dir(dst, mu, Vh).at(par, h);
 #pragma unroll
-  for (int k = 0; k < 9; k++) dst.p[(size_t)(par * 4 + mu) * 9 * Vh + (size_t)k * Vh + h] = u[k];
+  for (int k = 0; k < 9; k++) d[32 * k] = u[k];
   dst.e[(size_t)(par * 4 + mu) * Vh + h] = e;
 }
 
-// workspace of `mats` integer matrices per site and parity under `name`
-// (p given: the entries go there)
-inline int ws_fxm(const char *name, int mats, FxMat *f, void *p = nullptr) {
+// workspace of `mats` (1 or 4) integer matrices per site under `name`
+inline int ws_fxm(const char *name, int mats, FxMat *f) {
   const size_t Vh = ctx().Vh;
-  if (!p) MKS_TRY(ws(std::string(name) + "_p", (size_t)mats * 2 * 9 * Vh * sizeof(int4), &p));
-  f->p = (int4 *)p;
-  f->ps = (size_t)mats * 9 * Vh;
+  f->ps = (size_t)mats * 9 * FxMat::sites(Vh);
   f->es = (size_t)mats * Vh;
+  f->nd = mats;
+  MKS_TRY(ws(std::string(name) + "_p", 2 * f->ps * sizeof(int4), (void **)&f->p));
   return ws(std::string(name) + "_e", (size_t)mats * 2 * Vh * sizeof(int), (void **)&f->e);
 }
 
@@ -109,21 +123,28 @@ struct FxRef {
   int e, adj;
 };
 __device__ __forceinline__ FxRef fx_ref(const FxMat &f, int par, int h, int adj) {
-  return {f.p + par * f.ps + h, __ldg(f.e + par * f.es + h), adj};
+  return {f.at(par, h), __ldg(f.e + par * f.es + h), adj};
 }
 
 constexpr int FXM_BLOCK = 64;   // threads per block of the chain kernels
 struct FxRing { int4 v[3][9][FXM_BLOCK]; };
 
-__device__ __forceinline__ void fxm_fetch(FxRing &s, int slot, const FxRef &r, int Vh) {
+__device__ __forceinline__ void fxm_cp(FxRing &s, int slot, int k, const void *p) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(&s.v[slot][k][threadIdx.x])),
+               "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void fxm_fetch(FxRing &s, int slot, const FxRef &r) {
 #pragma unroll
-  for (int k = 0; k < 9; k++) {
-    const size_t off = (size_t)(r.adj ? (k % 3) * 3 + k / 3 : k) * Vh;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                     (uint32_t)__cvta_generic_to_shared(&s.v[slot][k][threadIdx.x])),
-                 "l"(r.p + off)
-                 : "memory");
-  }
+  for (int k = 0; k < 9; k++) fxm_cp(s, slot, k, r.p + 32 * k);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// a matrix of an FP64 field behind the chains (p = nullptr: nothing)
+__device__ __forceinline__ void fxm_fetch_f64(FxRing &s, int slot, const double2 *p, int Vh) {
+  if (p)
+#pragma unroll
+    for (int k = 0; k < 9; k++) fxm_cp(s, slot, k, p + (size_t)k * Vh);
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 __device__ __forceinline__ void fxm_take(const FxRing &s, int slot, int adj, int4 (&u)[9]) {
@@ -131,40 +152,30 @@ __device__ __forceinline__ void fxm_take(const FxRing &s, int slot, int adj, int
   const int sg = adj ? -1 : 1;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    u[k] = s.v[slot][k][threadIdx.x];
+    u[k] = s.v[slot][adj ? (k % 3) * 3 + k / 3 : k][threadIdx.x];
     u[k].z *= sg;
     u[k].w *= sg;
   }
 }
 
-// the right operand of a product with the sums of the three-product form
-struct FxRight { int ch[9], cl[9], mh[9], ml[9], ph[9], pl[9]; };
-__device__ __forceinline__ void fxm_right(const int4 (&u)[9], FxRight &r) {
+// element (i, j) of A B as (H, M)
+__device__ __forceinline__ void fxm_element(const int4 (&A)[9], int i, const int4 (&B)[9], int j, FxSum &re, FxSum &im) {
 #pragma unroll
-  for (int k = 0; k < 9; k++) {
-    r.ch[k] = u[k].x;
-    r.cl[k] = u[k].y;
-    r.mh[k] = u[k].z - u[k].x;
-    r.ml[k] = u[k].w - u[k].y;
-    r.ph[k] = u[k].x + u[k].z;
-    r.pl[k] = u[k].y + u[k].w;
-  }
-}
-// row i of A B
-__device__ __forceinline__ void fxm_row(const int4 (&A)[9], int i, const FxRight &B, s64 (&q)[6]) {
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    FxSum k1 = {0, 0}, k2 = {0, 0}, k3 = {0, 0};
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const int4 a = A[3 * i + k];
-      const int b = 3 * k + j;
-      fx_mac(k1, a.x + a.z, a.y + a.w, B.ch[b], B.cl[b]);
-      fx_mac(k2, a.x, a.y, B.mh[b], B.ml[b]);
-      fx_mac(k3, a.z, a.w, B.ph[b], B.pl[b]);
+  for (int k = 0; k < 3; k++) {
+    const int4 a = A[3 * i + k], b = B[3 * k + j];
+    if (k == 0) {
+      re.H = fx_mul(a.x, b.x);
+      re.M = fx_mul(a.x, b.y);
+      fx_mad(re.M, a.y, b.x);
+      im.H = fx_mul(a.x, b.z);
+      im.M = fx_mul(a.x, b.w);
+      fx_mad(im.M, a.y, b.z);
+    } else {
+      fx_mac(re, a.x, a.y, b.x, b.y);
+      fx_mac(im, a.x, a.y, b.z, b.w);
     }
-    q[2 * j] = (s64)((k1.H - k3.H) << 1) + ((s64)(k1.M - k3.M) >> 29);
-    q[2 * j + 1] = (s64)((k1.H + k2.H) << 1) + ((s64)(k1.M + k2.M) >> 29);
+    fx_mac(re, -a.z, -a.w, b.z, b.w);
+    fx_mac(im, a.z, a.w, b.x, b.y);
   }
 }
 
@@ -175,44 +186,46 @@ __device__ __forceinline__ void fxm_zero(FxSum9 &s) {
   for (int k = 0; k < 18; k++) s.q[k] = 0;
   s.E = 4 * FX_ZERO;
 }
+// exponent of a chain L (M R) of operands with these exponents; one with a
+// zero among them does not count
+__device__ __forceinline__ int fxm_exponent(int er, int em, int el) {
+  const int e = er + em + el + 5;
+  return e < FX_ZERO / 2 ? 4 * FX_ZERO : e;
+}
 
-// s += L (M R), or its adjoint; `right`: M R's right operand R
-__device__ __forceinline__ void fxm_add(FxSum9 &s, const int4 (&Lm)[9], const FxRight &X, int e, bool adj) {
-  if (e < FX_ZERO / 2) return;   // an operand is zero
-  const int up = e > s.E ? min(e - s.E, 63) : 0, dn = e > s.E ? 0 : min(s.E - e, 63);
-  s.E = max(e, s.E);
+// s += L X, or its adjoint, of exponent e <= s.E
+__device__ __forceinline__ void fxm_add(FxSum9 &s, const int4 (&Lm)[9], const int4 (&X)[9], int e, bool adj) {
+  const int dn = min(s.E - e, 63);
 #pragma unroll
-  for (int k = 0; k < 18; k++) s.q[k] >>= up;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    s64 q[6];
-    fxm_row(Lm, i, X, q);
+  for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      const s64 re = q[2 * j] >> dn, im = q[2 * j + 1] >> dn;
+      FxSum re, im;
+      fxm_element(Lm, i, X, j, re, im);
+      const s64 qr = ((s64)(re.H << 3) + ((s64)re.M >> 29)) >> dn;
+      const s64 qi = ((s64)(im.H << 3) + ((s64)im.M >> 29)) >> dn;
       if (adj) {
-        s.q[2 * (3 * j + i)] += re;
-        s.q[2 * (3 * j + i) + 1] -= im;
+        s.q[2 * (3 * j + i)] += qr;
+        s.q[2 * (3 * j + i) + 1] -= qi;
       } else {
-        s.q[2 * (3 * i + j)] += re;
-        s.q[2 * (3 * i + j) + 1] += im;
+        s.q[2 * (3 * i + j)] += qr;
+        s.q[2 * (3 * i + j) + 1] += qi;
       }
     }
-  }
 }
 
 // operand of a chain as doubles
-__device__ __forceinline__ M3<double> fxm_f64(const FxRef &r, int Vh) {
+__device__ __forceinline__ M3<double> fxm_f64(const FxRef &r) {
   M3<double> m;
   for (int k = 0; k < 9; k++) {
-    const int4 w = r.p[(size_t)(r.adj ? (k % 3) * 3 + k / 3 : k) * Vh];
+    const int4 w = r.p[32 * (r.adj ? (k % 3) * 3 + k / 3 : k)];
     double re = 0, im = 0;
     if (r.e == FX_SPECIAL) {
       re = __hiloint2double(w.x, w.y);
       im = __hiloint2double(w.z, w.w);
     } else if (r.e != FX_ZERO) {
-      re = fx_double(((s64)w.x << 32) + 4 * (s64)w.y, r.e);
-      im = fx_double(((s64)w.z << 32) + 4 * (s64)w.w, r.e);
+      re = fx_double(((s64)w.x << 32) + w.y, r.e);
+      im = fx_double(((s64)w.z << 32) + w.w, r.e);
     }
     m.e[k / 3][k % 3] = {re, r.adj ? -im : im};
   }
@@ -220,67 +233,83 @@ __device__ __forceinline__ M3<double> fxm_f64(const FxRef &r, int Vh) {
 }
 // chains [c0, c1) of `get` added up in plain FP64 (an operand is not finite)
 template <class Get>
-static __device__ __noinline__ void fxm_chains_f64(const Get &get, int c0, int c1, int Vh, M3<double> *out) {
+static __device__ __noinline__ void fxm_chains_f64(const Get &get, int c0, int c1, M3<double> *out) {
   M3<double> acc;
   for (int k = 0; k < 9; k++) acc.e[k / 3][k % 3] = {0.0, 0.0};
 #pragma unroll 1
   for (int c = c0; c < c1; c++) {
-    const M3<double> p = tnn<double>(fxm_f64(get(c, 2), Vh), tnn<double>(fxm_f64(get(c, 1), Vh), fxm_f64(get(c, 0), Vh)));
+    const M3<double> p = tnn<double>(fxm_f64(get(c, 2)), tnn<double>(fxm_f64(get(c, 1)), fxm_f64(get(c, 0))));
     tacc<double>(acc, get.adjoint(c) ? tadj<double>(p) : p, 1.0);
   }
   *out = acc;
 }
 
 // The chains [0, n) of `get`, the first n0 added into s0 and the others into
-// s1.  get(c, role): operand R, M, L of chain c for role 0, 1, 2.  Returns
-// true when an operand is not finite (the sums are then not to be used).
-template <class Get>
-__device__ __forceinline__ bool fxm_chains(const Get &get, int n, int n0, int Vh, FxRing &ring, FxSum9 &s0, FxSum9 &s1) {
+// s1.  get(c, role): operand R, M, L of chain c for role 0, 1, 2.  On return
+// the FP64 matrices at t0 and t1 (where given) are in the ring's slots 0 and
+// 1.  True when an operand is not finite (the sums are then not to be used).
+template <int n, int n0, class Get>
+__device__ __forceinline__ bool fxm_chains(const Get &get, int Vh, FxRing &ring, FxSum9 &s0, FxSum9 &s1,
+                                           const double2 *t0, const double2 *t1) {
   FxRef q[3];
   bool bad = false;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     q[k] = get(0, k);
-    fxm_fetch(ring, k, q[k], Vh);
+    fxm_fetch(ring, k, q[k]);
   }
   fxm_zero(s0);
   fxm_zero(s1);
+#pragma unroll
+  for (int c = 0; c < n; c++) {
+    int &E = c < n0 ? s0.E : s1.E;
+    E = max(E, fxm_exponent(get(c, 0).e, get(c, 1).e, get(c, 2).e));
+  }
 #pragma unroll 1
   for (int c = 0; c < n; c++) {
-    const int cn = c + 1 < n ? c + 1 : c;   // past the end: the last chain again, never used
-    int4 u[9];
-    FxRight X;
-    int e = q[0].e;
+    const bool last = c + 1 == n;
+    int4 u[9], X[9], v[9];
+    const int e = fxm_exponent(q[0].e, q[1].e, q[2].e);
     bad = bad || q[0].e == FX_SPECIAL || q[1].e == FX_SPECIAL || q[2].e == FX_SPECIAL;
-    fxm_take(ring, 0, q[0].adj, u);
-    fxm_right(u, X);
-    q[0] = get(cn, 0);
-    fxm_fetch(ring, 0, q[0], Vh);
-    e += q[1].e + 3;
+    fxm_take(ring, 0, q[0].adj, X);
+    if (!last) {
+      q[0] = get(c + 1, 0);
+      fxm_fetch(ring, 0, q[0]);
+    } else {
+      fxm_fetch_f64(ring, 0, t0, Vh);
+    }
     fxm_take(ring, 1, q[1].adj, u);
-    q[1] = get(cn, 1);
-    fxm_fetch(ring, 1, q[1], Vh);
-    int4 v[9];
+    if (!last) {
+      q[1] = get(c + 1, 1);
+      fxm_fetch(ring, 1, q[1]);
+    } else {
+      fxm_fetch_f64(ring, 1, t1, Vh);
+    }
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-      s64 w[6];
-      fxm_row(u, i, X, w);
+    for (int i = 0; i < 3; i++)
 #pragma unroll
       for (int j = 0; j < 3; j++) {
-        fxm_split(w[2 * j] + 2, v[3 * i + j].x, v[3 * i + j].y);
-        fxm_split(w[2 * j + 1] + 2, v[3 * i + j].z, v[3 * i + j].w);
+        FxSum re, im;
+        fxm_element(u, i, X, j, re, im);
+        fxm_split((s64)re.H + ((s64)re.M >> 32), v[3 * i + j].x, v[3 * i + j].y);
+        fxm_split((s64)im.H + ((s64)im.M >> 32), v[3 * i + j].z, v[3 * i + j].w);
       }
-    }
-    fxm_right(v, X);
-    e += q[2].e + 3;
     fxm_take(ring, 2, q[2].adj, u);
-    q[2] = get(cn, 2);
-    fxm_fetch(ring, 2, q[2], Vh);
-    if (c < n0) fxm_add(s0, u, X, e, get.adjoint(c));
-    else fxm_add(s1, u, X, e, get.adjoint(c));
+    const bool adj = get.adjoint(c);
+    if (!last) {
+      q[2] = get(c + 1, 2);
+      fxm_fetch(ring, 2, q[2]);
+    } else {
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (n0 == n || c < n0) fxm_add(s0, u, v, e, adj);
+    else fxm_add(s1, u, v, e, adj);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   return bad;
+}
+__device__ __forceinline__ double2 fxm_tail(const FxRing &ring, int slot, int k) {
+  return *reinterpret_cast<const double2 *>(&ring.v[slot][k][threadIdx.x]);
 }
 
 __device__ __forceinline__ double fxm_component(const FxSum9 &s, int k) {
@@ -301,12 +330,17 @@ struct FxStapleChains {
   __device__ __forceinline__ bool adjoint(int) const { return false; }
 };
 
-// S -> sout (integers) when sout.p, fat += coef S when fat.p
-static __global__ void __launch_bounds__(FXM_BLOCK) k_staple_fx(Geom g, int mu, int nu, FxMat U, FxMat A, MatF fat,
-                                                               double coef, FxMat sout) {
+// S -> sout (integers) when sout.p, fat += coef S when fat.p; mu = mu0 +
+// blockIdx.z, nu = mu + k
+static __global__ void __launch_bounds__(FXM_BLOCK, 5) k_staple_fx(Geom g, int mu0, int k1, FxMat L, FxMat Af,
+                                                                  MatD<double> fatf, double coef, FxMat soutf) {
   __shared__ FxRing ring;
   const int h = blockIdx.x * blockDim.x + threadIdx.x, par = blockIdx.y, Vh = g.Vh;
   if (h >= Vh) return;
+  const int mu = mu0 + blockIdx.z, nu = (mu + k1) & 3;
+  const FxMat U = fx_link_dir(L, nu, Vh), A = fx_link_dir(Af, mu, Vh), sout = fx_link_dir(soutf, mu, Vh);
+  const MatF fat = fatf.at(mu);
+  const bool keep = soutf.p != nullptr;
   FxStapleChains get;
   get.U = U;
   get.A = A;
@@ -317,18 +351,19 @@ static __global__ void __launch_bounds__(FXM_BLOCK) k_staple_fx(Geom g, int mu, 
   get.xmnu = nbr(g, par, h, nu, -1);
   get.xmnupmu = nbr2(g, par, h, nu, -1, mu, 1);
   FxSum9 s, none;
-  const bool bad = fxm_chains(get, 2, 2, Vh, ring, s, none);
+  double2 *f = fatf.p ? fat.p + par * fat.ps + h : nullptr;
+  const bool bad = fxm_chains<2, 2>(get, Vh, ring, s, none, f, nullptr);
   double2 v[9];
   int4 u[9];
   int e = FX_ZERO;
   if (bad) {
     M3<double> m;
-    fxm_chains_f64(get, 0, 2, Vh, &m);
+    fxm_chains_f64(get, 0, 2, &m);
 #pragma unroll
     for (int k = 0; k < 9; k++) v[k] = make_double2(m.e[k / 3][k % 3].re, m.e[k / 3][k % 3].im);
-    if (sout.p) fxm_encode(v, u, e);
+    if (keep) fxm_encode(v, u, e);
   } else {
-    if (sout.p) {
+    if (keep) {
       // normalised to |q| < 2^60: the exponents of a chain of three matrices
       // allow for 2^6 more than unitary ones reach, which a staple of a
       // staple would lose again
@@ -341,26 +376,26 @@ static __global__ void __launch_bounds__(FXM_BLOCK) k_staple_fx(Geom g, int mu, 
       for (int k = 0; k < 18; k++) s.q[k] = sh < 0 ? s.q[k] >> 1 : (s64)((u64)s.q[k] << sh);
 #pragma unroll
       for (int k = 0; k < 9; k++) {
-        fxm_split(s.q[2 * k] + 2, u[k].x, u[k].y);
-        fxm_split(s.q[2 * k + 1] + 2, u[k].z, u[k].w);
+        fxm_split(s.q[2 * k], u[k].x, u[k].y);
+        fxm_split(s.q[2 * k + 1], u[k].z, u[k].w);
       }
       s.E -= sh;
     }
-    if (fat.p) {
+    if (f) {
 #pragma unroll
       for (int k = 0; k < 9; k++) v[k] = make_double2(fxm_component(s, 2 * k), fxm_component(s, 2 * k + 1));
     }
   }
-  if (sout.p) {
+  if (keep) {
+    int4 *d = sout.at(par, h);
 #pragma unroll
-    for (int k = 0; k < 9; k++) sout.p[par * sout.ps + (size_t)k * Vh + h] = u[k];
+    for (int k = 0; k < 9; k++) d[32 * k] = u[k];
     sout.e[par * sout.es + h] = e;
   }
-  if (!fat.p) return;
-  double2 *f = fat.p + par * fat.ps + h;
+  if (!f) return;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    double2 a = f[(size_t)k * Vh];
+    double2 a = fxm_tail(ring, 0, k);
     a.x += coef * v[k].x;
     a.y += coef * v[k].y;
     f[(size_t)k * Vh] = a;
@@ -391,14 +426,19 @@ struct FxStapleAdjChains {
   __device__ __forceinline__ bool adjoint(int c) const { return c >= 4; }
 };
 
-// KA <- (init ? cinit init : KA) + f (its chains), KU += f (its chains); with
-// kout.p set KA goes there as integers instead of to its FP64 field
-static __global__ void __launch_bounds__(FXM_BLOCK) k_staple_adj_fx(Geom g, int mu, int nu, FxMat U, FxMat A, FxMat K,
-                                                                   double f, MatF init, double cinit, MatF KA,
-                                                                   FxMat kout, MatF KU) {
+// KA <- (init ? cinit init : KA) + f (its chains), KU_nu += f (its chains);
+// with kout.p set KA goes there as integers instead of to its FP64 field
+static __global__ void __launch_bounds__(FXM_BLOCK, 4) k_staple_adj_fx(Geom g, int mu0, int k1, FxMat L, FxMat Af,
+                                                                      FxMat Kf, double f, MatD<double> initf,
+                                                                      double cinit, MatD<double> KAf, FxMat koutf,
+                                                                      MatD<double> KUf) {
   __shared__ FxRing ring;
   const int h = blockIdx.x * blockDim.x + threadIdx.x, par = blockIdx.y, Vh = g.Vh;
   if (h >= Vh) return;
+  const int mu = mu0 + blockIdx.z, nu = (mu + k1) & 3;
+  const FxMat U = fx_link_dir(L, nu, Vh), A = fx_link_dir(Af, mu, Vh), K = fx_link_dir(Kf, mu, Vh);
+  const FxMat kout = fx_link_dir(koutf, mu, Vh);
+  const MatF KA = KAf.at(mu), KU = KUf.at(nu), init = initf.at(mu);
   FxStapleAdjChains get;
   get.U = U;
   get.A = A;
@@ -412,37 +452,37 @@ static __global__ void __launch_bounds__(FXM_BLOCK) k_staple_adj_fx(Geom g, int 
   get.ymnupmu = nbr2(g, par, h, nu, -1, mu, 1);
   get.ypnummu = nbr2(g, par, h, nu, 1, mu, -1);
   FxSum9 ka, ku;
-  const bool bad = fxm_chains(get, 6, 2, Vh, ring, ka, ku);
+  const MatF src = initf.p ? init : KA;
+  double2 *w = KU.p + par * KU.ps + h;
+  const bool bad = fxm_chains<6, 2>(get, Vh, ring, ka, ku, src.p + par * src.ps + h, w);
   M3<double> ma, mu_;
   if (bad) {
-    fxm_chains_f64(get, 0, 2, Vh, &ma);
-    fxm_chains_f64(get, 2, 6, Vh, &mu_);
+    fxm_chains_f64(get, 0, 2, &ma);
+    fxm_chains_f64(get, 2, 6, &mu_);
   }
   double2 v[9];
-  const MatF src = init.p ? init : KA;
-  const double c0 = init.p ? cinit : 1.0;
+  const double c0 = initf.p ? cinit : 1.0;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const double2 o = src.p[par * src.ps + (size_t)k * Vh + h];
+    const double2 o = fxm_tail(ring, 0, k);
     const double re = bad ? ma.e[k / 3][k % 3].re : fxm_component(ka, 2 * k);
     const double im = bad ? ma.e[k / 3][k % 3].im : fxm_component(ka, 2 * k + 1);
     v[k] = make_double2(c0 * o.x + f * re, c0 * o.y + f * im);
   }
-  if (kout.p) {
+  if (koutf.p) {
     int4 u[9];
     int e;
     fxm_encode(v, u, e);
 #pragma unroll
-    for (int k = 0; k < 9; k++) kout.p[par * kout.ps + (size_t)k * Vh + h] = u[k];
+    for (int k = 0; k < 9; k++) kout.at(par, h)[32 * k] = u[k];
     kout.e[par * kout.es + h] = e;
   } else {
 #pragma unroll
     for (int k = 0; k < 9; k++) KA.p[par * KA.ps + (size_t)k * Vh + h] = v[k];
   }
-  double2 *w = KU.p + par * KU.ps + h;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    double2 o = w[(size_t)k * Vh];
+    double2 o = fxm_tail(ring, 1, k);
     const double re = bad ? mu_.e[k / 3][k % 3].re : fxm_component(ku, 2 * k);
     const double im = bad ? mu_.e[k / 3][k % 3].im : fxm_component(ku, 2 * k + 1);
     o.x += f * re;

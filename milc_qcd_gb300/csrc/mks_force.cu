@@ -110,14 +110,16 @@ __global__ void __launch_bounds__(128) k_outer(Geom g, OuterArgs<R> a, typename 
 //   KA(y)    += U_nu(y-nu+mu)^dag K(y-nu) U_nu(y-nu) + U_nu(y+mu) K(y+nu) U_nu(y)^dag
 //   KUnu(y)  += A(y+nu) U_nu(y+mu)^dag K(y) + A(y-mu+nu)^dag U_nu(y-mu)^dag K(y-mu)^dag
 //             + K(y+nu)^dag U_nu(y+mu)^dag A(y)^dag + K(y+nu-mu) U_nu(y-mu)^dag A(y-mu)
-// Fields stored and products computed in precision R.
+// KA <- (init ? cinit init : KA) + f (...), KU_nu += f (...), for mu = mu0 +
+// blockIdx.z, nu = mu + k.  Fields stored and products computed in precision R.
 template <typename R>
-__global__ void __launch_bounds__(128) k_staple_adj(Geom g, int mu, int nu, MatT<R> Unu, MatT<R> A, MatT<R> K,
-                                                    double f, MatT<R> KA, MatT<R> KU) {
+__global__ void __launch_bounds__(128) k_staple_adj(Geom g, int mu0, int k, MatD<R> links, MatD<R> Af, MatD<R> Kf,
+                                                    double f, MatD<R> init, double cinit, MatD<R> KAf, MatD<R> KUf) {
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  const int par = blockIdx.y, op = 1 - par;
+  const int par = blockIdx.y, op = 1 - par, mu = mu0 + blockIdx.z, nu = (mu + k) & 3;
   const int Vh = g.Vh;
   if (h >= Vh) return;
+  const MatT<R> Unu = links.at(nu), A = Af.at(mu), K = Kf.at(mu), KA = KAf.at(mu), KU = KUf.at(nu);
   const int ymnu = nbr(g, par, h, nu, -1), ypnu = nbr(g, par, h, nu, 1), ypmu = nbr(g, par, h, mu, 1);
   const int ymmu = nbr(g, par, h, mu, -1);
   const int ymnupmu = nbr2(g, par, h, nu, -1, mu, 1), ypnummu = nbr2(g, par, h, nu, 1, mu, -1);
@@ -135,7 +137,17 @@ __global__ void __launch_bounds__(128) k_staple_adj(Geom g, int mu, int nu, MatT
     for (int i = 0; i < 3; i++)
 #pragma unroll
       for (int j = 0; j < 3; j++) { acc.e[i][j].re += t.e[i][j].re; acc.e[i][j].im += t.e[i][j].im; }
-    M3<R> out = KA.ld(par, h, Vh);
+    M3<R> out;
+    if (init.p) {
+      out = init.at(mu).ld(par, h, Vh);
+      const R c0 = (R)cinit;
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) { out.e[i][j].re *= c0; out.e[i][j].im *= c0; }
+    } else {
+      out = KA.ld(par, h, Vh);
+    }
     macc<R>(out, acc, fr);
     KA.st(par, h, Vh, out);
   }
@@ -312,92 +324,84 @@ template <typename R>
 struct ForceRun {
   typedef typename Stor<R>::t T2;
 
-  static int staple_fwd(int mu, int nu, MatT<R> Unu, MatT<R> A, MatT<R> S) {
+  // one staple level, or its reverse, for the directions mu0 .. mu0 + nb - 1
+  static int staple_fwd(int mu0, int nb, int k, MatD<R> U, MatD<R> A, MatD<R> S) {
     Context &c = ctx();
-    MatT<R> none = {nullptr, 0};
     timing_begin(MKS_K_FORCE);
-    k_staple<R><<<dim3(grid_for(c.Vh, 128), 2), 128, 0, c.stream>>>(c.geom, mu, nu, Unu, A, none, 0.0, S);
+    k_staple<R><<<dim3(grid_for(c.Vh, 128), 2, nb), 128, 0, c.stream>>>(c.geom, mu0, k, U, A, MatD<R>{nullptr, 0, 0},
+                                                                       0.0, S);
     timing_end(MKS_K_FORCE);
-    g_force_flops += 4.0 * 198 * c.V;
+    g_force_flops += nb * 4.0 * 198 * c.V;
+    MKS_CUDA(cudaGetLastError());
+    return MKS_OK;
+  }
+  static int staple_adj(int mu0, int nb, int k, MatD<R> U, MatD<R> A, MatD<R> K, double f, MatD<R> init, double cinit,
+                        MatD<R> KA, MatD<R>, MatD<R> KU) {
+    Context &c = ctx();
+    timing_begin(MKS_K_FORCE);
+    k_staple_adj<R><<<dim3(grid_for(c.Vh, 128), 2, nb), 128, 0, c.stream>>>(c.geom, mu0, k, U, A, K, f, init, cinit,
+                                                                           KA, KU);
+    timing_end(MKS_K_FORCE);
+    g_force_flops += nb * 12.0 * 198 * c.V;
+    MKS_CUDA(cudaGetLastError());
+    return MKS_OK;
+  }
+  // the same in integer arithmetic (FP64 fields)
+  static int staple_fwd(int mu0, int nb, int k, const FxMat &U, const FxMat &A, const FxMat &S) {
+    Context &c = ctx();
+    timing_begin(MKS_K_FORCE);
+    k_staple_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2, nb), FXM_BLOCK, 0, c.stream>>>(
+        c.geom, mu0, k, U, A, MatD<double>{nullptr, 0, 0}, 0.0, S);
+    timing_end(MKS_K_FORCE);
+    g_force_flops += nb * 4.0 * 198 * c.V;
+    MKS_CUDA(cudaGetLastError());
+    return MKS_OK;
+  }
+  static int staple_adj(int mu0, int nb, int k, const FxMat &U, const FxMat &A, const FxMat &K, double f,
+                        MatD<double> init, double cinit, MatD<double> KA, const FxMat &kout, MatD<double> KU) {
+    Context &c = ctx();
+    timing_begin(MKS_K_FORCE);
+    k_staple_adj_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2, nb), FXM_BLOCK, 0, c.stream>>>(c.geom, mu0, k, U, A, K, f,
+                                                                                     init, cinit, KA, kout, KU);
+    timing_end(MKS_K_FORCE);
+    g_force_flops += nb * 12.0 * 198 * c.V;
     MKS_CUDA(cudaGetLastError());
     return MKS_OK;
   }
 
-  static int staple_adj(int mu, int nu, MatT<R> Unu, MatT<R> A, MatT<R> K, double f, MatT<R> KA, MatT<R> KU) {
-    Context &c = ctx();
-    timing_begin(MKS_K_FORCE);
-    k_staple_adj<R><<<dim3(grid_for(c.Vh, 128), 2), 128, 0, c.stream>>>(c.geom, mu, nu, Unu, A, K, f, KA, KU);
-    timing_end(MKS_K_FORCE);
-    g_force_flops += 12.0 * 198 * c.V;
-    MKS_CUDA(cudaGetLastError());
-    return MKS_OK;
-  }
-
-  // FP64 fields: the staples and their reverse in integer arithmetic
-  static int staple_fwd_fx(int mu, int nu, const FxMat &U, const FxMat &A, const FxMat &S) {
-    Context &c = ctx();
-    const MatF none = {nullptr, 0};
-    timing_begin(MKS_K_FORCE);
-    k_staple_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2), FXM_BLOCK, 0, c.stream>>>(c.geom, mu, nu, U, A, none, 0.0, S);
-    timing_end(MKS_K_FORCE);
-    g_force_flops += 4.0 * 198 * c.V;
-    MKS_CUDA(cudaGetLastError());
-    return MKS_OK;
-  }
-  static int staple_adj_fx(int mu, int nu, const FxMat &U, const FxMat &A, const FxMat &K, double f, MatF init,
-                           double cinit, MatF KA, const FxMat &kout, MatF KU) {
-    Context &c = ctx();
-    timing_begin(MKS_K_FORCE);
-    k_staple_adj_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2), FXM_BLOCK, 0, c.stream>>>(c.geom, mu, nu, U, A, K, f, init,
-                                                                                 cinit, KA, kout, KU);
-    timing_end(MKS_K_FORCE);
-    g_force_flops += 12.0 * 198 * c.V;
-    MKS_CUDA(cudaGetLastError());
-    return MKS_OK;
-  }
-  // fat_adj on integers: links, Kfat and the staple fields once as integers;
-  // K2 leaves its kernel as integers, K1 with its last contribution
-  static int fat_adj_fx(double2 *links, const ForceCoeffs &cf, double2 *Kfat, double2 *KU, double2 *S1, double2 *S2,
-                        double2 *K1, double2 *K2) {
-    const size_t Vh = ctx().Vh;
-    FxMat L, K, fS1, fS2, fK1, fK2;
-    const FxMat off = {nullptr, nullptr, 0, 0};
-    const MatF none = {nullptr, 0}, mK1 = mat_field(K1, Vh);
-    MKS_TRY(ws_links_fxm("fxm_links", MKS_K_FORCE, links, &L));
-    MKS_TRY(ws_links_fxm("fxm_kfat", MKS_K_FORCE, Kfat, &K));
-    MKS_TRY(ws_fxm("fxm_s", 1, &fS1, S1));
-    MKS_TRY(ws_fxm("fxm_t", 1, &fS2, S2));
-    MKS_TRY(ws_fxm("fxm_k1", 1, &fK1));
-    MKS_TRY(ws_fxm("fxm_k2", 1, &fK2, K2));
-    for (int mu = 0; mu < 4; mu++) {
-      const MatF Kd = link_dir(Kfat, mu, Vh), KUm = link_dir(KU, mu, Vh);
-      const FxMat Km = fx_link_dir(K, mu, Vh), Um = fx_link_dir(L, mu, Vh);
-      for (int nu = 0; nu < 4; nu++) {
-        if (nu == mu) continue;
-        const FxMat Un = fx_link_dir(L, nu, Vh);
-        const MatF KUn = link_dir(KU, nu, Vh);
-        MKS_TRY(staple_fwd_fx(mu, nu, Un, Um, fS1));
-        bool first = true;   // K1's first contribution starts from c3 Kfat_mu
+  // Reverse of the staple recursion (load_fatlinks_cpu, ASQ_OPTIMIZED_
+  // FATTENING).  F: MatD or, in FP64, FxMat: there links, Kfat and the staple
+  // fields are integers, K2 leaves its kernel as integers and K1 with its last
+  // contribution (k1o); in FP32 k2 and k1o are the fields K2 and K1 themselves.
+  // KA: the adjoint of U_mu as the staples' start, one_link Kfat at first; KU
+  // that of the U_nu.  Two fields where one launch takes all four mu, whose
+  // KA_mu and KU_nu would meet.
+  template <class F>
+  static int staples_adj(const F &U, const F &K, const F &S1, const F &S2, const F &k2, const F &k1o, const F &none,
+                         MatD<R> Kd, MatD<R> K1, MatD<R> K2, MatD<R> KA, MatD<R> KU, const ForceCoeffs &cf) {
+    constexpr bool fx = sizeof(R) == 8;
+    const MatD<R> off = {nullptr, 0, 0};
+    const int nb = staple_batch(ctx().Vh);
+    for (int mu0 = 0; mu0 < 4; mu0 += nb)
+      for (int kn = 1; kn < 4; kn++) {
+        MKS_TRY(staple_fwd(mu0, nb, kn, U, U, S1));
+        MatD<R> start = Kd;   // K1 starts from c3 Kfat_mu
         if (cf.lepage != 0.0) {
-          MKS_TRY(staple_adj_fx(mu, nu, Un, fS1, Km, cf.lepage, Kd, cf.three_staple, mK1, off, KUn));
-          first = false;
+          MKS_TRY(staple_adj(mu0, nb, kn, U, S1, K, cf.lepage, start, cf.three_staple, K1, none, KU));
+          start = off;
         }
         int left = 2;
-        for (int rho = 0; rho < 4; rho++) {
-          if (rho == mu || rho == nu) continue;
-          const int sig = 6 - mu - nu - rho;
-          const FxMat Ur = fx_link_dir(L, rho, Vh), Us = fx_link_dir(L, sig, Vh);
-          MKS_TRY(staple_fwd_fx(mu, rho, Ur, fS1, fS2));
+        for (int kr = 1; kr < 4; kr++) {
+          if (kr == kn) continue;
+          MKS_TRY(staple_fwd(mu0, nb, kr, U, S1, S2));
           // K2 = c5 Kfat_mu + c7 (reverse of the sigma staple)
-          MKS_TRY(staple_adj_fx(mu, sig, Us, fS2, Km, cf.seven_staple, Kd, cf.five_staple, none, fK2,
-                                link_dir(KU, sig, Vh)));
-          MKS_TRY(staple_adj_fx(mu, rho, Ur, fS1, fK2, 1.0, first ? Kd : none, cf.three_staple, mK1,
-                                --left == 0 ? fK1 : off, link_dir(KU, rho, Vh)));
-          first = false;
+          MKS_TRY(staple_adj(mu0, nb, 6 - kn - kr, U, S2, K, cf.seven_staple, Kd, cf.five_staple, K2, k2, KU));
+          MKS_TRY(staple_adj(mu0, nb, kr, U, S1, k2, 1.0, start, cf.three_staple, K1,
+                             fx && --left == 0 ? k1o : none, KU));
+          start = off;
         }
-        MKS_TRY(staple_adj_fx(mu, nu, Un, Um, fK1, 1.0, none, 1.0, KUm, off, KUn));
+        MKS_TRY(staple_adj(mu0, nb, kn, U, U, k1o, 1.0, off, 1.0, KA, none, KU));
       }
-    }
     return MKS_OK;
   }
 
@@ -410,48 +414,43 @@ struct ForceRun {
     return MKS_OK;
   }
 
-  // reverse of the fat-link staple recursion (load_fatlinks_cpu, ASQ_OPTIMIZED_FATTENING):
   // KU += d fat(links) / d links contracted with Kfat
-  static int fat_adj(T2 *links, const ForceCoeffs &cf, T2 *Kfat, T2 *KU, T2 *S1, T2 *S2, T2 *K1, T2 *K2) {
-    const double one_link = cf.one_link - 6.0 * cf.lepage;
-    MKS_TRY(axpby(Kfat, KU, one_link, 1.0, 8 * 9 * ctx().Vh));
+  static int fat_adj(T2 *links, const ForceCoeffs &cf, T2 *Kfat, T2 *KU) {
+    const size_t Vh = ctx().Vh, nl = 8 * 9 * Vh;
+    MKS_TRY(axpby(Kfat, KU, cf.one_link - 6.0 * cf.lepage, 1.0, nl));
     if (cf.three_staple == 0.0 && cf.lepage == 0.0 && cf.five_staple == 0.0) return MKS_OK;
-    if constexpr (sizeof(R) == 8) return fat_adj_fx(links, cf, Kfat, KU, S1, S2, K1, K2);
-    else return fat_adj_direct(links, cf, Kfat, KU, S1, S2, K1, K2);
-  }
-  static int fat_adj_direct(T2 *links, const ForceCoeffs &cf, T2 *Kfat, T2 *KU, T2 *S1, T2 *S2, T2 *K1, T2 *K2) {
-    Context &c = ctx();
-    const size_t Vh = c.Vh, nm = 2 * 9 * Vh;
-    const MatT<R> mS1 = mat_field(S1, Vh), mS2 = mat_field(S2, Vh), mK1 = mat_field(K1, Vh), mK2 = mat_field(K2, Vh);
-    for (int mu = 0; mu < 4; mu++) {
-      const MatT<R> Kd = link_dir(Kfat, mu, Vh), Um = link_dir(links, mu, Vh), KUm = link_dir(KU, mu, Vh);
-      for (int nu = 0; nu < 4; nu++) {
-        if (nu == mu) continue;
-        const MatT<R> Un = link_dir(links, nu, Vh), KUn = link_dir(KU, nu, Vh);
-        MKS_TRY(staple_fwd(mu, nu, Un, Um, mS1));
-        // K1 = c3 Kfat_mu
-        MKS_CUDA(cudaMemsetAsync(K1, 0, nm * sizeof(T2), c.stream));
-        for (int p = 0; p < 2; p++)
-          MKS_TRY(axpby(Kd.p + p * Kd.ps, K1 + p * 9 * Vh, cf.three_staple, 1.0, 9 * Vh));
-        if (cf.lepage != 0.0) MKS_TRY(staple_adj(mu, nu, Un, mS1, Kd, cf.lepage, mK1, KUn));
-        for (int rho = 0; rho < 4; rho++) {
-          if (rho == mu || rho == nu) continue;
-          const MatT<R> Ur = link_dir(links, rho, Vh), KUr = link_dir(KU, rho, Vh);
-          MKS_TRY(staple_fwd(mu, rho, Ur, mS1, mS2));
-          MKS_CUDA(cudaMemsetAsync(K2, 0, nm * sizeof(T2), c.stream));
-          for (int p = 0; p < 2; p++)
-            MKS_TRY(axpby(Kd.p + p * Kd.ps, K2 + p * 9 * Vh, cf.five_staple, 1.0, 9 * Vh));
-          for (int sig = 0; sig < 4; sig++) {
-            if (sig == mu || sig == nu || sig == rho) continue;
-            const MatT<R> Us = link_dir(links, sig, Vh), KUs = link_dir(KU, sig, Vh);
-            MKS_TRY(staple_adj(mu, sig, Us, mS2, Kd, cf.seven_staple, mK2, KUs));
-          }
-          MKS_TRY(staple_adj(mu, rho, Ur, mS1, mK2, 1.0, mK1, KUr));
-        }
-        MKS_TRY(staple_adj(mu, nu, Un, Um, mK1, 1.0, KUm, KUn));
-      }
+    const int nd = staple_batch(Vh);
+    auto scratch = [&](const char *name, int mats, T2 **p) {
+      return ws(std::string("force_") + (sizeof(R) == 8 ? "64_" : "32_") + name, (size_t)mats * 18 * Vh * sizeof(T2),
+                (void **)p);
+    };
+    T2 *k1, *ka = KU;
+    MKS_TRY(scratch("k1", nd, &k1));
+    if (nd == 4) {
+      MKS_TRY(scratch("ka", 4, &ka));
+      MKS_CUDA(cudaMemsetAsync(ka, 0, nl * sizeof(T2), ctx().stream));
     }
-    return MKS_OK;
+    const MatD<R> Kd = mat_dirs(Kfat, Vh), K1 = mat_dirs(k1, Vh, nd), KA = mat_dirs(ka, Vh), KUd = mat_dirs(KU, Vh);
+    if constexpr (sizeof(R) == 8) {
+      FxMat L, K, S1, S2, fK1, fK2;
+      const FxMat none = {nullptr, nullptr, 0, 0, 1};
+      MKS_TRY(ws_links_fxm("fxm_links", MKS_K_FORCE, links, &L));
+      MKS_TRY(ws_links_fxm("fxm_kfat", MKS_K_FORCE, Kfat, &K));
+      MKS_TRY(ws_fxm("fxm_s", nd, &S1));
+      MKS_TRY(ws_fxm("fxm_t", nd, &S2));
+      MKS_TRY(ws_fxm("fxm_k1", nd, &fK1));
+      MKS_TRY(ws_fxm("fxm_k2", nd, &fK2));
+      MKS_TRY(staples_adj(L, K, S1, S2, fK2, fK1, none, Kd, K1, MatD<R>{nullptr, 0, 0}, KA, KUd, cf));
+    } else {
+      T2 *s1, *s2, *k2;
+      MKS_TRY(scratch("s1", nd, &s1));
+      MKS_TRY(scratch("s2", nd, &s2));
+      MKS_TRY(scratch("k2", nd, &k2));
+      const MatD<R> K2 = mat_dirs(k2, Vh, nd), none = {nullptr, 0, 0};
+      MKS_TRY(staples_adj(mat_dirs(links, Vh), Kd, mat_dirs(s1, Vh, nd), mat_dirs(s2, Vh, nd), K2, K1, none, Kd, K1,
+                          K2, KA, KUd, cf));
+    }
+    return ka == KU ? MKS_OK : axpby(ka, KU, 1.0, 1.0, nl);
   }
 
   static int naik_adj(const T2 *W, const T2 *Kl, T2 *KW, double cn) {
@@ -538,19 +537,18 @@ struct ForceRun {
   static int hisq(double eps, const double *residues, double2 *const *xs, int nterms, const int *orders, int n_naiks,
                   double *mom_dev, double2 *ku_out, T2 *const *xr = nullptr) {
     Context &c = ctx();
-    const size_t Vh = c.Vh, nl = 8 * 9 * Vh, nm = 2 * 9 * Vh;
+    const size_t Vh = c.Vh, nl = 8 * 9 * Vh;
     const ForceCoeffs c1 = {1.0 / 8.0, 0.0, -1.0 / 16.0, 1.0 / 64.0, -1.0 / 384.0, 0.0};
     const ForceCoeffs c2 = {1.0 / 8.0 + 2.0 * 6.0 / 16.0 + 1.0 / 8.0, -1.0 / 24.0, -1.0 / 16.0, 1.0 / 64.0,
                             -1.0 / 384.0, -2.0 / 16.0};
     const ForceCoeffs c3 = {1.0 / 8.0, -1.0 / 24.0, 0, 0, 0, 0};
     const bool low = sizeof(R) < 8;
-    // Kf Kl KW KV KU, S1 S2 K1 K2, and in FP32 the U and W copies and the inputs
-    const size_t total = 5 * nl + 4 * nm + (low ? 2 * nl + (xr ? 0 : (size_t)nterms * 6 * Vh) : 0);
+    // Kf Kl KW KV KU, and in FP32 the U and W copies and the inputs
+    const size_t total = 5 * nl + (low ? 2 * nl + (xr ? 0 : (size_t)nterms * 6 * Vh) : 0);
     T2 *buf = nullptr;
     MKS_TRY(dev_alloc((void **)&buf, total * sizeof(T2)));
     T2 *Kf = buf, *Kl = Kf + nl, *KW = Kl + nl, *KV = KW + nl, *KU = KV + nl;
-    T2 *S1 = KU + nl, *S2 = S1 + nm, *K1 = S2 + nm, *K2 = K1 + nm;
-    T2 *Ucp = K2 + nm, *Wcp = Ucp + nl, *xs32 = Wcp + nl;
+    T2 *Ucp = KU + nl, *Wcp = Ucp + nl, *xs32 = Wcp + nl;
     unsigned int *nfilt = nullptr;
     int rc = MKS_OK;
     do {
@@ -571,7 +569,7 @@ struct ForceRun {
       // level 2 with every term (the Naik group-0 table covers all terms)
       oa.j0 = 0; oa.j1 = nterms; oa.scale = 1.0;
       if ((rc = outer(oa, Kf, Kl)) < 0) break;
-      if ((rc = fat_adj(W, c2, Kf, KW, S1, S2, K1, K2)) < 0) break;
+      if ((rc = fat_adj(W, c2, Kf, KW)) < 0) break;
       if ((rc = naik_adj(W, Kl, KW, c2.naik)) < 0) break;
       // Naik-epsilon groups: eps_g (1-link + Naik)(W) for their own terms
       int off = orders[0];
@@ -580,7 +578,7 @@ struct ForceRun {
         oa.j0 = off; oa.j1 = off + orders[gi]; oa.scale = c.slots[gi].eps_naik;
         off += orders[gi];
         if ((rc = outer(oa, Kf, Kl)) < 0) break;
-        if ((rc = fat_adj(W, c3, Kf, KW, S1, S2, K1, K2)) < 0) break;
+        if ((rc = fat_adj(W, c3, Kf, KW)) < 0) break;
         if ((rc = naik_adj(W, Kl, KW, c3.naik)) < 0) break;
       }
       if (rc < 0) break;
@@ -589,7 +587,7 @@ struct ForceRun {
       timing_end(MKS_K_FORCE);
       g_force_flops += 20.0 * 198 * c.V * 4;
       if (cudaGetLastError() != cudaSuccess) { rc = MKS_ERR_CUDA; break; }
-      if ((rc = fat_adj(U, c1, KV, KU, S1, S2, K1, K2)) < 0) break;
+      if ((rc = fat_adj(U, c1, KV, KU)) < 0) break;
       if ((rc = finish(eps, KU, mom_dev, ku_out, nullptr)) < 0) break;
       cudaMemcpyAsync(&g_nfilter, nfilt, sizeof(unsigned int), cudaMemcpyDeviceToHost, c.stream);
       if (cudaStreamSynchronize(c.stream) != cudaSuccess) rc = MKS_ERR_CUDA;
@@ -606,19 +604,18 @@ struct ForceRun {
   static int asqtad(double eps, const double *residues, double2 *const *xs, int nterms, double *mom_dev,
                     double2 *ku_out) {
     Context &c = ctx();
-    const size_t Vh = c.Vh, nl = 8 * 9 * Vh, nm = 2 * 9 * Vh;
+    const size_t Vh = c.Vh, nl = 8 * 9 * Vh;
     g_nfilter = 0;
     const double u2 = c.aux_u0 * c.aux_u0, u4 = u2 * u2, u6 = u4 * u2;
     // asqtad_action.h with the tadpole division of ks_action_paths.c
     const ForceCoeffs ca = {1.0 / 8.0 + 6.0 / 16.0 + 1.0 / 8.0, -1.0 / 24.0 / u2, -1.0 / 16.0 / u2, 1.0 / 64.0 / u4,
                             -1.0 / 384.0 / u6, -1.0 / 16.0 / u4};
     const bool low = sizeof(R) < 8;
-    const size_t total = 3 * nl + 4 * nm + (low ? nl + (size_t)nterms * 6 * Vh : 0);
+    const size_t total = 3 * nl + (low ? nl + (size_t)nterms * 6 * Vh : 0);
     T2 *buf = nullptr;
     MKS_TRY(dev_alloc((void **)&buf, total * sizeof(T2)));
     T2 *Kf = buf, *Kl = Kf + nl, *KU = Kl + nl;
-    T2 *S1 = KU + nl, *S2 = S1 + nm, *K1 = S2 + nm, *K2 = K1 + nm;
-    T2 *Ucp = K2 + nm, *xs32 = Ucp + nl;
+    T2 *Ucp = KU + nl, *xs32 = Ucp + nl;
     int rc = MKS_OK;
     do {
       if (cudaMemsetAsync(buf, 0, 3 * nl * sizeof(T2), c.stream) != cudaSuccess) { rc = MKS_ERR_CUDA; break; }
@@ -630,7 +627,7 @@ struct ForceRun {
       for (int j = 0; j < nterms; j++) oa.res[j] = residues[j];
       oa.j0 = 0; oa.j1 = nterms; oa.scale = 1.0;
       if ((rc = outer(oa, Kf, Kl)) < 0) break;
-      if ((rc = fat_adj(U, ca, Kf, KU, S1, S2, K1, K2)) < 0) break;
+      if ((rc = fat_adj(U, ca, Kf, KU)) < 0) break;
       if ((rc = naik_adj(U, Kl, KU, ca.naik)) < 0) break;
       rc = finish(eps, KU, mom_dev, ku_out, nullptr);
     } while (0);

@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(128) k_unitarize(Geom g, const typename Stor<R
   if (Wr) link_dir(Wr, mu, g.Vh).st(par, h, g.Vh, w);
 }
 
+typedef MatD<double> MatF64D;
 struct FatCoeffs { double one_link, naik, three_staple, five_staple, seven_staple, lepage; };
 
 // the smearing stages with fields stored and multiplied in precision R
@@ -149,28 +150,46 @@ template <typename R>
 struct Smear {
   typedef typename Stor<R>::t T2;
 
-  static int launch_staple(int mu, int nu, MatT<R> Unu, MatT<R> A, MatT<R> fat, double coef, MatT<R> sout) {
+  // one staple level for the directions mu0 .. mu0 + nb - 1 (staple_batch)
+  static int staple(int mu0, int nb, int k, MatD<R> U, MatD<R> A, MatD<R> fat, double coef, MatD<R> sout) {
     Context &c = ctx();
     timing_begin(MKS_K_LINKS);
-    k_staple<R><<<dim3(grid_for(c.Vh, 128), 2), 128, 0, c.stream>>>(c.geom, mu, nu, Unu, A, fat, coef, sout);
+    k_staple<R><<<dim3(grid_for(c.Vh, 128), 2, nb), 128, 0, c.stream>>>(c.geom, mu0, k, U, A, fat, coef, sout);
     timing_end(MKS_K_LINKS);
     MKS_CUDA(cudaGetLastError());
     return MKS_OK;
   }
-
-  // the staples in integer arithmetic (FP64 fields): the links and the staple
-  // fields S, T as integers, fat links accumulated in FP64
-  static int staple_fx(int mu, int nu, const FxMat &U, const FxMat &A, MatF fat, double coef, const FxMat &sout) {
+  // the same in integer arithmetic (FP64 fields): the links and the staple
+  // fields as integers, fat links accumulated in FP64
+  static int staple(int mu0, int nb, int k, const FxMat &U, const FxMat &A, MatF64D fat, double coef,
+                    const FxMat &sout) {
     Context &c = ctx();
     timing_begin(MKS_K_LINKS);
-    k_staple_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2), FXM_BLOCK, 0, c.stream>>>(c.geom, mu, nu, U, A, fat, coef, sout);
+    k_staple_fx<<<dim3(grid_for(c.Vh, FXM_BLOCK), 2, nb), FXM_BLOCK, 0, c.stream>>>(c.geom, mu0, k, U, A, fat, coef,
+                                                                                   sout);
     timing_end(MKS_K_LINKS);
     MKS_CUDA(cudaGetLastError());
     return MKS_OK;
   }
+  // load_fatlinks_cpu, ASQ_OPTIMIZED_FATTENING (fermion_links_fn_load_milc.c:
+  // 207-253): nu, rho, sigma = mu + 1, 2, 3 in every order.  F: MatD or FxMat
+  template <class F>
+  static int staples(const F &U, const F &S, const F &T, const F &none, const FatCoeffs &cf, MatD<R> fat) {
+    const int nb = staple_batch(ctx().Vh);
+    for (int mu0 = 0; mu0 < 4; mu0 += nb)
+      for (int kn = 1; kn < 4; kn++) {
+        MKS_TRY(staple(mu0, nb, kn, U, U, fat, cf.three_staple, S));
+        if (cf.lepage != 0.0) MKS_TRY(staple(mu0, nb, kn, U, S, fat, cf.lepage, none));
+        for (int kr = 1; kr < 4; kr++) {
+          if (kr == kn) continue;
+          MKS_TRY(staple(mu0, nb, kr, U, S, fat, cf.five_staple, T));
+          MKS_TRY(staple(mu0, nb, 6 - kn - kr, U, T, fat, cf.seven_staple, none));
+        }
+      }
+    return MKS_OK;
+  }
 
-  // load_fatlinks_cpu, ASQ_OPTIMIZED_FATTENING (fermion_links_fn_load_milc.c:207-253)
-  static int fatten(T2 *links, const FatCoeffs &cf, T2 *fat, T2 *staple, T2 *tmp) {
+  static int fatten(T2 *links, const FatCoeffs &cf, T2 *fat) {
     Context &c = ctx();
     size_t Vh = c.Vh, nall = 8 * 9 * Vh;
     double one_link = cf.one_link - 6.0 * cf.lepage;
@@ -179,54 +198,22 @@ struct Smear {
     timing_end(MKS_K_LINKS);
     MKS_CUDA(cudaGetLastError());
     if (cf.three_staple == 0.0 && cf.lepage == 0.0 && cf.five_staple == 0.0) return MKS_OK;
+    const int nd = staple_batch(Vh);
     if constexpr (sizeof(R) == 8) {
       FxMat L, S, T;
-      const FxMat off = {nullptr, nullptr, 0, 0};
+      const FxMat none = {nullptr, nullptr, 0, 0, 1};
       MKS_TRY(ws_links_fxm("fxm_links", MKS_K_LINKS, links, &L));
-      MKS_TRY(ws_fxm("fxm_s", 1, &S, staple));
-      MKS_TRY(ws_fxm("fxm_t", 1, &T, tmp));
-      for (int mu = 0; mu < 4; mu++) {
-        const MatF Fm = link_dir(fat, mu, Vh);
-        const FxMat Um = fx_link_dir(L, mu, Vh);
-        for (int nu = 0; nu < 4; nu++) {
-          if (nu == mu) continue;
-          const FxMat Un = fx_link_dir(L, nu, Vh);
-          MKS_TRY(staple_fx(mu, nu, Un, Um, Fm, cf.three_staple, S));
-          if (cf.lepage != 0.0) MKS_TRY(staple_fx(mu, nu, Un, S, Fm, cf.lepage, off));
-          for (int rho = 0; rho < 4; rho++) {
-            if (rho == mu || rho == nu) continue;
-            MKS_TRY(staple_fx(mu, rho, fx_link_dir(L, rho, Vh), S, Fm, cf.five_staple, T));
-            for (int sig = 0; sig < 4; sig++) {
-              if (sig == mu || sig == nu || sig == rho) continue;
-              MKS_TRY(staple_fx(mu, sig, fx_link_dir(L, sig, Vh), T, Fm, cf.seven_staple, off));
-            }
-          }
-        }
-      }
+      MKS_TRY(ws_fxm("fxm_s", nd, &S));
+      MKS_TRY(ws_fxm("fxm_t", nd, &T));
+      return staples(L, S, T, none, cf, mat_dirs(fat, Vh));
     } else {
-      MatT<R> none = {nullptr, 0};
-      for (int mu = 0; mu < 4; mu++) {
-        MatT<R> Fm = link_dir(fat, mu, Vh), Um = link_dir(links, mu, Vh);
-        for (int nu = 0; nu < 4; nu++) {
-          if (nu == mu) continue;
-          MatT<R> Un = link_dir(links, nu, Vh);
-          MatT<R> S = mat_field(staple, Vh), T = mat_field(tmp, Vh);
-          MKS_TRY(launch_staple(mu, nu, Un, Um, Fm, cf.three_staple, S));
-          if (cf.lepage != 0.0) MKS_TRY(launch_staple(mu, nu, Un, S, Fm, cf.lepage, none));
-          for (int rho = 0; rho < 4; rho++) {
-            if (rho == mu || rho == nu) continue;
-            MatT<R> Ur = link_dir(links, rho, Vh);
-            MKS_TRY(launch_staple(mu, rho, Ur, S, Fm, cf.five_staple, T));
-            for (int sig = 0; sig < 4; sig++) {
-              if (sig == mu || sig == nu || sig == rho) continue;
-              MatT<R> Us = link_dir(links, sig, Vh);
-              MKS_TRY(launch_staple(mu, sig, Us, T, Fm, cf.seven_staple, none));
-            }
-          }
-        }
+      T2 *st[2];
+      for (int k = 0; k < 2; k++)
+        MKS_TRY(ws("staple" + std::to_string(k), (size_t)nd * 18 * Vh * sizeof(T2), (void **)&st[k]));
+      const MatD<R> none = {nullptr, 0, 0};
+      return staples(mat_dirs(links, Vh), mat_dirs(st[0], Vh, nd), mat_dirs(st[1], Vh, nd), none, cf,
+                     mat_dirs(fat, Vh));
     }
-    }
-    return MKS_OK;
   }
 
   static int naik(T2 *W, T2 *lng, double coef) {
@@ -258,9 +245,7 @@ struct Smear {
 };
 
 // the FP64 entry points of the MILC-facing loaders
-static int fatten(double2 *links, const FatCoeffs &cf, double2 *fat, double2 *staple, double2 *tmp) {
-  return Smear<double>::fatten(links, cf, fat, staple, tmp);
-}
+static int fatten(double2 *links, const FatCoeffs &cf, double2 *fat) { return Smear<double>::fatten(links, cf, fat); }
 static int naik(double2 *W, double2 *lng, double coef) { return Smear<double>::naik(W, lng, coef); }
 
 static unsigned int g_nsvd = 0;
@@ -293,11 +278,11 @@ static int build_links(int action, int n_naiks, const double *eps_naik, double u
       MKS_TRY(dev_alloc((void **)&s.lng64, nall * sizeof(double2)));
     }
   }
-  // staple, tmp; FP32: U, V, W, fat, long copies; Naik groups: f3, l3
-  const size_t nscr = 2 * 2 * 9 * Vh + (low ? 5 * nall : 0) + (n_naiks > 1 ? 2 * nall : 0);
+  // FP32: U, V, W, fat, long copies; Naik groups: f3, l3
+  const size_t nscr = (low ? 5 * nall : 0) + (n_naiks > 1 ? 2 * nall : 0);
   T2 *scr = nullptr;
   MKS_TRY(dev_alloc((void **)&scr, nscr * sizeof(T2)));
-  T2 *staple = scr, *tmp = staple + 2 * 9 * Vh, *p = tmp + 2 * 9 * Vh;
+  T2 *p = scr;
   T2 *Ucp = nullptr, *Vcp = nullptr, *Wcp = nullptr, *Fcp = nullptr, *Lcp = nullptr, *f3 = nullptr, *l3 = nullptr;
   if (low) { Ucp = p; Vcp = p + nall; Wcp = p + 2 * nall; Fcp = p + 3 * nall; Lcp = p + 4 * nall; p += 5 * nall; }
   if (n_naiks > 1) { f3 = p; l3 = p + nall; }
@@ -323,12 +308,12 @@ static int build_links(int action, int n_naiks, const double *eps_naik, double u
                             -1.0 / 384.0, -2.0 / 16.0};
       const FatCoeffs c3 = {1.0 / 8.0, -1.0 / 24.0, 0, 0, 0, 0};
       T2 *Vf = low ? Vcp : (T2 *)c.auxV, *W = low ? Wcp : (T2 *)c.auxW;
-      if ((rc = Sm::fatten(U, c1, Vf, staple, tmp)) < 0) break;
+      if ((rc = Sm::fatten(U, c1, Vf)) < 0) break;
       if ((rc = Sm::unitarize(Vf, low ? c.auxV : nullptr, c.auxW, low ? Wcp : nullptr, nsvd)) < 0) break;
-      if ((rc = Sm::fatten(W, c2, F, staple, tmp)) < 0) break;
+      if ((rc = Sm::fatten(W, c2, F)) < 0) break;
       if ((rc = Sm::naik(W, L, c2.naik)) < 0) break;
       if (n_naiks > 1) {
-        if ((rc = Sm::fatten(W, c3, f3, staple, tmp)) < 0) break;
+        if ((rc = Sm::fatten(W, c3, f3)) < 0) break;
         if ((rc = Sm::naik(W, l3, c3.naik)) < 0) break;
         for (int i = 1; i < n_naiks; i++) {
           LinkSlot &s = c.slots[i];
@@ -342,7 +327,7 @@ static int build_links(int action, int n_naiks, const double *eps_naik, double u
       const double u2 = u0 * u0, u4 = u2 * u2, u6 = u4 * u2;
       const FatCoeffs ca = {1.0 / 8.0 + 6.0 / 16.0 + 1.0 / 8.0, -1.0 / 24.0 / u2, -1.0 / 16.0 / u2, 1.0 / 64.0 / u4,
                             -1.0 / 384.0 / u6, -1.0 / 16.0 / u4};
-      if ((rc = Sm::fatten(U, ca, F, staple, tmp)) < 0) break;
+      if ((rc = Sm::fatten(U, ca, F)) < 0) break;
       if ((rc = Sm::naik(U, L, ca.naik)) < 0) break;
       n_naiks = 1;
     }
@@ -465,21 +450,19 @@ int mks_fatlong_links(const double coeffs[6], const double *links, double *fat, 
   const size_t Vh = c.Vh, nall = 8 * 9 * Vh, bytes = c.V * 72 * sizeof(double);
   const FatCoeffs cf = {coeffs[0], coeffs[1], coeffs[2], coeffs[3], coeffs[4], coeffs[5]};
   double *stage = nullptr;
-  double2 *L = nullptr, *F = nullptr, *S = nullptr, *T = nullptr;
+  double2 *L = nullptr, *F = nullptr;
   int rc = dev_alloc((void **)&stage, bytes);
   if (rc >= 0) rc = dev_alloc((void **)&L, nall * sizeof(double2));
   if (rc >= 0) rc = dev_alloc((void **)&F, nall * sizeof(double2));
-  if (rc >= 0) rc = dev_alloc((void **)&S, 2 * 9 * Vh * sizeof(double2));
-  if (rc >= 0) rc = dev_alloc((void **)&T, 2 * 9 * Vh * sizeof(double2));
   if (rc >= 0 && cudaMemcpyAsync(stage, links, bytes, cudaMemcpyHostToDevice, c.stream) != cudaSuccess)
     rc = MKS_ERR_CUDA;
   if (rc >= 0) rc = links_aos_to_soa64(stage, L);
-  if (rc >= 0 && fat) rc = fatten(L, cf, F, S, T);
+  if (rc >= 0 && fat) rc = fatten(L, cf, F);
   if (rc >= 0 && fat) rc = to_host(F, fat, stage);
   if (rc >= 0 && lng) rc = naik(L, F, cf.naik);
   if (rc >= 0 && lng) rc = to_host(F, lng, stage);
   cudaStreamSynchronize(c.stream);
-  dev_free(stage); dev_free(L); dev_free(F); dev_free(S); dev_free(T);
+  dev_free(stage); dev_free(L); dev_free(F);
   return rc;
 }
 
@@ -487,15 +470,12 @@ int mks_hisq_aux_links(const double coeffs1[6], const double *U, double *V, doub
   MKS_TRY(check_ready());
   if (!coeffs1 || !U) return MKS_ERR_ARG;
   Context &c = ctx();
-  const size_t Vh = c.Vh, bytes = c.V * 72 * sizeof(double);
+  const size_t bytes = c.V * 72 * sizeof(double);
   const FatCoeffs cf = {coeffs1[0], coeffs1[1], coeffs1[2], coeffs1[3], coeffs1[4], coeffs1[5]};
   MKS_TRY(ensure_aux());
   double *stage = nullptr;
-  double2 *S = nullptr, *T = nullptr;
   unsigned int *nsvd = nullptr;
   int rc = dev_alloc((void **)&stage, bytes);
-  if (rc >= 0) rc = dev_alloc((void **)&S, 2 * 9 * Vh * sizeof(double2));
-  if (rc >= 0) rc = dev_alloc((void **)&T, 2 * 9 * Vh * sizeof(double2));
   if (rc >= 0) rc = dev_alloc((void **)&nsvd, sizeof(unsigned int));
   if (rc >= 0 && cudaMemsetAsync(nsvd, 0, sizeof(unsigned int), c.stream) != cudaSuccess) rc = MKS_ERR_CUDA;
   if (rc >= 0 && cudaMemcpyAsync(stage, U, bytes, cudaMemcpyHostToDevice, c.stream) != cudaSuccess)
@@ -503,14 +483,14 @@ int mks_hisq_aux_links(const double coeffs1[6], const double *U, double *V, doub
   if (rc >= 0) rc = links_aos_to_soa64(stage, c.auxU);
   c.aux_action = MKS_ACTION_HISQ;
   c.aux_u0 = 1.0;
-  if (rc >= 0) rc = fatten(c.auxU, cf, c.auxV, S, T);
+  if (rc >= 0) rc = fatten(c.auxU, cf, c.auxV);
   if (rc >= 0) rc = Smear<double>::unitarize(c.auxV, nullptr, c.auxW, nullptr, nsvd);
   if (rc >= 0 && cudaMemcpyAsync(&g_nsvd, nsvd, sizeof(unsigned int), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess)
     rc = MKS_ERR_CUDA;
   if (rc >= 0 && V) rc = to_host(c.auxV, V, stage);
   if (rc >= 0 && W) rc = to_host(c.auxW, W, stage);
   cudaStreamSynchronize(c.stream);
-  dev_free(stage); dev_free(S); dev_free(T); dev_free(nsvd);
+  dev_free(stage); dev_free(nsvd);
   return rc;
 }
 

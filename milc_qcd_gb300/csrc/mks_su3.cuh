@@ -43,6 +43,30 @@ __host__ __device__ inline MatT<float> link_dir(float2 *base, int dir, size_t Vh
 __host__ __device__ inline MatT<double> mat_field(double2 *base, size_t Vh) { return {base, 9 * Vh}; }
 __host__ __device__ inline MatT<float> mat_field(float2 *base, size_t Vh) { return {base, 9 * Vh}; }
 
+// a field with one matrix per direction, [par][4][9][Vh], or a scratch field
+// whose one matrix per site every direction uses (ds = 0)
+template <typename R>
+struct MatD {
+  typename Stor<R>::t *p;
+  size_t ps, ds;
+  __device__ __forceinline__ MatT<R> at(int dir) const { return {p + dir * ds, ps}; }
+};
+template <typename T2> struct RealOf;
+template <> struct RealOf<double2> { typedef double t; };
+template <> struct RealOf<float2> { typedef float t; };
+template <typename T2> inline MatD<typename RealOf<T2>::t> mat_dirs(T2 *p, size_t Vh, int nd = 4) {
+  return {p, (size_t)nd * 9 * Vh, nd == 4 ? 9 * Vh : 0};
+}
+
+// How many directions mu one launch of the staple kernels takes (blockIdx.z):
+// the staples of the four mu do not depend on each other, and with nu, rho and
+// sigma at fixed distances from mu no two of them write to one direction.  One
+// launch for all four on lattices where a launch is short (12x14x10x20 in FP32,
+// links and force: 420 launches and 4.6 ms one by one); beyond a million sites
+// of a parity it gains nothing and its four scratch matrices per site are
+// memory that the largest lattices need.
+inline int staple_batch(size_t Vh) { return Vh <= ((size_t)1 << 20) ? 4 : 1; }
+
 // y = a x + b y, and precision conversions, over n complex numbers
 template <typename T2>
 __global__ void k_axpby_t(const T2 *x, T2 *y, double a, double b, size_t n) {
@@ -229,16 +253,17 @@ __device__ __forceinline__ int nbr2(const Geom &g, int par, int h, int mu, int d
 }
 
 // generalised staple S(x) = U_nu(x) A(x+nu) U_nu(x+mu)^dag + U_nu(x-nu)^dag A(x-nu) U_nu(x-nu+mu)
-// (generic/general_staple.c:42-140): S saved when sout.p != nullptr, and
-// fat_mu(x) += coef * S(x) when fat.p != nullptr; fields stored and
-// products computed in precision R
+// (generic/general_staple.c:42-140) for mu = mu0 + blockIdx.z, nu = mu + k: S
+// saved when sout.p != nullptr, and fat_mu(x) += coef * S(x) when fat.p !=
+// nullptr; fields stored and products computed in precision R
 template <typename R>
-static __global__ void __launch_bounds__(128) k_staple(Geom g, int mu, int nu, MatT<R> Unu, MatT<R> A, MatT<R> fat,
-                                                       double coef, MatT<R> sout) {
+static __global__ void __launch_bounds__(128) k_staple(Geom g, int mu0, int k, MatD<R> links, MatD<R> Af, MatD<R> fatf,
+                                                       double coef, MatD<R> soutf) {
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  const int par = blockIdx.y, opar = 1 - par;
+  const int par = blockIdx.y, opar = 1 - par, mu = mu0 + blockIdx.z, nu = (mu + k) & 3;
   const int Vh = g.Vh;
   if (h >= Vh) return;
+  const MatT<R> Unu = links.at(nu), A = Af.at(mu);
   const int xpnu = nbr(g, par, h, nu, 1), xpmu = nbr(g, par, h, mu, 1), xmnu = nbr(g, par, h, nu, -1);
   const int xmnupmu = nbr2(g, par, h, nu, -1, mu, 1);
   // upper: U_nu(x) [A(x+nu) U_nu(x+mu)^dag]
@@ -250,8 +275,9 @@ static __global__ void __launch_bounds__(128) k_staple(Geom g, int mu, int nu, M
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) s.e[i][j] = {up.e[i][j].re + dn.e[i][j].re, up.e[i][j].im + dn.e[i][j].im};
-  if (sout.p) sout.st(par, h, Vh, s);
-  if (!fat.p) return;
+  if (soutf.p) soutf.at(mu).st(par, h, Vh, s);
+  if (!fatf.p) return;
+  const MatT<R> fat = fatf.at(mu);
   M3<R> f = fat.ld(par, h, Vh);
   const R c = (R)coef;
 #pragma unroll
