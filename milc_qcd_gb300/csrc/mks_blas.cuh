@@ -2,9 +2,8 @@
 //
 // k_site<Op, NSUM, Fin> runs Op on every checkerboard site of one source
 // per blockIdx.y, accumulates NSUM FP64 sums, reduces them
-// deterministically (grid_reduce_last: per-block rows summed in a fixed
-// order) and lets the block that ends the reduction run the finisher Fin,
-// which updates the solver scalars held in device memory.
+// deterministically (grid_reduce_last: integer accumulators) and lets the
+// block that ends the reduction run the finisher Fin, which updates the solver scalars held in device memory.
 #pragma once
 #include "mks_internal.cuh"
 #include "mks_reduce.cuh"
@@ -32,12 +31,10 @@ __global__ void __launch_bounds__(256) k_site(const Op op, const Fin fin, const 
   __shared__ double smem[(256 / 32) * NS];
   __shared__ double row[2 * BLAS_MAXSRC * NS];  // gridDim.y <= 2 * BLAS_MAXSRC
   __shared__ double tot[2 * BLAS_MAXSRC * NS];
-  __shared__ double scratch[256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
 #pragma unroll
   for (int k = 0; k < NS; k++) {
-    double x = acc[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    const double x = warp_sum(acc[k]);
     if (lane == 0) smem[warp * NS + k] = x;
   }
   const int nsrc = gridDim.y, n = nsrc * NS;
@@ -49,8 +46,8 @@ __global__ void __launch_bounds__(256) k_site(const Op op, const Fin fin, const 
     row[s * NS + threadIdx.x] = t;
   }
   __syncthreads();
-  // each block's row carries its own source's NS sums and zeros elsewhere
-  if (!grid_reduce_last(row, n, red, tot, scratch)) return;
+  // each block's row carries its own source's NS sums and zeros elsewhere (which cost nothing)
+  if (!grid_reduce_last(row, n, red, tot)) return;
   if (threadIdx.x == 0 && totals)
     for (int i = 0; i < n; i++) totals[i] = tot[i];
   __syncthreads();

@@ -107,34 +107,27 @@ void capture_account(const Capture &k) {
   }
 }
 
-// Scratch for a reduction of nsum sums per block over `blocks` blocks
-// (grid_reduce_last in mks_reduce.cuh): block rows + group rows, and the
-// top counter + one counter per group.  Grown, never shrunk; counters are
-// zeroed when (re)allocated and are left at zero by every launch.
-int ensure_red(int nsum, int blocks) {
+// Scratch for a reduction of nsum sums (grid_reduce_last in mks_reduce.cuh).
+// Grown, never shrunk; zeroed when (re)allocated and left at zero by every
+// launch.
+int ensure_red(int nsum) {
   Context &c = g_ctx;
-  const size_t ngroups = ((size_t)blocks + RED_GROUP - 1) / RED_GROUP;
-  const size_t need = (size_t)nsum * ((size_t)blocks + ngroups), need_count = 1 + ngroups;
-  if (c.red.max_partials < need) {
-    dev_free(c.red.partials);
-    c.red.partials = nullptr;
-    c.red.max_partials = 0;
-    const size_t n = need < 65536 ? 65536 : need;
-    MKS_TRY(dev_alloc((void **)&c.red.partials, n * sizeof(double)));
-    c.red.max_partials = n;
-  }
   if (!c.red.err) {
     MKS_TRY(dev_alloc((void **)&c.red.err, sizeof(int)));
     MKS_CUDA(cudaMemsetAsync(c.red.err, 0, sizeof(int), c.stream));
   }
-  if (c.red.max_count < need_count) {
-    dev_free(c.red.count);
-    c.red.count = nullptr;
-    c.red.max_count = 0;
-    const size_t n = need_count < 4096 ? 4096 : need_count;
-    MKS_TRY(dev_alloc((void **)&c.red.count, n * sizeof(unsigned int)));
-    MKS_CUDA(cudaMemsetAsync(c.red.count, 0, n * sizeof(unsigned int), c.stream));
-    c.red.max_count = n;
+  if (!c.red.count) {
+    MKS_TRY(dev_alloc((void **)&c.red.count, sizeof(unsigned int)));
+    MKS_CUDA(cudaMemsetAsync(c.red.count, 0, sizeof(unsigned int), c.stream));
+  }
+  if (c.red.max_sums < (size_t)nsum) {
+    dev_free(c.red.limbs);
+    c.red.limbs = nullptr;
+    c.red.max_sums = 0;
+    const size_t n = nsum < 256 ? 256 : nsum, bytes = n * RED_LIMBS * sizeof(unsigned long long);
+    MKS_TRY(dev_alloc((void **)&c.red.limbs, bytes));
+    MKS_CUDA(cudaMemsetAsync(c.red.limbs, 0, bytes, c.stream));
+    c.red.max_sums = n;
   }
   return MKS_OK;
 }
@@ -454,7 +447,7 @@ int mks_finalize(void) {
   if (!c.initialised) return MKS_OK;
   cudaStreamSynchronize(c.stream);
   free_lattice_fields();
-  dev_free(c.red.partials); dev_free(c.red.count); dev_free(c.red.err);
+  dev_free(c.red.limbs); dev_free(c.red.count); dev_free(c.red.err);
   c.red = RedScratch();
   for (auto &e : c.ev_pool) cudaEventDestroy(e);
   c.ev_pool.clear();
@@ -485,13 +478,10 @@ int mks_set_lattice(const int dims[4]) {
   c.geom.nx = dims[0]; c.geom.ny = dims[1]; c.geom.nz = dims[2]; c.geom.nt = dims[3];
   c.geom.Vh = (int)c.Vh;
   c.geom.sx = 1; c.geom.sy = dims[0]; c.geom.sz = dims[0] * dims[1]; c.geom.st = dims[0] * dims[1] * dims[2];
-  // Reduction scratch for the largest reducing launch on this lattice, so
-  // that it is never reallocated while a solver batch is being captured:
-  // D_eo epilogues (up to 16 threads per site in blocks of >= 128 threads,
-  // 16 sources x 3 sums) and the BLAS site kernels (up to 4 blocks per SM
-  // per source row, 32 rows x 3 sums).
-  MKS_TRY(ensure_red(16 * 3, (int)((c.Vh * 16 + 127) / 128)));
-  MKS_TRY(ensure_red(32 * 3, c.sm_count * 4 * 32));
+  // Reduction scratch for the largest reducing launch, so that it is never
+  // reallocated while a solver batch is being captured: 32 rows x 3 sums of
+  // the BLAS site kernels (D_eo epilogues: 16 sources x 3 sums).
+  MKS_TRY(ensure_red(32 * 3));
   return MKS_OK;
 }
 

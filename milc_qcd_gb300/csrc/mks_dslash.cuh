@@ -467,11 +467,10 @@ __device__ __forceinline__ void dslash_body(const LinkT &fat, const LinkT &lng,
   if (NSUM > 0) {
     __shared__ double smem[(256 / 32 + 1) * MAXSRC * 3];
     __shared__ double tot[MAXSRC * 3];
-    __shared__ double scratch[256];
     block_reduce_grouped<R, NB, (NSUM > 0 ? NSUM : 1)>(sums, G, smem);
     const int nslots = G * NB;
     const double *btot = smem + (blockDim.x >> 5) * nslots * NSUM;
-    if (grid_reduce_last(btot, nslots * NSUM, a.red, tot, scratch)) {
+    if (grid_reduce_last(btot, nslots * NSUM, a.red, tot)) {
       if (threadIdx.x == 0) {
         for (int i = 0; i < a.nsrc * NSUM; i++) a.totals[i] = tot[i];
       }

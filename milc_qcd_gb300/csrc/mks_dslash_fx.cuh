@@ -222,13 +222,11 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
     __shared__ double smem[8 * NB * 3];
     __shared__ double bt[MAXSRC * 3];
     __shared__ double tot[MAXSRC * 3];
-    __shared__ double scratch[256];
 #pragma unroll
     for (int s = 0; s < NB; s++)
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        double v = sums[s][k];
-        for (int o = 16; o >= SPLIT; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const double v = warp_sum(sums[s][k]);
         if (lane == 0) smem[(warp * NB + s) * 3 + k] = v;
       }
     __syncthreads();
@@ -239,7 +237,7 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
       bt[i] = v;
     }
     __syncthreads();
-    if (grid_reduce_last(bt, G * NB * 3, a.red, tot, scratch)) {
+    if (grid_reduce_last(bt, G * NB * 3, a.red, tot)) {
       if (threadIdx.x == 0)
         for (int i = 0; i < a.nsrc * 3; i++) a.totals[i] = tot[i];
       __syncthreads();

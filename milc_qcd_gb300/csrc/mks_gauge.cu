@@ -469,7 +469,7 @@ static int site_sum(const Op &op, int rows, double *host_out) {
   const int Vh = (int)c.Vh;
   int gx = grid_for(Vh, 256);
   if (gx > c.sm_count * 4) gx = c.sm_count * 4;
-  MKS_TRY(ensure_red(NS * rows, gx * rows));
+  MKS_TRY(ensure_red(NS * rows));
   double *tot = nullptr;
   MKS_TRY(dev_alloc((void **)&tot, (size_t)NS * rows * sizeof(double)));
   timing_begin(MKS_K_GAUGE);

@@ -302,15 +302,13 @@ struct LinkF16 {
 };
 
 // ------------------------------------------------------------------
-// device-side reduction scratch for grid_reduce_last: per-block and
-// per-group rows of partial sums, and the arrival counters (top + one per
-// group of blocks), which return to 0 at the end of every launch
-constexpr int RED_GROUP = 64;  // blocks per first-level group
+// device-side reduction scratch for grid_reduce_last: integer accumulators
+// of each sum and the arrival counter
+constexpr int RED_LIMBS = 67;  // 64-bit integers per sum: 66 x 32 bits span every double, and flags
 struct RedScratch {
-  double *partials;     // capacity: max_partials doubles
-  unsigned int *count;  // capacity: max_count counters
-  size_t max_partials;
-  size_t max_count;
+  unsigned long long *limbs;  // capacity: max_sums * RED_LIMBS
+  unsigned int *count;
+  size_t max_sums;
   int *err;             // set on the device when a launch would overrun the scratch
 };
 // reads and clears the device error flag: MKS_ERR_CUDA if a reduction
@@ -428,7 +426,7 @@ int ws(const std::string &name, size_t bytes, void **out);
 void ws_free_all();
 
 // reduction scratch sized for `nsum` sums and `blocks` blocks
-int ensure_red(int nsum, int blocks);
+int ensure_red(int nsum);
 
 inline int grid_for(size_t n, int block) { return (int)((n + block - 1) / block); }
 

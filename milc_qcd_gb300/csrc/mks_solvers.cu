@@ -407,7 +407,7 @@ static int launch_site(int family, const Op &op, const Fin &fin, const int *skip
   if (!forced) per_sm = per_sm < 1 ? 1 : per_sm > 4 ? 4 : per_sm;
   int cap = c.sm_count * per_sm;
   if (gx > cap) gx = cap;
-  MKS_TRY(ensure_red(NSUM > 0 ? NSUM * nsrc : 1, gx * nsrc));  // one row per block of the (gx, nsrc) grid
+  MKS_TRY(ensure_red(NSUM > 0 ? NSUM * nsrc : 1));
   timing_begin(family);
   k_site<Op, NSUM, Fin><<<dim3(gx, nsrc), 256, 0, c.stream>>>(op, fin, skip, Vh, c.red,
                                                              totals);
@@ -550,7 +550,7 @@ static int launch_dslash_nb(int family, const LinkT &fat, const LinkT &lng,
       a.nvb = 0;
       const size_t smem = (size_t)as * 72 * (block / a.groups);
       if (NSUM > 0) {
-        MKS_TRY(ensure_red(NSUM * a.groups * NB, grid));
+        MKS_TRY(ensure_red(NSUM * a.groups * NB));
         a.red = c.red;
       }
       auto ka = as == 2 ? k_dslash_a<InT, OutT, NB, EPI, NSUM, Fin, 2> : k_dslash_a<InT, OutT, NB, EPI, NSUM, Fin, 3>;
@@ -595,7 +595,7 @@ static int launch_dslash_nb(int family, const LinkT &fat, const LinkT &lng,
     }
   }
   if (NSUM > 0) {
-    MKS_TRY(ensure_red(NSUM * a.groups * NB, grid));
+    MKS_TRY(ensure_red(NSUM * a.groups * NB));
     a.red = c.red;
   }
   timing_begin(family);
@@ -639,7 +639,7 @@ static int launch_shape(int family, const LinkT &fat, const LinkT &lng,
                                       TMA_MAX_SMEM));
         attr = true;
       }
-      MKS_TRY(ensure_red(NSUM > 0 ? NSUM * sh.G : 1, grid));
+      MKS_TRY(ensure_red(NSUM > 0 ? NSUM * sh.G : 1));
       a.red = c.red;
       timing_begin(family);
       k_dslash_tma<EPI, NSUM, Fin><<<grid, T * sh.G, smem, c.stream>>>(fat, lng, a, fin, T, Rr);
@@ -974,7 +974,7 @@ static int launch_fx_as(FxArgs &a, const Fin &fin, int mult, int rows) {
   a.G = (a.nsrc + NB - 1) / NB;
   const int block = 32 * a.G * mult, grid = grid_for(c.Vh, 32 / SPLIT * mult);
   if (EPI == EPI_AXPY) {
-    MKS_TRY(ensure_red(3 * a.G * NB, grid));
+    MKS_TRY(ensure_red(3 * a.G * NB));
     a.red = c.red;
   }
   (EPI == EPI_AXPY ? g_shape_epi : g_shape)[MKS_PREC_DOUBLE][a.nsrc] = {a.G * SPLIT, NB, block, 0, 0, 0, 0};
@@ -1423,7 +1423,7 @@ static int run_batch(const LinkSlot &sl, int par, int nsrc, int prec, const doub
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
   key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fx_exp); key_push(key, sl.fx_special);
-  key_push(key, S.st); key_push(key, S.skip); key_push(key, c.red.partials); key_push(key, c.red.count);
+  key_push(key, S.st); key_push(key, S.skip); key_push(key, c.red.limbs); key_push(key, c.red.count);
   for (int s = 0; s < nsrc; s++) {
     key_push(key, msq4[s]);
     key_push(key, f.x[s]); key_push(key, f.p[s]); key_push(key, f.r[s]); key_push(key, f.ttt[s]);
@@ -2130,14 +2130,19 @@ __device__ __forceinline__ void ms_alpha(MsState &m, const double *t) {
   const double rsq_new = rsq + 2.0 * bl * c_tr + bl * bl * c_tt;
   const double al = rsq_new / rsq;
   __syncwarp();
-  double zp = 1.0, bi = bl;
+  // with w = zeta_im1 beta_im1 / (c1 + c2): zeta_ip1 = zeta_i w, beta_i =
+  // beta w, alpha_i = alpha w^2, one division after the first two (570 clocks
+  // each; zeta_i zeta_im1 beta_im1 / (c1 + c2), beta zeta_ip1 / zeta_i and
+  // alpha zeta_ip1 beta_i / (zeta_i beta) took three, one after the other)
+  double zp = 1.0, bi = bl, w = 1.0;
   bool drop = false;
   if (mine && j != jl) {
     const double c1 = bl * alpha_l * (zm - zi);
     const double c2 = zm * bml * (1.0 + sh * bl);
-    zp = c1 + c2 != 0.0 ? zi * zm * bml / (c1 + c2) : 0.0;
+    w = c1 + c2 != 0.0 ? zm * bml / (c1 + c2) : 0.0;
     if (zi != 0.0) {
-      bi = bl * zp / zi;
+      zp = zi * w;
+      bi = bl * w;
     } else {
       zp = 0.0;
       bi = 0.0;
@@ -2151,7 +2156,7 @@ __device__ __forceinline__ void ms_alpha(MsState &m, const double *t) {
   for (int k = 0; k < now0; k++)
     if ((dm >> k & 1) && k == now - 1) now--;
   double aj = al;
-  if (mine && j != jl && j < now) aj = zi * bl != 0.0 ? al * zp * bi / (zi * bl) : 0.0;
+  if (mine && j != jl && j < now) aj = zi * bl != 0.0 ? al * w * w : 0.0;
   if (mine) {
     m.zeta_im1[j] = zm;
     m.zeta_i[j] = zi;
@@ -2370,15 +2375,16 @@ __global__ void __launch_bounds__(96 * NG) k_ms_update(const MsUpdate<R, RS, NF>
   }
   __shared__ double wsum[3];
   __shared__ double row[NF], tot[NF];
-  __shared__ double scratch[96 * NG];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0 && grp == 0) wsum[comp] = acc;
+  if (grp == 0) {
+    acc = warp_sum(acc);
+    if (lane == 0) wsum[comp] = acc;
+  }
   if (threadIdx.x < NF) row[threadIdx.x] = 0.0;
   __syncthreads();
   if (threadIdx.x == 0) row[blockIdx.y] = wsum[0] + wsum[1] + wsum[2];
   __syncthreads();
   const int n = gridDim.y;
-  if (!grid_reduce_last(row, n, red, tot, scratch)) return;
+  if (!grid_reduce_last(row, n, red, tot)) return;
   if (threadIdx.x == 0 && totals)
     for (int k = 0; k < n; k++) totals[k] = tot[k];
   __syncthreads();
@@ -2394,7 +2400,7 @@ static int launch_ms_update(const MsUpdate<R, RS, NF> &a, const Fin &fin, const 
   const int ng = nsh >= 8 && warps * 2 < full ? 4 : nsh >= 4 && warps < full ? 2 : 1;
   const int cap = c.sm_count * 16 / (ng * rows) > c.sm_count ? c.sm_count * 16 / (ng * rows) : c.sm_count;
   const int gx = ntiles < cap ? ntiles : cap;
-  MKS_TRY(ensure_red(rows, gx * rows));
+  MKS_TRY(ensure_red(rows));
   timing_begin(MKS_K_SHIFT);
   const dim3 grid(gx, rows);
   if (ng == 4) k_ms_update<R, RS, NF, 4, Fin><<<grid, 384, 0, c.stream>>>(a, fin, skip, c.red, nullptr);
@@ -2653,7 +2659,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
   key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fx_exp); key_push(key, sl.fx_special);
-  key_push(key, st); key_push(key, skip); key_push(key, tot); key_push(key, c.red.partials); key_push(key, c.red.count);
+  key_push(key, st); key_push(key, skip); key_push(key, tot); key_push(key, c.red.limbs); key_push(key, c.red.count);
   key_push(key, h.shift0); key_push(key, nsh); key_push(key, r); key_push(key, cgp); key_push(key, ttt);
   key_push(key, t); key_push(key, cgq.q); key_push(key, cgq.e); key_push(key, tq.q); key_push(key, tq.e);
   key_push(key, p16); key_push(key, t16); key_push(key, p16n); key_push(key, t16n);
@@ -2817,7 +2823,7 @@ static int multishift_multi_core(const LinkSlot &sl, int par, int nf, const doub
     key_push(key, c.geom.Vh); key_push(key, c.geom.nx); key_push(key, c.geom.ny); key_push(key, c.geom.nz);
     key_push(key, c.geom.nt); key_push(key, sl.fat32a); key_push(key, sl.lng32a); key_push(key, sl.fat32b);
     key_push(key, sl.lng32b); key_push(key, st); key_push(key, skip); key_push(key, tot);
-    key_push(key, c.red.partials); key_push(key, c.red.count); key_push(key, nact);
+    key_push(key, c.red.limbs); key_push(key, c.red.count); key_push(key, nact);
     for (int q = 0; q < nact; q++) {
       const int f = act[q];
       key_push(key, f); key_push(key, hs[f].shift0); key_push(key, nsh[f]); key_push(key, r[f]);
