@@ -75,7 +75,7 @@ static __device__ __noinline__ void fx_site_f64(const Geom &g, const double2 *fa
   for (int c = 0; c < 3; c++) { out[2 * c] = acc.c[c].re; out[2 * c + 1] = acc.c[c].im; }
 }
 
-template <int SPLIT, int NB, int OUT, int EPI, class Fin>
+template <int SPLIT, bool DENSE, int NB, int OUT, int EPI, class Fin>
 __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) {
   if (a.skip && *a.skip) return;
   const Geom &g = a.g;
@@ -84,6 +84,8 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
   const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nwarps = (int)blockDim.x >> 5;
   const int grp = warp % G, wsite = (bid * nwarps + warp) / G;   // blocks hold a multiple of G warps
   const int m0 = SPLIT == 1 ? 0 : lane % SPLIT;
+  // where the FP64 rate counts, an FP64 tail takes one colour per thread
+  constexpr int LANES = DENSE && OUT == FX_OUT_F64 ? 3 : 1, NC = 3 / LANES;
   const int h0 = wsite * (32 / SPLIT) + lane / SPLIT;
   // threads past the last site follow it, so that the shuffles of a warp see all lanes
   const int h = h0 < Vh ? h0 : Vh - 1;
@@ -92,7 +94,7 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
 #pragma unroll
   for (int s = 0; s < NB; s++) {
     const int S = grp * NB + s;
-    live[s] = h0 < Vh && S < a.nsrc && m0 == 0;
+    live[s] = h0 < Vh && S < a.nsrc && m0 < LANES;
     in[s] = a.in[S < a.nsrc ? S + (int)blockIdx.y : 0];   // blockIdx.y = 1: the second parity of a one-source launch
   }
   int x, y, z, t;
@@ -186,9 +188,17 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
     if (plain) {
       fx_site_f64(g, a.fat64, a.lng64, in[s], par, h, x, y, z, t, v);
       if (OUT == FX_OUT_BLOCK) fx_encode(v, q, e);
+      if (LANES > 1) {
+        v[0] = m0 == 0 ? v[0] : m0 == 1 ? v[2] : v[4];
+        v[1] = m0 == 0 ? v[1] : m0 == 1 ? v[3] : v[5];
+      }
     } else if (OUT != FX_OUT_BLOCK) {
+      if (LANES > 1) {
+        q[0] = m0 == 0 ? q[0] : m0 == 1 ? q[2] : q[4];
+        q[1] = m0 == 0 ? q[1] : m0 == 1 ? q[3] : q[5];
+      }
 #pragma unroll
-      for (int k = 0; k < 6; k++) v[k] = e == FX_ZERO ? 0.0 : fx_double(q[k], e);
+      for (int k = 0; k < 2 * NC; k++) v[k] = e == FX_ZERO ? 0.0 : fx_double(q[k], e);
     }
     if (OUT == FX_OUT_BLOCK) {
       fx_store(a.outq[S], h, Vh, q, e);
@@ -205,8 +215,8 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
       if (EPI == EPI_AXPY) {
         const double cf = a.coef[S];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const double2 pv = __ldg(a.p[S] + (size_t)c * Vh + h), rv = __ldg(a.r[S] + (size_t)c * Vh + h);
+        for (int c = 0; c < NC; c++) {
+          const double2 pv = __ldg(a.p[S] + (size_t)(LANES > 1 ? m0 : c) * Vh + h), rv = __ldg(a.r[S] + (size_t)(LANES > 1 ? m0 : c) * Vh + h);
           v[2 * c] = fma(cf, pv.x, v[2 * c]);
           v[2 * c + 1] = fma(cf, pv.y, v[2 * c + 1]);
           sums[s][0] = fma(pv.x, v[2 * c], fma(pv.y, v[2 * c + 1], sums[s][0]));
@@ -215,7 +225,7 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
         }
       }
 #pragma unroll
-      for (int c = 0; c < 3; c++) a.out[S][(size_t)c * Vh + h] = make_double2(v[2 * c], v[2 * c + 1]);
+      for (int c = 0; c < NC; c++) a.out[S][(size_t)(LANES > 1 ? m0 : c) * Vh + h] = make_double2(v[2 * c], v[2 * c + 1]);
     }
   }
   if (EPI == EPI_AXPY) {
@@ -248,7 +258,21 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
 
 template <int SPLIT, int NB, int OUT, int EPI, class Fin>
 __global__ void __launch_bounds__(256, NB == 1 ? 2 : 1) k_dslash_fx(const FxArgs a, const Fin fin) {
-  dslash_fx_body<SPLIT, NB, OUT, EPI, Fin>(a, fin);
+  dslash_fx_body<SPLIT, false, NB, OUT, EPI, Fin>(a, fin);
+}
+
+// Four threads per site in 102 registers: 20 warps per SM instead of 16, for
+// launches that 20 hold at once and 16 do not.  On 12^3x24 those left 160 of
+// 2592 warps to a second wave, and the FP64 tail of a warp (24 operations of
+// 64 clocks, 8 when its threads share the colours) is a good part of an
+// epilogue launch: the two D of a multi-shift iteration 55 and 48 us, the
+// FP64 trajectory 143 and 135 ms.  Elsewhere the registers count more
+// (12x14x10x20, one warp per SM under the line, D into MILC's layout: 24 and
+// 29 us; 16^3x32, 54 warps per SM: even or slower) and sharing colours costs
+// two exchanges (8^4 CG: 1.43 and 1.49 ms).
+template <int OUT, int EPI, class Fin>
+__global__ void __launch_bounds__(128, 5) k_dslash_fx_dense(const FxArgs a, const Fin fin) {
+  dslash_fx_body<4, true, 1, OUT, EPI, Fin>(a, fin);
 }
 
 }  // namespace mks

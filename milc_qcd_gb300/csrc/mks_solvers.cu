@@ -979,7 +979,14 @@ static int launch_fx_as(FxArgs &a, const Fin &fin, int mult, int rows) {
   }
   (EPI == EPI_AXPY ? g_shape_epi : g_shape)[MKS_PREC_DOUBLE][a.nsrc] = {a.G * SPLIT, NB, block, 0, 0, 0, 0};
   timing_begin(MKS_K_DSLASH_F64);
-  k_dslash_fx<SPLIT, NB, OUT, EPI, Fin><<<dim3(grid, rows), block, 0, c.stream>>>(a, fin);
+  // warps that the chip holds at once at 20 per SM (102 registers a thread), not at 16
+  const size_t warps = (size_t)grid * rows * (block / 32), sm = c.sm_count;
+  bool dense = false;
+  if constexpr (SPLIT == 4 && OUT != FX_OUT_AOS) {
+    dense = block <= 128 && warps > 16 * sm && warps <= 20 * sm;
+    if (dense) k_dslash_fx_dense<OUT, EPI, Fin><<<dim3(grid, rows), block, 0, c.stream>>>(a, fin);
+  }
+  if (!dense) k_dslash_fx<SPLIT, NB, OUT, EPI, Fin><<<dim3(grid, rows), block, 0, c.stream>>>(a, fin);
   timing_end(MKS_K_DSLASH_F64);
   MKS_CUDA(cudaGetLastError());
   return MKS_OK;
