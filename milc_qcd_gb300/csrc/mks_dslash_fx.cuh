@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(256, NB == 1 ? 2 : 1) k_dslash_fx(const FxArgs
 // 64 clocks, 8 when its threads share the colours) is a good part of an
 // epilogue launch: the two D of a multi-shift iteration 55 and 48 us, the
 // FP64 trajectory 143 and 135 ms.  Elsewhere the registers count more
-// (12x14x10x20, one warp per SM under the line, D into MILC's layout: 24 and
-// 29 us; 16^3x32, 54 warps per SM: even or slower) and sharing colours costs
+// (14x10x18x22, 23 warps per SM, D into MILC's layout: 24 and 29 us; 16^3x32,
+// 54 warps per SM: even or slower) and sharing colours costs
 // two exchanges (8^4 CG: 1.43 and 1.49 ms).
 template <int OUT, int EPI, class Fin>
 __global__ void __launch_bounds__(128, 5) k_dslash_fx_dense(const FxArgs a, const Fin fin) {

@@ -491,4 +491,64 @@ static __global__ void __launch_bounds__(FXM_BLOCK, 4) k_staple_adj_fx(Geom g, i
   }
 }
 
+// ---- paths of links (gauge force and action in FP64) ----
+// a running product as integers, normalised after each step so that a path of
+// five links keeps the bits of one
+struct FxPath { int4 u[9]; int e; };
+
+// site (par, h)'s matrix of one direction, as it is or its adjoint
+__device__ __forceinline__ void fxm_load(const FxMat &f, int par, int h, bool adj, int4 (&u)[9], int &e) {
+  const int4 *p = f.at(par, h);
+  const int sg = adj ? -1 : 1;
+  e = __ldg(f.e + par * f.es + h);
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    u[k] = __ldg(p + 32 * (adj ? (k % 3) * 3 + k / 3 : k));
+    u[k].z *= sg;
+    u[k].w *= sg;
+  }
+}
+// P <- P L
+__device__ __forceinline__ void fxm_step(FxPath &P, const int4 (&Lm)[9], int el) {
+  s64 q[18];
+  u64 mag = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      FxSum re, im;
+      fxm_element(P.u, i, Lm, j, re, im);
+      const s64 a = (s64)(re.H << 3) + ((s64)re.M >> 29), b = (s64)(im.H << 3) + ((s64)im.M >> 29);
+      q[2 * (3 * i + j)] = a;
+      q[2 * (3 * i + j) + 1] = b;
+      mag |= (u64)(a ^ (a >> 63)) | (u64)(b ^ (b >> 63));
+    }
+  const int sh = __clzll((s64)mag) - 4;   // from -2 on; 60 for zeros and -1
+  P.e += el + 1 - sh;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const s64 a = sh < 0 ? q[2 * k] >> -sh : (s64)((u64)q[2 * k] << sh);
+    const s64 b = sh < 0 ? q[2 * k + 1] >> -sh : (s64)((u64)q[2 * k + 1] << sh);
+    fxm_split(a, P.u[k].x, P.u[k].y);
+    fxm_split(b, P.u[k].z, P.u[k].w);
+  }
+}
+// Re tr(P L)
+__device__ __forceinline__ double fxm_trace(const FxPath &P, const int4 (&Lm)[9], int el) {
+  s64 t = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    FxSum re = {0, 0};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int4 a = P.u[3 * i + k], b = Lm[3 * k + i];
+      fx_mac(re, a.x, a.y, b.x, b.y);
+      fx_mac(re, -a.z, -a.w, b.z, b.w);
+    }
+    t += (s64)(re.H << 1) + ((s64)re.M >> 31);
+  }
+  const int e = P.e + el + 3;   // t 2^(P.e + el - 57)
+  return e < FX_ZERO / 2 ? 0.0 : fx_double(t, e);
+}
+
 }  // namespace mks

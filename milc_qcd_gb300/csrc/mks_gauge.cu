@@ -18,12 +18,16 @@
 // one site per thread; the loop/staple paths are tables in constant memory
 // generated on the host exactly as MILC generates its loop table.  The
 // force and action walk each path link by link (recomputation instead of
-// stored intermediate staple fields), in FP64.
+// stored intermediate staple fields): FP32 in floats, FP64 in integer
+// arithmetic on a copy of the links in the workspace, or in plain FP64 when
+// there is no memory for that copy (another 144 bytes per link) or a link is
+// not finite.
 #include <cmath>
 #include <cstring>
 #include <vector>
 #include "mks_internal.cuh"
 #include "mks_su3.cuh"
+#include "mks_fixed_mat.cuh"
 #include "mks_blas.cuh"
 
 namespace mks {
@@ -328,6 +332,24 @@ __device__ __forceinline__ M3<float> walk32(const Geom &g, const float2 *U32, in
   return P;
 }
 
+// one link's momentum m <- TA(m - eb3 G)
+__device__ __forceinline__ void mom_update(double *m, double eb3, const M3<double> &G) {
+  // A = uncompressed mom - eb3 G, then its traceless anti-Hermitian part
+  // (libraries/uncmp_ahmat.c, make_ahmat.c)
+  const double d0 = m[6] - eb3 * G.e[0][0].im, d1 = m[7] - eb3 * G.e[1][1].im, d2 = m[8] - eb3 * G.e[2][2].im;
+  const double t = (d0 + d1 + d2) * 0.33333333333333333;
+  const double a01r = m[0], a01i = m[1], a02r = m[2], a02i = m[3], a12r = m[4], a12i = m[5];
+  m[0] = ((a01r - eb3 * G.e[0][1].re) - (-a01r - eb3 * G.e[1][0].re)) * 0.5;
+  m[1] = ((a01i - eb3 * G.e[0][1].im) + (a01i - eb3 * G.e[1][0].im)) * 0.5;
+  m[2] = ((a02r - eb3 * G.e[0][2].re) - (-a02r - eb3 * G.e[2][0].re)) * 0.5;
+  m[3] = ((a02i - eb3 * G.e[0][2].im) + (a02i - eb3 * G.e[2][0].im)) * 0.5;
+  m[4] = ((a12r - eb3 * G.e[1][2].re) - (-a12r - eb3 * G.e[2][1].re)) * 0.5;
+  m[5] = ((a12i - eb3 * G.e[1][2].im) + (a12i - eb3 * G.e[2][1].im)) * 0.5;
+  m[6] = d0 - t;
+  m[7] = d1 - t;
+  m[8] = d2 - t;
+}
+
 // mom_mu(x) <- TA(mom_mu(x) - eb3 U_mu(x) sum_p c_p Q_p), Q_p the staple
 // paths from x+mu back to x (links without phases)
 // staple sum and product in arithmetic R (FP64 reproduces MILC's double
@@ -371,21 +393,92 @@ __global__ void __launch_bounds__(128) k_gauge_force(Geom g, const double2 *U, c
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) G.e[i][j] = {(double)Gr.e[i][j].re, (double)Gr.e[i][j].im};
-  double *m = mom + (((size_t)par * g.Vh + h) * 4 + mu) * 10;
-  // A = uncompressed mom - eb3 G, then its traceless anti-Hermitian part
-  // (libraries/uncmp_ahmat.c, make_ahmat.c)
-  const double d0 = m[6] - eb3 * G.e[0][0].im, d1 = m[7] - eb3 * G.e[1][1].im, d2 = m[8] - eb3 * G.e[2][2].im;
-  const double t = (d0 + d1 + d2) * 0.33333333333333333;
-  const double a01r = m[0], a01i = m[1], a02r = m[2], a02i = m[3], a12r = m[4], a12i = m[5];
-  m[0] = ((a01r - eb3 * G.e[0][1].re) - (-a01r - eb3 * G.e[1][0].re)) * 0.5;
-  m[1] = ((a01i - eb3 * G.e[0][1].im) + (a01i - eb3 * G.e[1][0].im)) * 0.5;
-  m[2] = ((a02r - eb3 * G.e[0][2].re) - (-a02r - eb3 * G.e[2][0].re)) * 0.5;
-  m[3] = ((a02i - eb3 * G.e[0][2].im) + (a02i - eb3 * G.e[2][0].im)) * 0.5;
-  m[4] = ((a12r - eb3 * G.e[1][2].re) - (-a12r - eb3 * G.e[2][1].re)) * 0.5;
-  m[5] = ((a12i - eb3 * G.e[1][2].im) + (a12i - eb3 * G.e[2][1].im)) * 0.5;
-  m[6] = d0 - t;
-  m[7] = d1 - t;
-  m[8] = d2 - t;
+  mom_update(mom + (((size_t)par * g.Vh + h) * 4 + mu) * 10, eb3, G);
+}
+
+// One link of a path from site c, which moves along it: the integers of the
+// link (its adjoint on a backward step), its exponent; the sign of its phase
+// goes to sg
+__device__ __forceinline__ void path_link(const Geom &g, const FxMat &U, int (&c)[4], int d, int4 (&u)[9], int &e,
+                                          int &sg) {
+  const int L[4] = {g.nx, g.ny, g.nz, g.nt}, dir = d < 4 ? d : 7 - d;
+  if (d >= 4) c[dir] = wrap_add(c[dir], -1, L[dir]);
+  if (stag_phase(g, c, dir) < 0) sg = -sg;
+  fxm_load(fx_link_dir(U, dir, g.Vh), (c[0] + c[1] + c[2] + c[3]) & 1, cb_index(g, c[0], c[1], c[2], c[3]), d >= 4, u, e);
+  if (d < 4) c[dir] = wrap_add(c[dir], 1, L[dir]);
+}
+// product of the first n links of a path; false when one is not finite
+__device__ __forceinline__ bool walk_fx(const Geom &g, const FxMat &U, int (&c)[4], const signed char *path, int n,
+                                        FxPath &P, int &sg) {
+  path_link(g, U, c, path[0], P.u, P.e, sg);
+  bool ok = P.e != FX_SPECIAL;
+#pragma unroll 1
+  for (int k = 1; k < n; k++) {
+    int4 u[9];
+    int e;
+    path_link(g, U, c, path[k], u, e, sg);
+    ok = ok && e != FX_SPECIAL;
+    fxm_step(P, u, e);
+  }
+  return ok;
+}
+
+// a staple sum in plain FP64 (a link of its paths is not finite)
+static __device__ __noinline__ void staple_sum_f64(const Geom &g, const double2 *U, const int *x0, int mu, double *S) {
+  const int L[4] = {g.nx, g.ny, g.nz, g.nt};
+  for (int k = 0; k < 18; k++) S[64 * k] = 0.0;
+#pragma unroll 1
+  for (int p = 0; p < c_staples.n[mu]; p++) {
+    int c[4] = {x0[0], x0[1], x0[2], x0[3]};
+    c[mu] = wrap_add(c[mu], 1, L[mu]);
+    const M3<double> Q = walk(g, U, c, c_staples.dir[mu][p], c_staples.len[mu][p]);
+    for (int k = 0; k < 9; k++) {
+      S[64 * (2 * k)] += c_staples.c[mu][p] * Q.e[k / 3][k % 3].re;
+      S[64 * (2 * k + 1)] += c_staples.c[mu][p] * Q.e[k / 3][k % 3].im;
+    }
+  }
+}
+
+// The FP64 gauge force with its paths in integer arithmetic (mks_fixed_mat.cuh):
+// a product of two matrices is 108 FP64 fmas at 64 clocks each, or 324
+// integer multiply-adds at 2 and the normalising, and the 180 products of a
+// link are the launch's time.  The sum over the paths, in shared memory (36
+// registers that the products need), and the last product stay FP64.
+// 12^3x24: 7.03 ms in FP64, 2.23 ms here (162 products of 324 at the measured
+// rate alone are 0.5 ms; 164 registers leave 12 warps per SM to hide the
+// rest).  Blocks of 64: 1296 of them on that lattice.
+static __global__ void __launch_bounds__(64) k_gauge_force_fx(Geom g, const double2 *U, FxMat Ux, double *mom,
+                                                             double eb3) {
+  __shared__ double sum[18][64];
+  const int h = blockIdx.x * blockDim.x + threadIdx.x, par = blockIdx.y, mu = blockIdx.z;
+  if (h >= g.Vh) return;
+  double *S = &sum[0][threadIdx.x];
+  int x0[4];
+  site_coords(g, par, h, x0[0], x0[1], x0[2], x0[3]);
+  const int L[4] = {g.nx, g.ny, g.nz, g.nt};
+#pragma unroll
+  for (int k = 0; k < 18; k++) S[64 * k] = 0.0;
+  bool ok = true;
+#pragma unroll 1
+  for (int p = 0; p < c_staples.n[mu]; p++) {
+    int c[4] = {x0[0], x0[1], x0[2], x0[3]}, sg = 1;
+    c[mu] = wrap_add(c[mu], 1, L[mu]);
+    FxPath P;
+    ok = walk_fx(g, Ux, c, c_staples.dir[mu][p], c_staples.len[mu][p], P, sg) && ok;
+    if (P.e < FX_ZERO / 2) continue;
+    const double cf = sg * c_staples.c[mu][p];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      S[64 * (2 * k)] = fma(cf, fx_double(((s64)P.u[k].x << 32) + P.u[k].y, P.e), S[64 * (2 * k)]);
+      S[64 * (2 * k + 1)] = fma(cf, fx_double(((s64)P.u[k].z << 32) + P.u[k].w, P.e), S[64 * (2 * k + 1)]);
+    }
+  }
+  if (!ok) staple_sum_f64(g, U, x0, mu, S);
+  M3<double> Sm;
+#pragma unroll
+  for (int k = 0; k < 9; k++) Sm.e[k / 3][k % 3] = {S[64 * (2 * k)], S[64 * (2 * k + 1)]};
+  const M3<double> G = mul_nn<double>(load_link(g, U, x0, mu, true), Sm);
+  mom_update(mom + (((size_t)par * g.Vh + h) * 4 + mu) * 10, eb3, G);
 }
 
 // sum over sites of one parity (row = parity) of c (3 - Re tr W) over every
@@ -403,6 +496,33 @@ struct OpGaugeAction {
       acc += c_loops.c[p] * (3.0 - (W.e[0][0].re + W.e[1][1].re + W.e[2][2].re));
     }
     out[0] = acc;
+  }
+};
+
+// the same with the products in integer arithmetic; a last product is only
+// traced (12^3x24: 2.64 and 0.68 ms)
+struct OpGaugeActionFx {
+  OpGaugeAction f64;
+  FxMat Ux;
+  __device__ void operator()(int h, int par, double *out) const {
+    const Geom &g = f64.g;
+    int x0[4];
+    site_coords(g, par, h, x0[0], x0[1], x0[2], x0[3]);
+    double acc = 0.0;
+    bool ok = true;
+#pragma unroll 1
+    for (int p = 0; p < c_loops.n; p++) {
+      int c[4] = {x0[0], x0[1], x0[2], x0[3]}, sg = 1, e;
+      const int n = c_loops.len[p];
+      FxPath P;
+      int4 u[9];
+      ok = walk_fx(g, Ux, c, c_loops.dir[p], n - 1, P, sg) && ok;
+      path_link(g, Ux, c, c_loops.dir[p][n - 1], u, e, sg);
+      ok = ok && e != FX_SPECIAL;
+      acc += c_loops.c[p] * (3.0 - sg * fxm_trace(P, u, e));
+    }
+    if (ok) out[0] = acc;
+    else f64(h, par, out);
   }
 };
 
@@ -718,12 +838,24 @@ static void thin_changed() {
 
 static dim3 link_grid() { return dim3(grid_for(ctx().Vh, 128), 2, 4); }
 
+// the thin links as integers, in the link construction's workspace; false
+// when there is no memory for them (the FP64 kernels need none)
+static bool thin_fxm(FxMat *f) {
+  Context &c = ctx();
+  return ws_links_fxm("fxm_links", MKS_K_GAUGE, c.auxU, f) >= 0;
+}
+
 int gauge_force_dev(double eps, double beta, double u0, int nflavors, int prec) {
   Context &c = ctx();
   MKS_TRY(upload_paths(nflavors, u0));
+  FxMat Ux;
+  const bool fx = prec == MKS_PREC_DOUBLE && thin_fxm(&Ux);
   timing_begin(MKS_K_GAUGE);
   if (prec == MKS_PREC_DOUBLE) {
-    k_gauge_force<double><<<link_grid(), 128, 0, c.stream>>>(c.geom, c.auxU, nullptr, c.mom, eps * beta / 3.0);
+    if (fx)
+      k_gauge_force_fx<<<dim3(grid_for(c.Vh, 64), 2, 4), 64, 0, c.stream>>>(c.geom, c.auxU, Ux, c.mom, eps * beta / 3.0);
+    else
+      k_gauge_force<double><<<link_grid(), 128, 0, c.stream>>>(c.geom, c.auxU, nullptr, c.mom, eps * beta / 3.0);
   } else {
     if (g_u32_sites != c.V) {
       dev_free(g_u32);
@@ -744,7 +876,10 @@ int gauge_action_dev(double beta, double u0, int nflavors, double *action) {
   Context &c = ctx();
   MKS_TRY(upload_paths(nflavors, u0));
   double tot[2];
-  MKS_TRY((site_sum<OpGaugeAction, 1>(OpGaugeAction{c.geom, c.auxU}, 2, tot)));
+  const OpGaugeAction f64 = {c.geom, c.auxU};
+  FxMat Ux;
+  if (thin_fxm(&Ux)) MKS_TRY((site_sum<OpGaugeActionFx, 1>(OpGaugeActionFx{f64, Ux}, 2, tot)));
+  else MKS_TRY((site_sum<OpGaugeAction, 1>(f64, 2, tot)));
   *action = beta / 3.0 * (tot[0] + tot[1]);
   return MKS_OK;
 }
