@@ -390,7 +390,7 @@ def extras(m, lib, _lib, torch, srcs):
         ms[name] = {"s": dt, "iters": it, "max_final_rsq": max(res[k].final_rsq for k in range(len(sig))),
                     "converged": all(res[k].converged for k in range(len(sig))), "kernel_ms": fam}
         # rooflines of the multi-shift iteration's two kernels: the update
-        # kernel (OpShiftUpdate) and the single-source D_eo pair
+        # kernel (k_ms_update) and the single-source D_eo pair
         n_it, n_upd = ctypes.c_longlong(), ctypes.c_longlong()
         lib.mks_multishift_counts(ctypes.byref(n_it), ctypes.byref(n_upd))
         # update-kernel vectors: r (read, write), ttt (read) and the lowest
@@ -503,7 +503,7 @@ def gpu_arm(args):
     arg64 = _lib.InvertArg(1000, 10, m.EVEN, m.PREC_DOUBLE, RESID, 0.0, 0.1)
     res64 = _lib.InvertResult()
     d64 = torch.zeros_like(d_src[0])
-    for rep in range(2):  # the first call tunes the FP64 D_eo shape and captures the graphs
+    for rep in range(2):  # the first call captures the graphs
         d64.zero_()
         torch.cuda.synchronize()
         t0 = time.time()

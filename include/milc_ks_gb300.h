@@ -331,7 +331,8 @@ int mks_bench_dslash(int prec, int nsrc, int parity, int slot, int iters, int fl
  * count, and every count of the class takes that shape (environment
  * MKS_TUNE=0 keeps a fixed table).  Returns MKS_ERR_STATE when no shape
  * has been chosen for nsrc yet (a class's widest count has its shape as
- * soon as any count of the class was launched). */
+ * soon as any count of the class was launched).  FP64 launches take their
+ * shape by rule: the last launch's. */
 int mks_tuned_shape(int prec, int nsrc, int *G, int *nb, int *block);
 
 /* The same for the launches with the fused CG epilogue (D_eo, axpy and
