@@ -206,20 +206,37 @@ __global__ void k_links_soa_to_aos(const double2 *__restrict__ soa, double *__re
 #pragma unroll
   for (int k = 0; k < 9; k++) { double2 v = s[(size_t)k * Vh]; d[2 * k] = v.x; d[2 * k + 1] = v.y; }
 }
-// out[0]: bits of the largest |component|; out[1]: non-zero when one is not finite
-__global__ void k_links_maxabs(const double2 *__restrict__ src, size_t n, unsigned long long *out) {
-  double m = 0;
+// What the reduced-precision and integer forms need to know of a link field:
+// its largest |component|, the smallest of its matrices that are not zero (by
+// their largest component), and whether one is not finite.  All zero before
+// the launch.
+struct LinkStats {
+  unsigned long long max, inv_min, bad;   // bits of the doubles; inv_min: of the smallest, complemented
+};
+__global__ void k_links_stats(const double2 *__restrict__ src, int Vh, LinkStats *out) {
+  double top = 0, low = __longlong_as_double(0x7ff0000000000000ll);
   bool bad = false;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double2 v = src[i];
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-    bad = bad || !isfinite(v.x) || !isfinite(v.y);
+  for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += gridDim.x * blockDim.x) {
+    const double2 *s = src + (size_t)blockIdx.y * 9 * Vh + h;   // par*4+dir
+    double m = 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const double2 v = s[(size_t)k * Vh];
+      m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+      bad = bad || !isfinite(v.x) || !isfinite(v.y);
+    }
+    top = fmax(top, m);
+    if (m > 0) low = fmin(low, m);
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int o = 16; o > 0; o >>= 1) {
+    top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    low = fmin(low, __shfl_xor_sync(0xffffffffu, low, o));
+  }
   bad = __any_sync(0xffffffffu, bad);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(out, (unsigned long long)__double_as_longlong(m));
-    if (bad) atomicMax(out + 1, 1ull);
+    atomicMax(&out->max, (unsigned long long)__double_as_longlong(top));
+    if (top > 0) atomicMax(&out->inv_min, ~(unsigned long long)__double_as_longlong(low));
+    if (bad) atomicMax(&out->bad, 1ull);
   }
 }
 // the FP32, FP16 and integer forms of a link field in one pass over its
@@ -237,6 +254,7 @@ __global__ void k_links_lowprec(const double2 *__restrict__ src, float4 *__restr
   for (int k = 0; k < 9; k++) {
     const double2 u = s[(size_t)k * Vh];
     f[k] = make_float2((float)u.x, (float)u.y);
+    if (!fx) continue;   // links that the integer form does not suit
     int4 w;
     fx_split(fx_scale(u.x, fx_exp) + 8, w.x, w.y);  // + 8: rounds the cut at 16
     fx_split(fx_scale(u.y, fx_exp) + 8, w.z, w.w);
@@ -331,33 +349,40 @@ int links_make_lowprec(LinkSlot &s) {
   MKS_TRY(need(s.lng16b, n32b));
   MKS_TRY(need(s.fat_fx, nfx));
   MKS_TRY(need(s.lng_fx, nfx));
-  // largest component of either field: the FP16 scales and the integers' exponent
-  unsigned long long *mx, bits[4];
-  MKS_TRY(dev_alloc((void **)&mx, sizeof bits));
-  MKS_CUDA(cudaMemsetAsync(mx, 0, sizeof bits, c.stream));
-  k_links_maxabs<<<c.sm_count * 4, 256, 0, c.stream>>>(s.fat64, nfx, mx);
-  k_links_maxabs<<<c.sm_count * 4, 256, 0, c.stream>>>(s.lng64, nfx, mx + 2);
-  MKS_CUDA(cudaMemcpyAsync(bits, mx, sizeof bits, cudaMemcpyDeviceToHost, c.stream));
+  // the FP16 scales, and the integers' exponents if they serve these links
+  LinkStats *dst, st[2];
+  MKS_TRY(dev_alloc((void **)&dst, sizeof st));
+  MKS_CUDA(cudaMemsetAsync(dst, 0, sizeof st, c.stream));
+  const dim3 sgrid((c.sm_count + 1) / 2, 8);
+  k_links_stats<<<sgrid, 256, 0, c.stream>>>(s.fat64, Vh, dst);
+  k_links_stats<<<sgrid, 256, 0, c.stream>>>(s.lng64, Vh, dst + 1);
+  MKS_CUDA(cudaMemcpyAsync(st, dst, sizeof st, cudaMemcpyDeviceToHost, c.stream));
   MKS_CUDA(cudaStreamSynchronize(c.stream));
-  dev_free(mx);
-  double m[2];
-  memcpy(&m[0], &bits[0], 8);
-  memcpy(&m[1], &bits[2], 8);
-  s.fat16scale = (float)m[0];
-  s.lng16scale = (float)m[1];
-  s.fx_special = bits[1] || bits[3];
-  int ex = -1021;
-  if (!s.fx_special) {
-    const double top = m[0] > m[1] ? m[0] : m[1];
-    int k = 0;
-    frexp(top, &k);
-    if (top > 0 && k > ex) ex = k;
+  dev_free(dst);
+  double top[2], low[2];
+  int ex[2] = {-1021, -1021};
+  s.fx_plain = 0;
+  for (int k = 0; k < 2; k++) {
+    memcpy(&top[k], &st[k].max, 8);
+    const unsigned long long b = ~st[k].inv_min;
+    memcpy(&low[k], &b, 8);
+    if (st[k].bad) s.fx_plain = 1;
+    if (st[k].bad || !(top[k] > 0)) continue;
+    if (ldexp(low[k], FX_SPREAD) < top[k]) s.fx_plain = 1;
+    int e = 0;
+    frexp(top[k], &e);
+    if (e > ex[k]) ex[k] = e;
   }
-  s.fx_exp = ex;
-  const float inv[2] = {m[0] > 0 ? (float)(1.0 / m[0]) : 0.f, m[1] > 0 ? (float)(1.0 / m[1]) : 0.f};
+  s.fat16scale = (float)top[0];
+  s.lng16scale = (float)top[1];
+  s.fat_exp = ex[0];
+  s.lng_exp = ex[1];
+  const float inv[2] = {top[0] > 0 ? (float)(1.0 / top[0]) : 0.f, top[1] > 0 ? (float)(1.0 / top[1]) : 0.f};
   const dim3 grid(grid_for(Vh, 256), 8);
-  k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.fat64, s.fat32a, s.fat32b, s.fat16a, s.fat16b, s.fat_fx, inv[0], ex, Vh);
-  k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.lng64, s.lng32a, s.lng32b, s.lng16a, s.lng16b, s.lng_fx, inv[1], ex, Vh);
+  k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.fat64, s.fat32a, s.fat32b, s.fat16a, s.fat16b,
+                                              s.fx_plain ? nullptr : s.fat_fx, inv[0], ex[0], Vh);
+  k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.lng64, s.lng32a, s.lng32b, s.lng16a, s.lng16b,
+                                              s.fx_plain ? nullptr : s.lng_fx, inv[1], ex[1], Vh);
   c.launches += 4;
   MKS_CUDA(cudaGetLastError());
   return MKS_OK;

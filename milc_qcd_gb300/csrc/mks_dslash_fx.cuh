@@ -19,7 +19,9 @@
 // aligned to their largest exponent.  The result is written as blocks (the
 // first D of D_eo D_oe: the second reads them as they are), as FP64 SoA, or
 // in MILC's AoS layout.  A site with an infinity or a NaN among its
-// neighbours, or a slot whose links hold one, is done in plain FP64.
+// neighbours is done in plain FP64; so is a slot whose links do not suit the
+// integer form, by a kernel of its own (k_dslash_raw) on fields that hold
+// doubles in the place of the blocks' integers.
 #pragma once
 #include "mks_fixed.cuh"
 #include "mks_dslash.cuh"
@@ -35,7 +37,7 @@ struct FxArgs {
   int rev;                 // blocks take the sites in reverse order
   FxLinks fat, lng;
   const double2 *fat64, *lng64;   // the same links for sites done in plain FP64
-  int EL, special;
+  int EL, dE;                     // exponent of the fat links, and how far the Naik links' is above it
   FxVec in[MAXSRC];        // by source; by output parity in a launch of two grid rows (one source)
   FxVec outq[MAXSRC];
   double2 *out[MAXSRC];    // SoA, or MILC's AoS field
@@ -46,7 +48,7 @@ struct FxArgs {
   double *totals;
 };
 
-// one site in plain FP64 (a neighbour or a link is not finite)
+// one site in plain FP64 (a neighbour is not finite)
 static __device__ __noinline__ void fx_site_f64(const Geom &g, const double2 *fat, const double2 *lng, const FxVec &in,
                                                 int par, int h, int x, int y, int z, int t, double *out) {
   const LinkF64 F = {fat}, Lg = {lng};
@@ -73,6 +75,48 @@ static __device__ __noinline__ void fx_site_f64(const Geom &g, const double2 *fa
     amv_sub(Lg.load(1 - par, mu, hb3, g.Vh), vec(hb3), acc);
   }
   for (int c = 0; c < 3; c++) { out[2 * c] = acc.c[c].re; out[2 * c + 1] = acc.c[c].im; }
+}
+
+// the epilogue's sums over the block (up to W warps, warp w of source group w
+// % G) and the grid, and the finisher
+template <int W, int NB, class Fin>
+__device__ __forceinline__ void fx_sums(const double (&sums)[NB][3], const FxArgs &a, const Fin &fin) {
+  __shared__ double smem[W * NB * 3];
+  __shared__ double bt[MAXSRC * 3];
+  __shared__ double tot[MAXSRC * 3];
+  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nwarps = (int)blockDim.x >> 5, G = a.G;
+#pragma unroll
+  for (int s = 0; s < NB; s++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const double v = warp_sum(sums[s][k]);
+      if (lane == 0) smem[(warp * NB + s) * 3 + k] = v;
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < G * NB * 3; i += blockDim.x) {   // warp order
+    const int g0 = i / (NB * 3), j = i - g0 * NB * 3;
+    double v = 0;
+    for (int w = g0; w < nwarps; w += G) v += smem[w * NB * 3 + j];
+    bt[i] = v;
+  }
+  __syncthreads();
+  if (grid_reduce_last(bt, G * NB * 3, a.red, tot)) {
+    if (threadIdx.x == 0)
+      for (int i = 0; i < a.nsrc * 3; i++) a.totals[i] = tot[i];
+    __syncthreads();
+    fin(tot, a.nsrc);
+  }
+}
+
+// a site's result stored in MILC's AoS field
+__device__ __forceinline__ void fx_store_aos(double2 *d, const double (&v)[6]) {
+  if (((uintptr_t)d & 15) == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) d[c] = make_double2(v[2 * c], v[2 * c + 1]);
+  } else {  // a caller's field on an 8-byte boundary
+#pragma unroll
+    for (int k = 0; k < 6; k++) reinterpret_cast<double *>(d)[k] = v[k];
+  }
 }
 
 template <int SPLIT, bool DENSE, int NB, int OUT, int EPI, class Fin>
@@ -102,14 +146,15 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
   const int c0[4] = {x, y, z, t}, L[4] = {g.nx, g.ny, g.nz, g.nt};
   int E[NB];
 #pragma unroll
-  for (int s = 0; s < NB; s++) E[s] = FX_ZERO;
+  for (int s = 0; s < NB; s++) E[s] = 2 * FX_ZERO;
 #pragma unroll
   for (int k = 0; k < 4 / SPLIT; k++) {
     int f1, b1, f3, b3;
     nbr4(g, c0, L, SPLIT == 1 ? k : m0, f1, b1, f3, b3);
 #pragma unroll
     for (int s = 0; s < NB; s++)
-      E[s] = max(max(max(E[s], __ldg(in[s].e + f1)), max(__ldg(in[s].e + b1), __ldg(in[s].e + f3))), __ldg(in[s].e + b3));
+      E[s] = max(max(E[s], max(__ldg(in[s].e + f1), __ldg(in[s].e + b1))),
+                 max(__ldg(in[s].e + f3), __ldg(in[s].e + b3)) + a.dE);
   }
   if (SPLIT > 1) {
 #pragma unroll
@@ -135,14 +180,14 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
       for (int s = 0; s < NB; s++) {
         s64 q[6];
         fx_load(in[s], nf, Vh, q);
-        fx_operand<1>(q, min(E[s] - __ldg(in[s].e + nf), 63), o[s]);
+        fx_operand<1>(q, min((kind ? E[s] - a.dE : E[s]) - __ldg(in[s].e + nf), 63), o[s]);
       }
       fx_mv<false, NB>(U, par, mu, h, Vh, o, acc);
 #pragma unroll
       for (int s = 0; s < NB; s++) {
         s64 q[6];
         fx_load(in[s], nbk, Vh, q);
-        fx_operand<-1>(q, min(E[s] - __ldg(in[s].e + nbk), 63), o[s]);
+        fx_operand<-1>(q, min((kind ? E[s] - a.dE : E[s]) - __ldg(in[s].e + nbk), 63), o[s]);
       }
       fx_mv<true, NB>(U, op, mu, nbk, Vh, o, acc);
     }
@@ -179,13 +224,12 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
 #pragma unroll
     for (int k = 0; k < 6; k++) { mag |= (u64)(T[k] ^ (T[k] >> 63)); any |= f[k]; }
     const int sh = min(28, __clzll((s64)mag) - 4);
-    int e = (mag | any) == 0 || E[s] == FX_ZERO ? FX_ZERO : E[s] + a.EL + 4 - sh;
+    int e = (mag | any) == 0 || E[s] < FX_ZERO / 2 ? FX_ZERO : E[s] + a.EL + 4 - sh;
     s64 q[6];
 #pragma unroll
     for (int k = 0; k < 6; k++) q[k] = sh > 0 ? (s64)(((u64)T[k] << sh) + (f[k] >> (28 - sh))) : T[k] >> -sh;
-    const bool plain = E[s] == FX_SPECIAL || a.special;
     double v[6];
-    if (plain) {
+    if (E[s] > FX_SPECIAL / 2) {
       fx_site_f64(g, a.fat64, a.lng64, in[s], par, h, x, y, z, t, v);
       if (OUT == FX_OUT_BLOCK) fx_encode(v, q, e);
       if (LANES > 1) {
@@ -203,14 +247,7 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
     if (OUT == FX_OUT_BLOCK) {
       fx_store(a.outq[S], h, Vh, q, e);
     } else if (OUT == FX_OUT_AOS) {
-      double2 *d = a.out[S] + ((size_t)par * Vh + h) * 3;
-      if (((uintptr_t)d & 15) == 0) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) d[c] = make_double2(v[2 * c], v[2 * c + 1]);
-      } else {  // a caller's field on an 8-byte boundary
-#pragma unroll
-        for (int k = 0; k < 6; k++) reinterpret_cast<double *>(d)[k] = v[k];
-      }
+      fx_store_aos(a.out[S] + ((size_t)par * Vh + h) * 3, v);
     } else {
       if (EPI == EPI_AXPY) {
         const double cf = a.coef[S];
@@ -228,32 +265,7 @@ __device__ __forceinline__ void dslash_fx_body(const FxArgs &a, const Fin &fin) 
       for (int c = 0; c < NC; c++) a.out[S][(size_t)(LANES > 1 ? m0 : c) * Vh + h] = make_double2(v[2 * c], v[2 * c + 1]);
     }
   }
-  if (EPI == EPI_AXPY) {
-    __shared__ double smem[8 * NB * 3];
-    __shared__ double bt[MAXSRC * 3];
-    __shared__ double tot[MAXSRC * 3];
-#pragma unroll
-    for (int s = 0; s < NB; s++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const double v = warp_sum(sums[s][k]);
-        if (lane == 0) smem[(warp * NB + s) * 3 + k] = v;
-      }
-    __syncthreads();
-    for (int i = threadIdx.x; i < G * NB * 3; i += blockDim.x) {   // warp order
-      const int g0 = i / (NB * 3), j = i - g0 * NB * 3;
-      double v = 0;
-      for (int w = g0; w < nwarps; w += G) v += smem[w * NB * 3 + j];
-      bt[i] = v;
-    }
-    __syncthreads();
-    if (grid_reduce_last(bt, G * NB * 3, a.red, tot)) {
-      if (threadIdx.x == 0)
-        for (int i = 0; i < a.nsrc * 3; i++) a.totals[i] = tot[i];
-      __syncthreads();
-      fin(tot, a.nsrc);
-    }
-  }
+  if (EPI == EPI_AXPY) fx_sums<8, NB>(sums, a, fin);
 }
 
 template <int SPLIT, int NB, int OUT, int EPI, class Fin>
@@ -273,6 +285,50 @@ __global__ void __launch_bounds__(256, NB == 1 ? 2 : 1) k_dslash_fx(const FxArgs
 template <int OUT, int EPI, class Fin>
 __global__ void __launch_bounds__(128, 5) k_dslash_fx_dense(const FxArgs a, const Fin fin) {
   dslash_fx_body<4, true, 1, OUT, EPI, Fin>(a, fin);
+}
+
+// D_eo in plain FP64 on links that the integer form does not suit: in[].q and
+// out[] hold doubles (a field of blocks keeps its size and its place).  One
+// thread per site and source, sources by warps.  Bound by the FP64 rate (576
+// fmas a site at 2 lanes per clock and SM).
+template <int OUT, int EPI, class Fin>
+__global__ void __launch_bounds__(512) k_dslash_raw(const FxArgs a, const Fin fin) {
+  if (a.skip && *a.skip) return;
+  const Geom &g = a.g;
+  const int Vh = g.Vh, par = a.out_par ^ (int)blockIdx.y, G = a.G;
+  const int bid = a.rev ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nwarps = (int)blockDim.x >> 5;
+  const int S = warp % G + (int)blockIdx.y;   // blocks hold a multiple of G = nsrc warps
+  const int h = (bid * nwarps + warp) / G * 32 + lane;
+  double sums[1][3] = {{0, 0, 0}};
+  if (h < Vh) {
+    int x, y, z, t;
+    site_coords(g, par, h, x, y, z, t);
+    const int c0[4] = {x, y, z, t};
+    const VecF64 in = {reinterpret_cast<double2 *>(a.in[S].q)};
+    V3<double> acc[1] = {{{{0, 0}, {0, 0}, {0, 0}}}};
+    site_terms<double, LinkF64, VecF64, 1, false>(LinkF64{a.fat64}, LinkF64{a.lng64}, &in, 1, 0, g, par, h, c0, acc);
+    double v[6] = {acc[0].c[0].re, acc[0].c[0].im, acc[0].c[1].re, acc[0].c[1].im, acc[0].c[2].re, acc[0].c[2].im};
+    if (EPI == EPI_AXPY) {
+      const double cf = a.coef[S];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double2 pv = __ldg(a.p[S] + (size_t)c * Vh + h), rv = __ldg(a.r[S] + (size_t)c * Vh + h);
+        v[2 * c] = fma(cf, pv.x, v[2 * c]);
+        v[2 * c + 1] = fma(cf, pv.y, v[2 * c + 1]);
+        sums[0][0] = fma(pv.x, v[2 * c], fma(pv.y, v[2 * c + 1], sums[0][0]));
+        sums[0][1] = fma(rv.x, v[2 * c], fma(rv.y, v[2 * c + 1], sums[0][1]));
+        sums[0][2] = fma(v[2 * c], v[2 * c], fma(v[2 * c + 1], v[2 * c + 1], sums[0][2]));
+      }
+    }
+    if (OUT == FX_OUT_AOS) {
+      fx_store_aos(a.out[S] + ((size_t)par * Vh + h) * 3, v);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; c++) a.out[S][(size_t)c * Vh + h] = make_double2(v[2 * c], v[2 * c + 1]);
+    }
+  }
+  if (EPI == EPI_AXPY) fx_sums<16, 1>(sums, a, fin);
 }
 
 }  // namespace mks

@@ -143,7 +143,14 @@ __device__ __forceinline__ void fx_operand(const s64 (&q)[6], int shift, FxOpera
 }
 
 // Links: an entry's halves {a_h, a_l, b_h, b_l} (a + ib), value
-// (h 2^28 + l) 2^(EL-56), one exponent EL for the slot's fat and Naik links
+// (h 2^28 + l) 2^(EL-56), one exponent EL for the slot's fat links and one for
+// its Naik links.  A link keeps 2^-57 of the largest of its kind, so the form
+// is for links of one size: within FX_SPREAD bits, measured by a matrix's
+// largest component, every link keeps the 53 bits of a double.  Smeared links
+// lie within 0.2 bits of each other on smooth fields (exp(i 0.3 H)) and within
+// 1.7 where the thin links are random; a slot that does not fit is done in
+// plain FP64 (k_dslash_raw).
+constexpr int FX_SPREAD = 4;
 struct FxLinks {
   const int4 *p;  // [par][dir][9][Vh]
 };

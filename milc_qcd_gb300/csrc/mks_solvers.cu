@@ -158,10 +158,15 @@ struct PtrSet32 { float2 *p[BLAS_MAXSRC]; };
 struct PtrSet16 { __half2 *p[BLAS_MAXSRC]; float *n[BLAS_MAXSRC]; };
 
 // a site's FP64 components stored as a block of integers (mks_fixed.cuh), the
-// form that the FP64 D_eo reads
-__device__ __forceinline__ void fx_put(const FxVec &d, int h, int Vh, const double (&v)[6]) {
+// form that the FP64 D_eo reads, or as they are (raw: for k_dslash_raw)
+__device__ __forceinline__ void fx_put(const FxVec &d, int h, int Vh, const double (&v)[6], int raw) {
   s64 q[6];
   int e;
+  if (raw) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) reinterpret_cast<double2 *>(d.q)[(size_t)c * Vh + h] = make_double2(v[2 * c], v[2 * c + 1]);
+    return;
+  }
   fx_encode(v, q, e);
   fx_store(d, h, Vh, q, e);
 }
@@ -170,7 +175,7 @@ __device__ __forceinline__ void fx_put(const FxVec &d, int h, int Vh, const doub
 struct OpToBlocks {
   const double2 *v[BLAS_MAXSRC];
   FxVec q[BLAS_MAXSRC];
-  int Vh;
+  int Vh, raw;
   __device__ void operator()(int h, int s, double *) const {
     double w[6];
 #pragma unroll
@@ -179,7 +184,7 @@ struct OpToBlocks {
       w[2 * c] = a.x;
       w[2 * c + 1] = a.y;
     }
-    fx_put(q[s], h, Vh, w);
+    fx_put(q[s], h, Vh, w, raw);
   }
 };
 
@@ -209,7 +214,7 @@ struct OpResid64 {
   const CgState *st;
   double msq4[BLAS_MAXSRC];
   int map[BLAS_MAXSRC], tzero[BLAS_MAXSRC];
-  int Vh, setp;           // setp: p <- r (FP64 solve)
+  int Vh, setp, raw;      // setp: p <- r (FP64 solve)
   __device__ void operator()(int h, int s, double *out) const {
     if (st && st[map[s]].status != ST_HOST) { out[0] = 0; out[1] = 0; return; }
     double a = 0, xx = 0, pv[6];
@@ -225,7 +230,7 @@ struct OpResid64 {
       a += rv.x * rv.x + rv.y * rv.y;
       xx += xv.x * xv.x + xv.y * xv.y;
     }
-    if (setp) fx_put(pq[s], h, Vh, pv);
+    if (setp) fx_put(pq[s], h, Vh, pv, raw);
     out[0] = a;
     out[1] = (xx == 0) ? 1.0 : a / xx;
   }
@@ -259,7 +264,7 @@ template <typename R> struct OpUpdate {
   float *p16n[BLAS_MAXSRC];
   FxVec pq[BLAS_MAXSRC];  // FP64: p as blocks
   const CgState *st;
-  int Vh, relres;
+  int Vh, relres, raw;
   // split epilogue: ttt holds D D p only and the update forms
   // ttt - msq4 p itself (the same fma as the fused D_eo epilogue)
   int fold;
@@ -285,7 +290,7 @@ template <typename R> struct OpUpdate {
     }
     if constexpr (sizeof(R) == 8) {
       const double w[6] = {pn.c[0].re, pn.c[0].im, pn.c[1].re, pn.c[1].im, pn.c[2].re, pn.c[2].im};
-      fx_put(pq[s], h, Vh, w);
+      fx_put(pq[s], h, Vh, w, raw);
     } else if (p16[s]) {
       float m = 0.f;
 #pragma unroll
@@ -992,6 +997,27 @@ static int launch_fx_as(FxArgs &a, const Fin &fin, int mult, int rows) {
   return MKS_OK;
 }
 
+// the same in plain FP64 on links that the integer form does not suit; a
+// field of blocks holds doubles there
+template <int OUT, int EPI, class Fin>
+static int launch_raw(FxArgs &a, const Fin &fin, int mult, int rows) {
+  Context &c = ctx();
+  if (OUT == FX_OUT_BLOCK)
+    for (int s = 0; s < a.nsrc; s++) a.out[s] = reinterpret_cast<double2 *>(a.outq[s].q);
+  a.G = a.nsrc;
+  const int block = 32 * a.G * mult, grid = grid_for(c.Vh, 32 * mult);
+  if (EPI == EPI_AXPY) {
+    MKS_TRY(ensure_red(3 * a.G));
+    a.red = c.red;
+  }
+  (EPI == EPI_AXPY ? g_shape_epi : g_shape)[MKS_PREC_DOUBLE][a.nsrc] = {a.G, 1, block, 0, 0, 0, 0};
+  timing_begin(MKS_K_DSLASH_F64);
+  k_dslash_raw<OUT == FX_OUT_BLOCK ? FX_OUT_F64 : OUT, EPI, Fin><<<dim3(grid, rows), block, 0, c.stream>>>(a, fin);
+  timing_end(MKS_K_DSLASH_F64);
+  MKS_CUDA(cudaGetLastError());
+  return MKS_OK;
+}
+
 // rows = 2: both parities of one source in one launch (in[y], out[y] of
 // output parity y).  One source per thread up to 8 (blocks of one warp per
 // source share their sites' links in L1), two beyond.
@@ -1003,9 +1029,10 @@ static int launch_fx(const LinkSlot &sl, FxArgs &a, const Fin &fin, int rows = 1
   a.lng = {sl.lng_fx};
   a.fat64 = sl.fat64;
   a.lng64 = sl.lng64;
-  a.EL = sl.fx_exp;
-  a.special = sl.fx_special;
+  a.EL = sl.fat_exp;
+  a.dE = sl.lng_exp - sl.fat_exp;
   const int mult = a.nsrc == 1 ? 4 : a.nsrc == 2 ? 2 : 1;
+  if (sl.fx_plain) return launch_raw<OUT, EPI>(a, fin, mult, rows);
   if (a.nsrc <= 8 && c.Vh * a.nsrc * rows < (size_t)c.sm_count * FX_SPLIT_THREADS)
     return launch_fx_as<4, 1, OUT, EPI>(a, fin, mult > 2 ? 2 : mult, rows);
   if constexpr (OUT != FX_OUT_AOS) {
@@ -1028,11 +1055,11 @@ static int dslash_blocks(const LinkSlot &sl, int out_par, int nsrc, const FxVec 
   return outq ? launch_fx<FX_OUT_BLOCK, EPI_PLAIN>(sl, a, FinNone()) : launch_fx<FX_OUT_F64, EPI_PLAIN>(sl, a, FinNone());
 }
 
-static int to_blocks(int nsrc, const double2 *const *v, const FxVec *q) {
+static int to_blocks(const LinkSlot &sl, int nsrc, const double2 *const *v, const FxVec *q) {
   OpToBlocks op;
   memset(&op, 0, sizeof op);
   for (int s = 0; s < nsrc; s++) { op.v[s] = v[s]; op.q[s] = q[s]; }
-  op.Vh = (int)ctx().Vh;
+  op.Vh = (int)ctx().Vh; op.raw = sl.fx_plain;
   return launch_site<OpToBlocks, 0, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, nsrc);
 }
 
@@ -1045,7 +1072,7 @@ static int ws_blocks(const std::string &name, FxVec *v) {
 static int dslash64(const LinkSlot &sl, int out_par, int nsrc, double2 *const *in, double2 *const *out) {
   FxVec q[MAXSRC];
   for (int s = 0; s < nsrc; s++) MKS_TRY(ws_blocks("fx_in" + std::to_string(s), &q[s]));
-  MKS_TRY(to_blocks(nsrc, in, q));
+  MKS_TRY(to_blocks(sl, nsrc, in, q));
   return dslash_blocks(sl, out_par, nsrc, q, nullptr, out, 1);
 }
 
@@ -1071,7 +1098,8 @@ static int slot_ok(int slot) {
 // public D
 
 // MILC AoS field (rows: one parity, or both from par0 on) to blocks
-__global__ void __launch_bounds__(128) k_aos_to_blocks(const double *__restrict__ aos, FxVec q0, FxVec q1, int par0, int Vh) {
+__global__ void __launch_bounds__(128) k_aos_to_blocks(const double *__restrict__ aos, FxVec q0, FxVec q1, int par0, int Vh,
+                                                        int raw) {
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= Vh) return;
   const int par = par0 ^ (int)blockIdx.y;
@@ -1079,12 +1107,13 @@ __global__ void __launch_bounds__(128) k_aos_to_blocks(const double *__restrict_
   double v[6];
 #pragma unroll
   for (int k = 0; k < 6; k++) v[k] = b[k];
-  fx_put(blockIdx.y ? q1 : q0, h, Vh, v);
+  fx_put(blockIdx.y ? q1 : q0, h, Vh, v, raw);
 }
-static int aos_to_blocks(const double *aos, FxVec q0, FxVec q1, int par0, int rows) {
+static int aos_to_blocks(const LinkSlot &sl, const double *aos, FxVec q0, FxVec q1, int par0, int rows) {
   Context &c = ctx();
   const int block = c.Vh < (size_t)c.sm_count * 128 ? 32 : 128;
-  k_aos_to_blocks<<<dim3(grid_for(c.Vh, block), rows), block, 0, c.stream>>>(aos, q0, q1, par0, (int)c.Vh);
+  k_aos_to_blocks<<<dim3(grid_for(c.Vh, block), rows), block, 0, c.stream>>>(aos, q0, q1, par0, (int)c.Vh,
+                                                                           sl.fx_plain);
   c.launches++;
   MKS_CUDA(cudaGetLastError());
   return MKS_OK;
@@ -1106,7 +1135,7 @@ static int dslash_dev_impl(const double *src_dev, double *dst_dev, int parity, i
     a.in[y] = in[1 - op];
     a.out[y] = (double2 *)dst_dev;
   }
-  MKS_TRY(aos_to_blocks(src_dev, in[1 - a.out_par], in[a.out_par], 1 - a.out_par, rows));
+  MKS_TRY(aos_to_blocks(c.slots[slot], src_dev, in[1 - a.out_par], in[a.out_par], 1 - a.out_par, rows));
   return launch_fx<FX_OUT_AOS, EPI_PLAIN>(c.slots[slot], a, FinNone(), rows);
 }
 
@@ -1205,7 +1234,7 @@ int dslash32_multi(int slot, int out_par, int nsrc, float2 *const *in, float2 *c
 // ttt <- D_par D_opar x  (FP64) for the sources listed; xq, tq scratch
 static int apply_DD64(const LinkSlot &sl, int par, int nsrc, double2 *const *x, const FxVec *xq, const FxVec *tq,
                       double2 *const *ttt) {
-  MKS_TRY(to_blocks(nsrc, x, xq));
+  MKS_TRY(to_blocks(sl, nsrc, x, xq));
   MKS_TRY(dslash_blocks(sl, 1 - par, nsrc, xq, tq, nullptr, 1));
   return dslash_blocks(sl, par, nsrc, tq, nullptr, ttt, 0);
 }
@@ -1239,7 +1268,7 @@ static int cg_iteration(const LinkSlot &sl, int par, int nsrc, int prec, const d
     OpUpdate<double> up;
     memset(&up, 0, sizeof up);
     for (int s = 0; s < nsrc; s++) { up.x[s] = f.x[s]; up.p[s] = f.p[s]; up.r[s] = f.r[s]; up.ttt[s] = f.ttt[s]; up.pq[s] = f.pq[s]; }
-    up.st = S.st; up.Vh = (int)ctx().Vh; up.relres = 0;
+    up.st = S.st; up.Vh = (int)ctx().Vh; up.relres = 0; up.raw = sl.fx_plain;
     MKS_TRY((launch_site<OpUpdate<double>, 1, FinCgUpdate>(MKS_K_BLAS, up, FinCgUpdate{S.st, S.skip}, S.skip, nsrc)));
     return MKS_OK;
   }
@@ -1429,7 +1458,8 @@ static int run_batch(const LinkSlot &sl, int par, int nsrc, int prec, const doub
   key_push(key, sl.fat64); key_push(key, sl.lng64); key_push(key, sl.fat32a); key_push(key, sl.lng32a);
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
-  key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fx_exp); key_push(key, sl.fx_special);
+  key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fat_exp); key_push(key, sl.lng_exp);
+  key_push(key, sl.fx_plain);
   key_push(key, S.st); key_push(key, S.skip); key_push(key, c.red.limbs); key_push(key, c.red.count);
   for (int s = 0; s < nsrc; s++) {
     key_push(key, msq4[s]);
@@ -1466,7 +1496,7 @@ static int true_residual(const LinkSlot &sl, int par, int nsrc, const double *ms
     op.msq4[k] = msq4[s]; op.map[k] = s; op.tzero[k] = xzero[s];
     fin.map[k] = s;
   }
-  op.st = S.st; op.Vh = (int)ctx().Vh; op.setp = setp;
+  op.st = S.st; op.Vh = (int)ctx().Vh; op.setp = setp; op.raw = sl.fx_plain;
   fin.st = S.st; fin.skip = S.skip;
   double *tot;
   MKS_TRY(wsv("cg_tot2", 2 * MAXSRC, &tot));
@@ -2265,7 +2295,7 @@ template <typename R, typename RS, int NF> struct MsUpdate {
   float *p16n;
   const MsState *st;
   int map[NF];        // field of a grid row
-  int Vh;
+  int Vh, raw;
 };
 
 // The update is elementwise but for |r|^2 and the shadows, so a thread takes
@@ -2365,7 +2395,7 @@ __global__ void __launch_bounds__(96 * NG) k_ms_update(const MsUpdate<R, RS, NF>
           double w[6];
 #pragma unroll
           for (int k = 0; k < 6; k++) w[k] = s_low[k][lane];
-          fx_put(a.cgq, h, Vh, w);
+          fx_put(a.cgq, h, Vh, w, a.raw);
         } else {
           float mx = 0.f;
 #pragma unroll
@@ -2428,7 +2458,7 @@ template <typename R, typename RS = R> struct OpShiftInit {
   const double2 *src;
   __half2 *p16;
   float *p16n;
-  int Vh, n;
+  int Vh, n, raw;
   __device__ void operator()(int h, int, double *out) const {
     double a = 0;
     float mx = 0.f;
@@ -2451,7 +2481,7 @@ template <typename R, typename RS = R> struct OpShiftInit {
         psim[j][i] = z;
       }
     }
-    if (sizeof(R) == 8) fx_put(cgq, h, Vh, w);
+    if (sizeof(R) == 8) fx_put(cgq, h, Vh, w, raw);
     if (p16) {
       float inv = mx > 0.f ? 1.f / mx : 0.f;
       p16n[h] = mx;
@@ -2585,6 +2615,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
     memset(&op, 0, sizeof op);
     for (int j = 0; j < nsh; j++) { op.psim[j] = psim[j]; op.pm[j] = pm[j]; }
     op.r = r; op.cgp = cgp; op.cgq = cgq; op.src = src64; op.p16 = p16; op.p16n = p16n; op.Vh = Vh; op.n = nsh;
+    op.raw = sl.fx_plain;
     double *tot;
     MKS_TRY(wsv("ms_tot", 4, &tot));
     MKS_TRY((launch_site<OpShiftInit<R, RS>, 1, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, 1, tot)));
@@ -2653,7 +2684,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
       MsUpdate<R, RS, 1> up;
       memset(&up, 0, sizeof up);
       for (int j = 0; j < nsh; j++) { up.psim[0][j] = psim[j]; up.pm[0][j] = pm[j]; }
-      up.r[0] = r; up.ttt[0] = ttt; up.cgp[0] = cgp; up.cgq = cgq; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh;
+      up.r[0] = r; up.ttt[0] = ttt; up.cgp[0] = cgp; up.cgq = cgq; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh; up.raw = sl.fx_plain;
       MKS_TRY(launch_ms_update(up, FinMsUpdate{st, skip}, skip, 1, nsh));
     }
     return MKS_OK;
@@ -2665,7 +2696,8 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
   key_push(key, sl.fat64); key_push(key, sl.lng64); key_push(key, sl.fat32a); key_push(key, sl.lng32a);
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
-  key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fx_exp); key_push(key, sl.fx_special);
+  key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fat_exp); key_push(key, sl.lng_exp);
+  key_push(key, sl.fx_plain);
   key_push(key, st); key_push(key, skip); key_push(key, tot); key_push(key, c.red.limbs); key_push(key, c.red.count);
   key_push(key, h.shift0); key_push(key, nsh); key_push(key, r); key_push(key, cgp); key_push(key, ttt);
   key_push(key, t); key_push(key, cgq.q); key_push(key, cgq.e); key_push(key, tq.q); key_push(key, tq.e);
