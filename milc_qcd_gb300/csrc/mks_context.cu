@@ -208,35 +208,36 @@ __global__ void k_links_soa_to_aos(const double2 *__restrict__ soa, double *__re
 }
 // What the reduced-precision and integer forms need to know of a link field:
 // its largest |component|, the smallest of its matrices that are not zero (by
-// their largest component), and whether one is not finite.  All zero before
-// the launch.
+// their largest component), and whether one is not finite or uneven
+// (mks_fixed.cuh).  All zero before the launch.
 struct LinkStats {
-  unsigned long long max, inv_min, bad;   // bits of the doubles; inv_min: of the smallest, complemented
+  unsigned long long max, inv_min, bad, uneven;   // bits of the doubles; inv_min: of the smallest, complemented
 };
 __global__ void k_links_stats(const double2 *__restrict__ src, int Vh, LinkStats *out) {
-  double top = 0, low = __longlong_as_double(0x7ff0000000000000ll);
-  bool bad = false;
+  u64 top = 0, low = ~0ull;
+  bool bad = false, uneven = false;
   for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += gridDim.x * blockDim.x) {
     const double2 *s = src + (size_t)blockIdx.y * 9 * Vh + h;   // par*4+dir
-    double m = 0;
+    FxShape f;
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-      const double2 v = s[(size_t)k * Vh];
-      m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-      bad = bad || !isfinite(v.x) || !isfinite(v.y);
-    }
-    top = fmax(top, m);
-    if (m > 0) low = fmin(low, m);
+    for (int k = 0; k < 9; k++) f.add(s[(size_t)k * Vh]);
+    bad = bad || f.bad;
+    uneven = uneven || f.uneven();
+    top = f.top > top ? f.top : top;
+    low = f.top != 0 && f.top < low ? f.top : low;
   }
   for (int o = 16; o > 0; o >>= 1) {
-    top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
-    low = fmin(low, __shfl_xor_sync(0xffffffffu, low, o));
+    const u64 t = __shfl_xor_sync(0xffffffffu, top, o), l = __shfl_xor_sync(0xffffffffu, low, o);
+    top = t > top ? t : top;
+    low = l < low ? l : low;
   }
   bad = __any_sync(0xffffffffu, bad);
+  uneven = __any_sync(0xffffffffu, uneven);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(&out->max, (unsigned long long)__double_as_longlong(top));
-    if (top > 0) atomicMax(&out->inv_min, ~(unsigned long long)__double_as_longlong(low));
+    atomicMax(&out->max, top);
+    if (top > 0) atomicMax(&out->inv_min, ~low);
     if (bad) atomicMax(&out->bad, 1ull);
+    if (uneven) atomicMax(&out->uneven, 1ull);
   }
 }
 // the FP32, FP16 and integer forms of a link field in one pass over its
@@ -366,7 +367,7 @@ int links_make_lowprec(LinkSlot &s) {
     memcpy(&top[k], &st[k].max, 8);
     const unsigned long long b = ~st[k].inv_min;
     memcpy(&low[k], &b, 8);
-    if (st[k].bad) s.fx_plain = 1;
+    if (st[k].bad || st[k].uneven) s.fx_plain = 1;
     if (st[k].bad || !(top[k] > 0)) continue;
     if (ldexp(low[k], FX_SPREAD) < top[k]) s.fx_plain = 1;
     int e = 0;

@@ -290,7 +290,8 @@ __global__ void __launch_bounds__(128, 5) k_dslash_fx_dense(const FxArgs a, cons
 // D_eo in plain FP64 on links that the integer form does not suit: in[].q and
 // out[] hold doubles (a field of blocks keeps its size and its place).  One
 // thread per site and source, sources by warps.  Bound by the FP64 rate (576
-// fmas a site at 2 lanes per clock and SM).
+// fmas a site at 2 lanes per clock and SM): 32^3x64 1.00 ms for one source and
+// 7.88 for 8 with the copy of the input.
 template <int OUT, int EPI, class Fin>
 __global__ void __launch_bounds__(512) k_dslash_raw(const FxArgs a, const Fin fin) {
   if (a.skip && *a.skip) return;

@@ -151,6 +151,38 @@ __device__ __forceinline__ void fx_operand(const s64 (&q)[6], int shift, FxOpera
 // 1.7 where the thin links are random; a slot that does not fit is done in
 // plain FP64 (k_dslash_raw).
 constexpr int FX_SPREAD = 4;
+
+// Components of a vector share an exponent, so a component far below the
+// others is as good as a matrix that mixes them makes its part in a result:
+// an entry of size 2^-k leaves 56 - k bits.  A matrix is uneven when it has an
+// entry more than FX_ENTRY bits, or a real or imaginary part more than FX_PART
+// bits, below its largest component: free, diagonal, real or block matrices,
+// which do not mix some components at all.  Fields with an uneven matrix are
+// done in plain FP64.  (Least entry and least part of 262,144 smeared links:
+// 13 and 25 bits below for thin links exp(i 0.3 H), 13 and 29 for random ones,
+// 17.5 and 29 for exp(i 0.05 H); four times the links bring an entry one bit
+// lower, a part two.)
+constexpr int FX_ENTRY = 28, FX_PART = 48;
+constexpr u64 FX_INF = 0x7ff0000000000000ull;
+struct FxShape {
+  u64 top, ent, part;   // bits of the largest component, the least entry and the least part
+  bool bad;             // a component is not finite (a NaN does not count as the largest)
+  __device__ __forceinline__ FxShape() : top(0), ent(~0ull), part(~0ull), bad(false) {}
+  __device__ __forceinline__ void add(double2 v) {
+    u64 x = (u64)__double_as_longlong(v.x) & ~(1ull << 63), y = (u64)__double_as_longlong(v.y) & ~(1ull << 63);
+    bad = bad || x >= FX_INF || y >= FX_INF;
+    if (x > FX_INF) x = 0;
+    if (y > FX_INF) y = 0;
+    const u64 e = x > y ? x : y, p = x > y ? y : x;
+    top = e > top ? e : top;
+    ent = e < ent ? e : ent;
+    part = p < part ? p : part;
+  }
+  __device__ __forceinline__ bool uneven() const {
+    const int t = (int)(top >> 52);
+    return top != 0 && (t - (int)(ent >> 52) > FX_ENTRY || t - (int)(part >> 52) > FX_PART);
+  }
+};
 struct FxLinks {
   const int4 *p;  // [par][dir][9][Vh]
 };

@@ -358,8 +358,8 @@ struct LinkSlot {
   __half2 *fat16b = nullptr, *lng16b = nullptr;          // [2][4][Vh]
   float fat16scale = 1.f, lng16scale = 1.f;
   // the links as integers (mks_fixed.cuh), one exponent for the fat and one
-  // for the long links; fx_plain: one of them is not finite, or they are of
-  // too different size for one exponent, and D_eo works in plain FP64
+  // for the long links; fx_plain: one of them is not finite or uneven, or they
+  // are of too different size for one exponent, and D_eo works in plain FP64
   int4 *fat_fx = nullptr, *lng_fx = nullptr;             // [2][4][9][Vh]
   int fat_exp = 0, lng_exp = 0, fx_plain = 0;
 };

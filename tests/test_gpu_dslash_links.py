@@ -128,3 +128,50 @@ def test_slots_keep_their_own_form(gpu, oracle_cls):
         m.dslash_fn_field(src, got, m.EVENANDODD, slot)
         want = orc.dslash(fat, lng, src, m.EVENANDODD)
         assert np.all(np.linalg.norm(got - want, axis=1) <= TOL * _site_bound(dims, fat, lng, src))
+
+def _free(dims, kind):
+    """Links with zero entries: free, diagonal, real, or an SU(2) block and a phase."""
+    V = int(np.prod(dims))
+    rng = np.random.default_rng(4)
+    M = np.zeros((V, 4, 3, 3), complex)
+    if kind == "free":
+        M[..., range(3), range(3)] = 1.0
+    elif kind == "diagonal":
+        M[..., range(3), range(3)] = np.exp(1j * rng.uniform(-3, 3, (V, 4, 3)))
+    elif kind == "real":
+        M[:] = np.linalg.qr(rng.standard_normal((V, 4, 3, 3)))[0]
+    else:
+        q = rng.standard_normal((V, 4, 4))
+        q /= np.linalg.norm(q, axis=-1, keepdims=True)
+        a, b = q[..., 0] + 1j * q[..., 1], q[..., 2] + 1j * q[..., 3]
+        M[..., 0, 0], M[..., 0, 1], M[..., 1, 0], M[..., 1, 1], M[..., 2, 2] = a, b, -b.conj(), a.conj(), 1.0
+    return np.ascontiguousarray(np.stack([M.real, M.imag], -1).reshape(V, 4, 18))
+
+
+@pytest.mark.parametrize("dims", LATTICES)
+@pytest.mark.parametrize("kind", ["free", "diagonal", "real", "block"])
+def test_small_components_beside_large_ones(gpu, oracle_cls, dims, kind):
+    """Links that do not mix all components: a component of 1e-20 beside one
+    of 1 keeps its digits."""
+    m = gpu
+    orc = oracle_cls(dims)
+    links = _free(dims, kind)
+    fat, lng = links, -links / 24
+    m.set_lattice(dims)
+    m.load_fn_links(fat, lng)
+    src = m.gen_vector(dims, 5, m.EVENANDODD).reshape(-1, 3, 2)
+    scale = np.ones((3, 2))
+    if kind == "real":
+        scale[:, 1] = 1e-20      # imaginary parts
+    else:
+        scale[2] = 1e-20         # the third colour
+        if kind != "block":
+            scale[1] = 1e-30
+    for s in (scale, 1.0 / scale):
+        v = np.ascontiguousarray((src * s).reshape(-1, 6))
+        got = np.zeros_like(v)
+        m.dslash_fn_field(v, got, m.EVENANDODD)
+        want = orc.dslash(fat, lng, v, m.EVENANDODD)
+        # per component: 256 roundings of the largest term of its own scale (|v| <= 6, |U| <= 1, 16 terms)
+        err = np.abs(got - want).reshape(-1, 3, 2)
+        assert np.all(err <= TOL * 16 * 6 * s)
