@@ -2,10 +2,11 @@
 // fermion-link residency (the part of the C ABI that replaces MILC's QUDA
 // set-up and link cache: generic/milc_to_quda_utilities.c:11-41,
 // generic_ks/fermion_links_fn_load_gpu.c:19-78, include/fn_links.h:9-17).
-#include <cstring>
 #include <cstdlib>
+#include <cstring>
 #include <cmath>
 #include <string>
+#include <unordered_map>
 #include "mks_internal.cuh"
 #include "mks_fixed.cuh"
 
@@ -26,20 +27,81 @@ int check_ready(bool need_lattice) {
   return MKS_OK;
 }
 
+// MKS_MEM_LIMIT (MiB): the most device memory that the library's own
+// allocations may add up to (0 or unset: what the device has)
+static size_t mem_limit() {
+  static long long v = -1;
+  if (v < 0) {
+    const char *e = getenv("MKS_MEM_LIMIT");
+    v = e && atoll(e) > 0 ? atoll(e) : 0;
+  }
+  return (size_t)v << 20;
+}
+static std::unordered_map<void *, size_t> g_sizes;   // with a limit: the live allocations
+static size_t g_used = 0;
+
+static cudaError_t try_alloc(void **p, size_t bytes) {
+  *p = nullptr;
+  const size_t limit = mem_limit();
+  if (limit && g_used + bytes > limit) return cudaErrorMemoryAllocation;
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+  } else if (limit) {
+    g_sizes[*p] = bytes;
+    g_used += bytes;
+  }
+  return e;
+}
+
 int dev_alloc(void **p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) return MKS_OK;
-  cudaError_t e = cudaMalloc(p, bytes);
+  cudaError_t e = try_alloc(p, bytes);
+  if (e != cudaSuccess && mem_release()) e = try_alloc(p, bytes);
   if (e != cudaSuccess) {
     set_last_error(e, "cudaMalloc", __FILE__, __LINE__);
-    cudaGetLastError();
     return MKS_ERR_NOMEM;
   }
   return MKS_OK;
 }
 
 void dev_free(void *p) {
-  if (p) cudaFree(p);
+  if (!p) return;
+  if (mem_limit()) {
+    auto it = g_sizes.find(p);
+    if (it != g_sizes.end()) {
+      g_used -= it->second;
+      g_sizes.erase(it);
+    }
+  }
+  cudaFree(p);
+}
+
+void mem_info(size_t *free_bytes, size_t *total) {
+  const size_t limit = mem_limit();
+  if (cudaMemGetInfo(free_bytes, total) != cudaSuccess) {
+    cudaGetLastError();
+    *free_bytes = *total = 0;
+  }
+  if (limit && limit < *total) {
+    *total = limit;
+    if (limit - g_used < *free_bytes) *free_bytes = limit - g_used;
+  }
+}
+
+bool mem_release() {
+  Context &c = g_ctx;
+  if (c.fx_busy || c.capture) return false;
+  bool any = false;
+  for (auto &s : c.slots) {
+    if (s.fat_fx || s.lng_fx) any = c.fx_off = true;
+    dev_free(s.fat_fx);
+    dev_free(s.lng_fx);
+    s.fat_fx = s.lng_fx = nullptr;
+    s.fx_made = 0;
+  }
+  return any;
 }
 
 // ---------------- timing ----------------
@@ -240,9 +302,9 @@ __global__ void k_links_stats(const double2 *__restrict__ src, int Vh, LinkStats
     if (uneven) atomicMax(&out->uneven, 1ull);
   }
 }
-// the FP32, FP16 and integer forms of a link field in one pass over its
-// FP64 entries (a pass each read them three times; HBM-bound: 144 B read and
-// 252 B written per link)
+// the FP32, FP16 and, where the slot keeps them, integer forms of a link field
+// in one pass over its FP64 entries (a pass each read them three times;
+// HBM-bound: 144 B read and 252 B written per link)
 __global__ void k_links_lowprec(const double2 *__restrict__ src, float4 *__restrict__ a32, float2 *__restrict__ b32,
                                 uint4 *__restrict__ a16, __half2 *__restrict__ b16, int4 *__restrict__ fx, float inv,
                                 int fx_exp, int Vh) {
@@ -255,7 +317,7 @@ __global__ void k_links_lowprec(const double2 *__restrict__ src, float4 *__restr
   for (int k = 0; k < 9; k++) {
     const double2 u = s[(size_t)k * Vh];
     f[k] = make_float2((float)u.x, (float)u.y);
-    if (!fx) continue;   // links that the integer form does not suit
+    if (!fx) continue;   // no integer copies
     int4 w;
     fx_split(fx_scale(u.x, fx_exp) + 8, w.x, w.y);  // + 8: rounds the cut at 16
     fx_split(fx_scale(u.y, fx_exp) + 8, w.z, w.w);
@@ -335,10 +397,28 @@ static void free_slot(LinkSlot &s) {
   s = LinkSlot();
 }
 
+// Room for the integer copies of a slot's links, 2304 bytes per site of a
+// parity beside the 4032 of its other forms: taken only if an eighth of the
+// memory stays free.  D_eo does without them where there is none.
+static bool alloc_fx(LinkSlot &s) {
+  const size_t bytes = (size_t)8 * 9 * g_ctx.Vh * sizeof(int4);
+  if (s.fat_fx && s.lng_fx) return true;
+  if (g_ctx.fx_off) return false;
+  size_t avail, total;
+  mem_info(&avail, &total);
+  if (avail < 2 * bytes + total / 8) return false;
+  if (try_alloc((void **)&s.fat_fx, bytes) == cudaSuccess && try_alloc((void **)&s.lng_fx, bytes) == cudaSuccess)
+    return true;
+  dev_free(s.fat_fx);
+  s.fat_fx = s.lng_fx = nullptr;
+  return false;
+}
+
 int links_make_lowprec(LinkSlot &s) {
   Context &c = g_ctx;
   int Vh = (int)c.Vh;
-  size_t n32a = (size_t)8 * 4 * Vh, n32b = (size_t)8 * Vh, nfx = (size_t)8 * 9 * Vh;
+  size_t n32a = (size_t)8 * 4 * Vh, n32b = (size_t)8 * Vh;
+  s.fx_made = 0;
   auto need = [](auto *&q, size_t n) { return q ? (int)MKS_OK : dev_alloc((void **)&q, n * sizeof *q); };
   MKS_TRY(need(s.fat32a, n32a));
   MKS_TRY(need(s.lng32a, n32a));
@@ -348,8 +428,6 @@ int links_make_lowprec(LinkSlot &s) {
   MKS_TRY(need(s.lng16a, n32a / 2));
   MKS_TRY(need(s.fat16b, n32b));
   MKS_TRY(need(s.lng16b, n32b));
-  MKS_TRY(need(s.fat_fx, nfx));
-  MKS_TRY(need(s.lng_fx, nfx));
   // the FP16 scales, and the integers' exponents if they serve these links
   LinkStats *dst, st[2];
   MKS_TRY(dev_alloc((void **)&dst, sizeof st));
@@ -362,14 +440,14 @@ int links_make_lowprec(LinkSlot &s) {
   dev_free(dst);
   double top[2], low[2];
   int ex[2] = {-1021, -1021};
-  s.fx_plain = 0;
+  bool plain = false;
   for (int k = 0; k < 2; k++) {
     memcpy(&top[k], &st[k].max, 8);
     const unsigned long long b = ~st[k].inv_min;
     memcpy(&low[k], &b, 8);
-    if (st[k].bad || st[k].uneven) s.fx_plain = 1;
+    if (st[k].bad || st[k].uneven) plain = true;
     if (st[k].bad || !(top[k] > 0)) continue;
-    if (ldexp(low[k], FX_SPREAD) < top[k]) s.fx_plain = 1;
+    if (ldexp(low[k], FX_SPREAD) < top[k]) plain = true;
     int e = 0;
     frexp(top[k], &e);
     if (e > ex[k]) ex[k] = e;
@@ -380,12 +458,14 @@ int links_make_lowprec(LinkSlot &s) {
   s.lng_exp = ex[1];
   const float inv[2] = {top[0] > 0 ? (float)(1.0 / top[0]) : 0.f, top[1] > 0 ? (float)(1.0 / top[1]) : 0.f};
   const dim3 grid(grid_for(Vh, 256), 8);
+  const bool fx = !plain && alloc_fx(s);
   k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.fat64, s.fat32a, s.fat32b, s.fat16a, s.fat16b,
-                                              s.fx_plain ? nullptr : s.fat_fx, inv[0], ex[0], Vh);
+                                              fx ? s.fat_fx : nullptr, inv[0], ex[0], Vh);
   k_links_lowprec<<<grid, 256, 0, c.stream>>>(s.lng64, s.lng32a, s.lng32b, s.lng16a, s.lng16b,
-                                              s.fx_plain ? nullptr : s.lng_fx, inv[1], ex[1], Vh);
+                                              fx ? s.lng_fx : nullptr, inv[1], ex[1], Vh);
   c.launches += 4;
   MKS_CUDA(cudaGetLastError());
+  s.fx_made = fx;
   return MKS_OK;
 }
 
@@ -464,6 +544,7 @@ static void free_lattice_fields() {
   c.aux_action = 0;
   dev_free(c.mom);
   c.mom = nullptr;
+  c.fx_off = false;
   gauge_free();
   rhmc_free();
 }

@@ -358,10 +358,11 @@ struct LinkSlot {
   __half2 *fat16b = nullptr, *lng16b = nullptr;          // [2][4][Vh]
   float fat16scale = 1.f, lng16scale = 1.f;
   // the links as integers (mks_fixed.cuh), one exponent for the fat and one
-  // for the long links; fx_plain: one of them is not finite or uneven, or they
-  // are of too different size for one exponent, and D_eo works in plain FP64
+  // for the long links.  fx_made: the copies hold these links; without them
+  // D_eo works in plain FP64: one of the links is not finite or uneven, they
+  // are of too different size for one exponent, or there was no memory.
   int4 *fat_fx = nullptr, *lng_fx = nullptr;             // [2][4][9][Vh]
-  int fat_exp = 0, lng_exp = 0, fx_plain = 0;
+  int fat_exp = 0, lng_exp = 0, fx_made = 0;
 };
 
 struct Context {
@@ -387,6 +388,10 @@ struct Context {
   // integration), and the one the current fermion links were built with
   int md_prec = MKS_PREC_DOUBLE;
   int links_prec = MKS_PREC_DOUBLE;
+  // integer copies of links: calls in progress that use them, and whether
+  // they had to be given back on this lattice (none are made any more)
+  int fx_busy = 0;
+  bool fx_off = false;
   // timing
   bool timing = false;
   double kernel_ms[MKS_K_COUNT] = {0};
@@ -418,9 +423,32 @@ void timing_begin(int family);
 void timing_end(int family);
 int timing_flush();
 
-// memory helpers (stream-ordered)
+// Device memory.  An allocation that fails is tried again after mem_release,
+// which gives back what the library holds for speed alone (the links' integer
+// copies); it does nothing while a call that uses them is in progress
+// (FxBusy): such a call ends with MKS_ERR_NOMEM and is repeated without them
+// (with_memory).
 int dev_alloc(void **p, size_t bytes);
 void dev_free(void *p);
+bool mem_release();
+// free and total device memory as the library may use it
+void mem_info(size_t *free_bytes, size_t *total);
+struct FxBusy {
+  FxBusy() { ctx().fx_busy++; }
+  ~FxBusy() { ctx().fx_busy--; }
+};
+template <class F> inline int with_memory(const F &once) {
+  int rc;
+  {
+    FxBusy busy;
+    rc = once();
+  }
+  if (rc == MKS_ERR_NOMEM && mem_release()) {
+    FxBusy busy;
+    rc = once();
+  }
+  return rc;
+}
 
 // named workspace buffers kept across calls, until the lattice changes (mks_solvers.cu)
 int ws(const std::string &name, size_t bytes, void **out);

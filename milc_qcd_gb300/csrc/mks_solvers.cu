@@ -997,8 +997,8 @@ static int launch_fx_as(FxArgs &a, const Fin &fin, int mult, int rows) {
   return MKS_OK;
 }
 
-// the same in plain FP64 on links that the integer form does not suit; a
-// field of blocks holds doubles there
+// the same in plain FP64 where the links have no integer copies; a field of
+// blocks holds doubles there
 template <int OUT, int EPI, class Fin>
 static int launch_raw(FxArgs &a, const Fin &fin, int mult, int rows) {
   Context &c = ctx();
@@ -1032,7 +1032,7 @@ static int launch_fx(const LinkSlot &sl, FxArgs &a, const Fin &fin, int rows = 1
   a.EL = sl.fat_exp;
   a.dE = sl.lng_exp - sl.fat_exp;
   const int mult = a.nsrc == 1 ? 4 : a.nsrc == 2 ? 2 : 1;
-  if (sl.fx_plain) return launch_raw<OUT, EPI>(a, fin, mult, rows);
+  if (!sl.fx_made) return launch_raw<OUT, EPI>(a, fin, mult, rows);
   if (a.nsrc <= 8 && c.Vh * a.nsrc * rows < (size_t)c.sm_count * FX_SPLIT_THREADS)
     return launch_fx_as<4, 1, OUT, EPI>(a, fin, mult > 2 ? 2 : mult, rows);
   if constexpr (OUT != FX_OUT_AOS) {
@@ -1059,7 +1059,7 @@ static int to_blocks(const LinkSlot &sl, int nsrc, const double2 *const *v, cons
   OpToBlocks op;
   memset(&op, 0, sizeof op);
   for (int s = 0; s < nsrc; s++) { op.v[s] = v[s]; op.q[s] = q[s]; }
-  op.Vh = (int)ctx().Vh; op.raw = sl.fx_plain;
+  op.Vh = (int)ctx().Vh; op.raw = !sl.fx_made;
   return launch_site<OpToBlocks, 0, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, nsrc);
 }
 
@@ -1067,12 +1067,29 @@ static int ws_blocks(const std::string &name, FxVec *v) {
   MKS_TRY(wsv(name + "_q", 3 * ctx().Vh, &v->q));
   return wsv(name + "_e", ctx().Vh, &v->e);
 }
+// scratch of a multi-shift's reliable update: D input, D of it, D D of it
+static int ws_rel(const LinkSlot &sl, FxVec *xq, FxVec *dq, double2 **dd) {
+  *xq = *dq = {nullptr, nullptr};
+  if (sl.fx_made) {
+    MKS_TRY(ws_blocks("ms_rel_x", xq));
+    MKS_TRY(wsv("ms_rel_t64_e", ctx().Vh, &dq->e));
+  }
+  MKS_TRY(wsv("ms_rel_t64", 3 * ctx().Vh, &dq->q));
+  return wsv("ms_rel_dd64", 3 * ctx().Vh, dd);
+}
+
+// an FP64 field in the place of blocks, for links without integer copies
+static FxVec raw_blocks(double2 *v) { return {reinterpret_cast<longlong2 *>(v), nullptr}; }
 
 // plain D on FP64 SoA fields, nsrc sources
 static int dslash64(const LinkSlot &sl, int out_par, int nsrc, double2 *const *in, double2 *const *out) {
   FxVec q[MAXSRC];
-  for (int s = 0; s < nsrc; s++) MKS_TRY(ws_blocks("fx_in" + std::to_string(s), &q[s]));
-  MKS_TRY(to_blocks(sl, nsrc, in, q));
+  if (sl.fx_made) {
+    for (int s = 0; s < nsrc; s++) MKS_TRY(ws_blocks("fx_in" + std::to_string(s), &q[s]));
+    MKS_TRY(to_blocks(sl, nsrc, in, q));
+  } else {
+    for (int s = 0; s < nsrc; s++) q[s] = raw_blocks(in[s]);
+  }
   return dslash_blocks(sl, out_par, nsrc, q, nullptr, out, 1);
 }
 
@@ -1113,7 +1130,7 @@ static int aos_to_blocks(const LinkSlot &sl, const double *aos, FxVec q0, FxVec 
   Context &c = ctx();
   const int block = c.Vh < (size_t)c.sm_count * 128 ? 32 : 128;
   k_aos_to_blocks<<<dim3(grid_for(c.Vh, block), rows), block, 0, c.stream>>>(aos, q0, q1, par0, (int)c.Vh,
-                                                                           sl.fx_plain);
+                                                                           !sl.fx_made);
   c.launches++;
   MKS_CUDA(cudaGetLastError());
   return MKS_OK;
@@ -1121,7 +1138,7 @@ static int aos_to_blocks(const LinkSlot &sl, const double *aos, FxVec q0, FxVec 
 
 // MILC field -> blocks of the parities that D reads -> D straight into the
 // caller's field: two launches for any parity.
-static int dslash_dev_impl(const double *src_dev, double *dst_dev, int parity, int slot) {
+static int dslash_dev_once(const double *src_dev, double *dst_dev, int parity, int slot) {
   Context &c = ctx();
   FxVec in[2];
   for (int k = 0; k < 2; k++) MKS_TRY(ws_blocks("ds_in" + std::to_string(k), &in[k]));
@@ -1137,6 +1154,9 @@ static int dslash_dev_impl(const double *src_dev, double *dst_dev, int parity, i
   }
   MKS_TRY(aos_to_blocks(c.slots[slot], src_dev, in[1 - a.out_par], in[a.out_par], 1 - a.out_par, rows));
   return launch_fx<FX_OUT_AOS, EPI_PLAIN>(c.slots[slot], a, FinNone(), rows);
+}
+static int dslash_dev_impl(const double *src_dev, double *dst_dev, int parity, int slot) {
+  return with_memory([&] { return dslash_dev_once(src_dev, dst_dev, parity, slot); });
 }
 
 }  // namespace mks
@@ -1183,7 +1203,9 @@ struct CgFields {
   float *p16n[MAXSRC], *t16n[MAXSRC];
 };
 
-static int alloc_cg_fields(CgFields &f, int nsrc, int prec) {
+// The fields of a solve on sl's links.  Where those have no integer copies D
+// reads the FP64 fields themselves: pq is p, and a residual's D input x.
+static int alloc_cg_fields(const LinkSlot &sl, CgFields &f, int nsrc, int prec) {
   Context &c = ctx();
   size_t n = 3 * c.Vh;
   for (int s = 0; s < nsrc; s++) {
@@ -1193,8 +1215,13 @@ static int alloc_cg_fields(CgFields &f, int nsrc, int prec) {
     MKS_TRY(wsv("cg_r" + k, n, &f.r[s]));
     MKS_TRY(wsv("cg_p" + k, n, &f.p[s]));
     MKS_TRY(wsv("cg_ttt" + k, n, &f.ttt[s]));
-    MKS_TRY(ws_blocks("cg_p" + k, &f.pq[s]));
-    MKS_TRY(ws_blocks("cg_t" + k, &f.tq[s]));
+    MKS_TRY(wsv("cg_t" + k, n, &f.tq[s].q));
+    f.tq[s].e = nullptr;
+    f.pq[s] = raw_blocks(f.p[s]);
+    if (sl.fx_made) {
+      MKS_TRY(ws_blocks("cg_p" + k, &f.pq[s]));
+      MKS_TRY(wsv("cg_t" + k + "_e", c.Vh, &f.tq[s].e));
+    }
     if (prec != MKS_PREC_DOUBLE) {
       MKS_TRY(wsv("cg_x32" + k, n, &f.x32[s]));
       MKS_TRY(wsv("cg_r32" + k, n, &f.r32[s]));
@@ -1231,11 +1258,14 @@ int dslash32_multi(int slot, int out_par, int nsrc, float2 *const *in, float2 *c
   return MKS_OK;
 }
 
-// ttt <- D_par D_opar x  (FP64) for the sources listed; xq, tq scratch
+// ttt <- D_par D_opar x  (FP64) for the sources listed; xq (with integer
+// copies of the links), tq scratch
 static int apply_DD64(const LinkSlot &sl, int par, int nsrc, double2 *const *x, const FxVec *xq, const FxVec *tq,
                       double2 *const *ttt) {
-  MKS_TRY(to_blocks(sl, nsrc, x, xq));
-  MKS_TRY(dslash_blocks(sl, 1 - par, nsrc, xq, tq, nullptr, 1));
+  FxVec in[MAXSRC];
+  for (int s = 0; s < nsrc; s++) in[s] = sl.fx_made ? xq[s] : raw_blocks(x[s]);
+  if (sl.fx_made) MKS_TRY(to_blocks(sl, nsrc, x, xq));
+  MKS_TRY(dslash_blocks(sl, 1 - par, nsrc, in, tq, nullptr, 1));
   return dslash_blocks(sl, par, nsrc, tq, nullptr, ttt, 0);
 }
 
@@ -1268,7 +1298,7 @@ static int cg_iteration(const LinkSlot &sl, int par, int nsrc, int prec, const d
     OpUpdate<double> up;
     memset(&up, 0, sizeof up);
     for (int s = 0; s < nsrc; s++) { up.x[s] = f.x[s]; up.p[s] = f.p[s]; up.r[s] = f.r[s]; up.ttt[s] = f.ttt[s]; up.pq[s] = f.pq[s]; }
-    up.st = S.st; up.Vh = (int)ctx().Vh; up.relres = 0; up.raw = sl.fx_plain;
+    up.st = S.st; up.Vh = (int)ctx().Vh; up.relres = 0; up.raw = !sl.fx_made;
     MKS_TRY((launch_site<OpUpdate<double>, 1, FinCgUpdate>(MKS_K_BLAS, up, FinCgUpdate{S.st, S.skip}, S.skip, nsrc)));
     return MKS_OK;
   }
@@ -1459,7 +1489,7 @@ static int run_batch(const LinkSlot &sl, int par, int nsrc, int prec, const doub
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
   key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fat_exp); key_push(key, sl.lng_exp);
-  key_push(key, sl.fx_plain);
+  key_push(key, sl.fx_made);
   key_push(key, S.st); key_push(key, S.skip); key_push(key, c.red.limbs); key_push(key, c.red.count);
   for (int s = 0; s < nsrc; s++) {
     key_push(key, msq4[s]);
@@ -1496,7 +1526,7 @@ static int true_residual(const LinkSlot &sl, int par, int nsrc, const double *ms
     op.msq4[k] = msq4[s]; op.map[k] = s; op.tzero[k] = xzero[s];
     fin.map[k] = s;
   }
-  op.st = S.st; op.Vh = (int)ctx().Vh; op.setp = setp; op.raw = sl.fx_plain;
+  op.st = S.st; op.Vh = (int)ctx().Vh; op.setp = setp; op.raw = !sl.fx_made;
   fin.st = S.st; fin.skip = S.skip;
   double *tot;
   MKS_TRY(wsv("cg_tot2", 2 * MAXSRC, &tot));
@@ -1756,13 +1786,13 @@ static int check_arg(const mks_invert_arg *arg, bool need_parity) {
 }
 
 // dev variant core: fields already in device AoS FP64 (MILC layout)
-static int congrad_block_dev(int nsrc, const double *const *src_dev, double *const *dst_dev, double mass, int slot,
-                             const mks_invert_arg *arg, mks_invert_result *res) {
+static int congrad_block_once(int nsrc, const double *const *src_dev, double *const *dst_dev, double mass, int slot,
+                              const mks_invert_arg *arg, mks_invert_result *res) {
   int par;
   MKS_TRY(parity_index(arg->parity, &par));
   CgFields f;
   memset(&f, 0, sizeof f);
-  MKS_TRY(alloc_cg_fields(f, nsrc, arg->prec));
+  MKS_TRY(alloc_cg_fields(ctx().slots[slot], f, nsrc, arg->prec));
   for (int s = 0; s < nsrc; s++) {
     MKS_TRY(vec_aos_to_soa64(src_dev[s], f.src[s], par));
     MKS_TRY(vec_aos_to_soa64(dst_dev[s], f.x[s], par));
@@ -1778,6 +1808,10 @@ static int congrad_block_dev(int nsrc, const double *const *src_dev, double *con
   for (int s = 0; s < nsrc; s++) MKS_TRY(vec_soa64_to_aos(f.x[s], dst_dev[s], par));
   MKS_CUDA(cudaStreamSynchronize(ctx().stream));
   return MKS_OK;
+}
+static int congrad_block_dev(int nsrc, const double *const *src_dev, double *const *dst_dev, double mass, int slot,
+                             const mks_invert_arg *arg, mks_invert_result *res) {
+  return with_memory([&] { return congrad_block_once(nsrc, src_dev, dst_dev, mass, slot, arg, res); });
 }
 
 // The device address of a page-locked host array mapped into the device
@@ -1922,13 +1956,13 @@ static int lin64(int nsrc, double2 *const *out, double alpha, double2 *const *a,
 // M^{-1} for nsrc sources given device AoS fields (generic_ks/mat_invert.c:328-483):
 //   tmp = M^dag src = 2m src - D src; even CG on tmp; dst_o = (src_o - D_oe dst_e)/(2m);
 //   odd CG on tmp (polish).
-static int mat_invert_dev(int nsrc, const double *const *src_dev, double *const *dst_dev, double mass, int slot,
-                          const mks_invert_arg *arg, mks_invert_result *res) {
+static int mat_invert_once(int nsrc, const double *const *src_dev, double *const *dst_dev, double mass, int slot,
+                           const mks_invert_arg *arg, mks_invert_result *res) {
   Context &c = ctx();
   const LinkSlot &sl = c.slots[slot];
   CgFields f;
   memset(&f, 0, sizeof f);
-  MKS_TRY(alloc_cg_fields(f, nsrc, arg->prec));
+  MKS_TRY(alloc_cg_fields(sl, f, nsrc, arg->prec));
   double2 *se[MAXSRC], *so[MAXSRC], *te[MAXSRC], *to[MAXSRC], *de[MAXSRC], *dn[MAXSRC];
   size_t n = 3 * c.Vh;
   for (int s = 0; s < nsrc; s++) {
@@ -1969,6 +2003,10 @@ static int mat_invert_dev(int nsrc, const double *const *src_dev, double *const 
   }
   MKS_CUDA(cudaStreamSynchronize(c.stream));
   return MKS_OK;
+}
+static int mat_invert_dev(int nsrc, const double *const *src_dev, double *const *dst_dev, double mass, int slot,
+                          const mks_invert_arg *arg, mks_invert_result *res) {
+  return with_memory([&] { return mat_invert_once(nsrc, src_dev, dst_dev, mass, slot, arg, res); });
 }
 
 static int mat_invert_host(int nsrc, const double *const *src, double *const *dst, double mass, int slot,
@@ -2046,12 +2084,7 @@ __global__ void k_flush(float4 *buf, size_t n, float v) {
 
 }  // namespace mks
 
-extern "C" int mks_bench_dslash(int prec, int nsrc, int parity, int slot, int iters, int flush_l2, double *ms) {
-  MKS_TRY(check_ready());
-  MKS_TRY(slot_ok(slot));
-  if (nsrc < 1 || nsrc > MAXSRC || iters < 1 || !ms) return MKS_ERR_ARG;
-  int par;
-  MKS_TRY(parity_index(parity, &par));
+static int bench_dslash_once(int prec, int nsrc, int par, int slot, int iters, int flush_l2, double *ms) {
   Context &c = ctx();
   const LinkSlot &sl = c.slots[slot];
   size_t n = 3 * c.Vh;
@@ -2112,6 +2145,15 @@ extern "C" int mks_bench_dslash(int prec, int nsrc, int parity, int slot, int it
   cudaEventDestroy(e1);
   *ms = total / iters;
   return MKS_OK;
+}
+
+extern "C" int mks_bench_dslash(int prec, int nsrc, int parity, int slot, int iters, int flush_l2, double *ms) {
+  MKS_TRY(check_ready());
+  MKS_TRY(slot_ok(slot));
+  if (nsrc < 1 || nsrc > MAXSRC || iters < 1 || !ms) return MKS_ERR_ARG;
+  int par;
+  MKS_TRY(parity_index(parity, &par));
+  return with_memory([&] { return bench_dslash_once(prec, nsrc, par, slot, iters, flush_l2, ms); });
 }
 
 // ====================================================================
@@ -2575,8 +2617,12 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
   MKS_TRY(wsv(std::string("ms_p") + tag, n, &cgp));
   MKS_TRY(wsv(std::string("ms_ttt") + tag, n, &ttt));
   if (sizeof(R) == 8) {
-    MKS_TRY(ws_blocks("ms_p", &cgq));
-    MKS_TRY(ws_blocks("ms_t", &tq));
+    cgq = raw_blocks((double2 *)cgp);
+    MKS_TRY(wsv("ms_t64", n, &tq.q));
+    if (sl.fx_made) {
+      MKS_TRY(ws_blocks("ms_p", &cgq));
+      MKS_TRY(wsv("ms_t64_e", c.Vh, &tq.e));
+    }
   } else {
     MKS_TRY(wsv(std::string("ms_t") + tag, n, &t));
   }
@@ -2615,7 +2661,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
     memset(&op, 0, sizeof op);
     for (int j = 0; j < nsh; j++) { op.psim[j] = psim[j]; op.pm[j] = pm[j]; }
     op.r = r; op.cgp = cgp; op.cgq = cgq; op.src = src64; op.p16 = p16; op.p16n = p16n; op.Vh = Vh; op.n = nsh;
-    op.raw = sl.fx_plain;
+    op.raw = !sl.fx_made;
     double *tot;
     MKS_TRY(wsv("ms_tot", 4, &tot));
     MKS_TRY((launch_site<OpShiftInit<R, RS>, 1, FinNone>(MKS_K_BLAS, op, FinNone(), nullptr, 1, tot)));
@@ -2684,7 +2730,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
       MsUpdate<R, RS, 1> up;
       memset(&up, 0, sizeof up);
       for (int j = 0; j < nsh; j++) { up.psim[0][j] = psim[j]; up.pm[0][j] = pm[j]; }
-      up.r[0] = r; up.ttt[0] = ttt; up.cgp[0] = cgp; up.cgq = cgq; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh; up.raw = sl.fx_plain;
+      up.r[0] = r; up.ttt[0] = ttt; up.cgp[0] = cgp; up.cgq = cgq; up.p16 = p16; up.p16n = p16n; up.st = st; up.Vh = Vh; up.raw = !sl.fx_made;
       MKS_TRY(launch_ms_update(up, FinMsUpdate{st, skip}, skip, 1, nsh));
     }
     return MKS_OK;
@@ -2697,7 +2743,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
   key_push(key, sl.fat32b); key_push(key, sl.lng32b); key_push(key, sl.fat16a); key_push(key, sl.lng16a);
   key_push(key, sl.fat16b); key_push(key, sl.lng16b); key_push(key, sl.fat16scale); key_push(key, sl.lng16scale);
   key_push(key, sl.fat_fx); key_push(key, sl.lng_fx); key_push(key, sl.fat_exp); key_push(key, sl.lng_exp);
-  key_push(key, sl.fx_plain);
+  key_push(key, sl.fx_made);
   key_push(key, st); key_push(key, skip); key_push(key, tot); key_push(key, c.red.limbs); key_push(key, c.red.count);
   key_push(key, h.shift0); key_push(key, nsh); key_push(key, r); key_push(key, cgp); key_push(key, ttt);
   key_push(key, t); key_push(key, cgq.q); key_push(key, cgq.e); key_push(key, tq.q); key_push(key, tq.e);
@@ -2713,9 +2759,7 @@ static int multishift_core(const LinkSlot &sl, int par, int prec, const double2 
       if (!wide) MKS_TRY(ms_fold(nsh, x64, psim_out));
       FxVec xq, dq;
       double2 *dd64;
-      MKS_TRY(ws_blocks("ms_rel_x", &xq));
-      MKS_TRY(ws_blocks("ms_rel_t", &dq));
-      MKS_TRY(wsv("ms_rel_dd64", n, &dd64));
+      MKS_TRY(ws_rel(sl, &xq, &dq, &dd64));
       double2 *xl = x64[h.j_low];
       MKS_TRY(apply_DD64(sl, par, 1, &xl, &xq, &dq, &dd64));
       OpMsResid op;
@@ -2888,9 +2932,7 @@ static int multishift_multi_core(const LinkSlot &sl, int par, int nf, const doub
       if (!wide) MKS_TRY(ms_fold(nsh[f], x64[f], (void *const *)psim[f]));
       FxVec xq, dq;
       double2 *dd64;
-      MKS_TRY(ws_blocks("ms_rel_x", &xq));
-      MKS_TRY(ws_blocks("ms_rel_t", &dq));
-      MKS_TRY(wsv("ms_rel_dd64", n, &dd64));
+      MKS_TRY(ws_rel(sl, &xq, &dq, &dd64));
       double2 *xl = x64[f][h.j_low];
       MKS_TRY(apply_DD64(sl, par, 1, &xl, &xq, &dq, &dd64));
       OpMsResid op;
@@ -2980,7 +3022,7 @@ static int multishift_multi_dev_once(int nf, const double *const *src_dev, const
     CgFields cf;
     memset(&cf, 0, sizeof cf);
     const mks_invert_arg ra = refine_arg(arg);
-    MKS_TRY(alloc_cg_fields(cf, nb, ra.prec));
+    MKS_TRY(alloc_cg_fields(c.slots[slot], cf, nb, ra.prec));
     double sig[MAXSRC];
     for (int q = 0; q < nb; q++) {
       const int f = fld[b0 + q], j = shf[b0 + q];
@@ -3054,7 +3096,7 @@ static int multishift_dev_once(const double *src_dev, double *const *psim_dev, c
     CgFields f;
     memset(&f, 0, sizeof f);
     const mks_invert_arg ra = refine_arg(arg);
-    MKS_TRY(alloc_cg_fields(f, nb, ra.prec));
+    MKS_TRY(alloc_cg_fields(c.slots[slot], f, nb, ra.prec));
     for (int s = 0; s < nb; s++) {
       f.src[s] = src64;       // read only in the block CG
       f.x[s] = x64[b0 + s];   // the sloppy solve's FP64 solution is the initial guess
@@ -3075,18 +3117,20 @@ static int multishift_dev_once(const double *src_dev, double *const *psim_dev, c
 }
 
 // The multi-shift entry cores, repeated once when the staged D_eo kernel gave
-// up during the call (it is off afterwards; the solutions are outputs only).
+// up during the call (it is off afterwards; the solutions are outputs only),
+// or without the links' integer copies when memory ran out.
 static int multishift_dev(const double *src_dev, double *const *psim_dev, const double *offsets, int nsh, int slot,
                           const mks_invert_arg *arg, mks_invert_result *res) {
-  int rc = multishift_dev_once(src_dev, psim_dev, offsets, nsh, slot, arg, res);
-  if (rc == MKS_ERR_TIMEOUT && take_tma_retry()) rc = multishift_dev_once(src_dev, psim_dev, offsets, nsh, slot, arg, res);
+  auto once = [&] { return multishift_dev_once(src_dev, psim_dev, offsets, nsh, slot, arg, res); };
+  int rc = with_memory(once);
+  if (rc == MKS_ERR_TIMEOUT && take_tma_retry()) rc = with_memory(once);
   return rc;
 }
 static int multishift_multi_dev(int nf, const double *const *src_dev, const int *num_offsets, const double *offsets,
                                 double *const *psim_dev, int slot, const mks_invert_arg *arg, mks_invert_result *res) {
-  int rc = multishift_multi_dev_once(nf, src_dev, num_offsets, offsets, psim_dev, slot, arg, res);
-  if (rc == MKS_ERR_TIMEOUT && take_tma_retry())
-    rc = multishift_multi_dev_once(nf, src_dev, num_offsets, offsets, psim_dev, slot, arg, res);
+  auto once = [&] { return multishift_multi_dev_once(nf, src_dev, num_offsets, offsets, psim_dev, slot, arg, res); };
+  int rc = with_memory(once);
+  if (rc == MKS_ERR_TIMEOUT && take_tma_retry()) rc = with_memory(once);
   return rc;
 }
 
