@@ -101,7 +101,7 @@ bool mem_release() {
     s.fat_fx = s.lng_fx = nullptr;
     s.fx_made = 0;
   }
-  return any;
+  return ws_smear_free() || any;
 }
 
 // ---------------- timing ----------------
@@ -544,7 +544,7 @@ static void free_lattice_fields() {
   c.aux_action = 0;
   dev_free(c.mom);
   c.mom = nullptr;
-  c.fx_off = false;
+  c.fx_off = c.fxm_off = false;
   gauge_free();
   rhmc_free();
 }

@@ -96,14 +96,31 @@ static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__re
   dst.e[(size_t)(par * 4 + mu) * Vh + h] = e;
 }
 
+// Runs `once`, which takes its integer fields from the workspace before it
+// launches anything that changes a result; true when there was no memory for
+// them and the caller is to do without (and is not to ask again on this
+// lattice).  *rc: what `once` returned.
+template <class F> inline bool fxm_refused(const F &once, int *rc) {
+  Context &c = ctx();
+  if (c.fxm_off) return true;
+  {
+    FxBusy busy;
+    *rc = once();
+  }
+  if (*rc != MKS_ERR_NOMEM) return false;
+  c.fxm_off = true;
+  ws_smear_free();
+  return true;
+}
+
 // workspace of `mats` (1 or 4) integer matrices per site under `name`
 inline int ws_fxm(const char *name, int mats, FxMat *f) {
   const size_t Vh = ctx().Vh;
   f->ps = (size_t)mats * 9 * FxMat::sites(Vh);
   f->es = (size_t)mats * Vh;
   f->nd = mats;
-  MKS_TRY(ws(std::string(name) + "_p", 2 * f->ps * sizeof(int4), (void **)&f->p));
-  return ws(std::string(name) + "_e", (size_t)mats * 2 * Vh * sizeof(int), (void **)&f->e);
+  MKS_TRY(ws(std::string("smear_") + name + "_p", 2 * f->ps * sizeof(int4), (void **)&f->p));
+  return ws(std::string("smear_") + name + "_e", (size_t)mats * 2 * Vh * sizeof(int), (void **)&f->e);
 }
 
 // a link field [2][4][9][Vh] as integers in the workspace

@@ -23,6 +23,7 @@
 // so nothing is written by two threads.
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 #include "mks_internal.cuh"
 #include "mks_su3.cuh"
@@ -370,18 +371,18 @@ struct ForceRun {
   }
 
   // Reverse of the staple recursion (load_fatlinks_cpu, ASQ_OPTIMIZED_
-  // FATTENING).  F: MatD or, in FP64, FxMat: there links, Kfat and the staple
-  // fields are integers, K2 leaves its kernel as integers and K1 with its last
-  // contribution (k1o); in FP32 k2 and k1o are the fields K2 and K1 themselves.
+  // FATTENING), nb directions mu a launch.  F: MatD or, in FP64, FxMat: there
+  // links, Kfat and the staple fields are integers, K2 leaves its kernel as
+  // integers and K1 with its last contribution (k1o); with MatD k2 and k1o are
+  // the fields K2 and K1 themselves.
   // KA: the adjoint of U_mu as the staples' start, one_link Kfat at first; KU
   // that of the U_nu.  Two fields where one launch takes all four mu, whose
   // KA_mu and KU_nu would meet.
   template <class F>
-  static int staples_adj(const F &U, const F &K, const F &S1, const F &S2, const F &k2, const F &k1o, const F &none,
+  static int staples_adj(int nb, const F &U, const F &K, const F &S1, const F &S2, const F &k2, const F &k1o, const F &none,
                          MatD<R> Kd, MatD<R> K1, MatD<R> K2, MatD<R> KA, MatD<R> KU, const ForceCoeffs &cf) {
-    constexpr bool fx = sizeof(R) == 8;
+    constexpr bool fx = std::is_same<F, FxMat>::value;
     const MatD<R> off = {nullptr, 0, 0};
-    const int nb = staple_batch(ctx().Vh);
     for (int mu0 = 0; mu0 < 4; mu0 += nb)
       for (int kn = 1; kn < 4; kn++) {
         MKS_TRY(staple_fwd(mu0, nb, kn, U, U, S1));
@@ -419,38 +420,49 @@ struct ForceRun {
     const size_t Vh = ctx().Vh, nl = 8 * 9 * Vh;
     MKS_TRY(axpby(Kfat, KU, cf.one_link - 6.0 * cf.lepage, 1.0, nl));
     if (cf.three_staple == 0.0 && cf.lepage == 0.0 && cf.five_staple == 0.0) return MKS_OK;
-    const int nd = staple_batch(Vh);
-    auto scratch = [&](const char *name, int mats, T2 **p) {
-      return ws(std::string("force_") + (sizeof(R) == 8 ? "64_" : "32_") + name, (size_t)mats * 18 * Vh * sizeof(T2),
-                (void **)p);
-    };
-    T2 *k1, *ka = KU;
-    MKS_TRY(scratch("k1", nd, &k1));
-    if (nd == 4) {
-      MKS_TRY(scratch("ka", 4, &ka));
-      MKS_CUDA(cudaMemsetAsync(ka, 0, nl * sizeof(T2), ctx().stream));
-    }
-    const MatD<R> Kd = mat_dirs(Kfat, Vh), K1 = mat_dirs(k1, Vh, nd), KA = mat_dirs(ka, Vh), KUd = mat_dirs(KU, Vh);
+    int nd = staple_batch(Vh), rc = MKS_OK;
     if constexpr (sizeof(R) == 8) {
-      FxMat L, K, S1, S2, fK1, fK2;
-      const FxMat none = {nullptr, nullptr, 0, 0, 1};
-      MKS_TRY(ws_links_fxm("fxm_links", MKS_K_FORCE, links, &L));
-      MKS_TRY(ws_links_fxm("fxm_kfat", MKS_K_FORCE, Kfat, &K));
-      MKS_TRY(ws_fxm("fxm_s", nd, &S1));
-      MKS_TRY(ws_fxm("fxm_t", nd, &S2));
-      MKS_TRY(ws_fxm("fxm_k1", nd, &fK1));
-      MKS_TRY(ws_fxm("fxm_k2", nd, &fK2));
-      MKS_TRY(staples_adj(L, K, S1, S2, fK2, fK1, none, Kd, K1, MatD<R>{nullptr, 0, 0}, KA, KUd, cf));
-    } else {
-      T2 *s1, *s2, *k2;
-      MKS_TRY(scratch("s1", nd, &s1));
-      MKS_TRY(scratch("s2", nd, &s2));
-      MKS_TRY(scratch("k2", nd, &k2));
-      const MatD<R> K2 = mat_dirs(k2, Vh, nd), none = {nullptr, 0, 0};
-      MKS_TRY(staples_adj(mat_dirs(links, Vh), Kd, mat_dirs(s1, Vh, nd), mat_dirs(s2, Vh, nd), K2, K1, none, Kd, K1,
-                          K2, KA, KUd, cf));
+      if (!fxm_refused([&] { return fat_adj_fx(links, nd, cf, Kfat, KU); }, &rc)) return rc;
     }
-    return ka == KU ? MKS_OK : axpby(ka, KU, 1.0, 1.0, nl);
+    // in precision R: K1, the staples S1 and S2, and K2
+    Adj f;
+    rc = adj_fields(nd, 4, KU, &f);
+    if (rc == MKS_ERR_NOMEM && nd > 1) rc = adj_fields(nd = 1, 4, KU, &f);
+    MKS_TRY(rc);
+    auto field = [&](int k) { return mat_dirs(f.mats + (size_t)k * nd * 18 * Vh, Vh, nd); };
+    const MatD<R> Kd = mat_dirs(Kfat, Vh), K1 = field(0), K2 = field(3), none = {nullptr, 0, 0};
+    MKS_TRY(staples_adj(nd, mat_dirs(links, Vh), Kd, field(1), field(2), K2, K1, none, Kd, K1, K2, mat_dirs(f.ka, Vh),
+                        mat_dirs(KU, Vh), cf));
+    return f.ka == KU ? MKS_OK : axpby(f.ka, KU, 1.0, 1.0, nl);
+  }
+  static int fat_adj_fx(T2 *links, int nd, const ForceCoeffs &cf, T2 *Kfat, T2 *KU) {
+    const size_t Vh = ctx().Vh;
+    FxMat L, K, S1, S2, fK1, fK2;
+    const FxMat none = {nullptr, nullptr, 0, 0, 1};
+    Adj f;
+    MKS_TRY(adj_fields(nd, 1, KU, &f));
+    MKS_TRY(ws_fxm("s", nd, &S1));
+    MKS_TRY(ws_fxm("t", nd, &S2));
+    MKS_TRY(ws_fxm("k1", nd, &fK1));
+    MKS_TRY(ws_fxm("k2", nd, &fK2));
+    MKS_TRY(ws_links_fxm("links", MKS_K_FORCE, links, &L));
+    MKS_TRY(ws_links_fxm("kfat", MKS_K_FORCE, Kfat, &K));
+    MKS_TRY(staples_adj(nd, L, K, S1, S2, fK2, fK1, none, mat_dirs(Kfat, Vh), mat_dirs(f.mats, Vh, nd),
+                        MatD<R>{nullptr, 0, 0}, mat_dirs(f.ka, Vh), mat_dirs(KU, Vh), cf));
+    return f.ka == KU ? MKS_OK : axpby(f.ka, KU, 1.0, 1.0, 8 * 9 * Vh);
+  }
+  // `mats` fields of nd matrices per site in one buffer, and KA: a zeroed field
+  // of its own where a launch takes all four mu
+  struct Adj { T2 *mats, *ka; };
+  static int adj_fields(int nd, int mats, T2 *KU, Adj *f) {
+    const size_t Vh = ctx().Vh, nm = (size_t)mats * nd * 18 * Vh, nl = 8 * 9 * Vh;
+    MKS_TRY(ws("smear_adj", (nm + (nd == 4 ? nl : 0)) * sizeof(T2), (void **)&f->mats));
+    f->ka = KU;
+    if (nd == 4) {
+      f->ka = f->mats + nm;
+      MKS_CUDA(cudaMemsetAsync(f->ka, 0, nl * sizeof(T2), ctx().stream));
+    }
+    return MKS_OK;
   }
 
   static int naik_adj(const T2 *W, const T2 *Kl, T2 *KW, double cn) {
@@ -594,6 +606,7 @@ struct ForceRun {
     } while (0);
     dev_free(nfilt);
     dev_free(buf);
+    ws_smear_done();
     return rc;
   }
 
@@ -632,6 +645,7 @@ struct ForceRun {
       rc = finish(eps, KU, mom_dev, ku_out, nullptr);
     } while (0);
     dev_free(buf);
+    ws_smear_done();
     return rc;
   }
 };

@@ -838,18 +838,18 @@ static void thin_changed() {
 
 static dim3 link_grid() { return dim3(grid_for(ctx().Vh, 128), 2, 4); }
 
-// the thin links as integers, in the link construction's workspace; false
-// when there is no memory for them (the FP64 kernels need none)
-static bool thin_fxm(FxMat *f) {
-  Context &c = ctx();
-  return ws_links_fxm("fxm_links", MKS_K_GAUGE, c.auxU, f) >= 0;
-}
-
 int gauge_force_dev(double eps, double beta, double u0, int nflavors, int prec) {
   Context &c = ctx();
   MKS_TRY(upload_paths(nflavors, u0));
+  // the thin links as integers, in the link construction's workspace (the FP64
+  // kernel needs no memory)
   FxMat Ux;
-  const bool fx = prec == MKS_PREC_DOUBLE && thin_fxm(&Ux);
+  bool fx = false;
+  if (prec == MKS_PREC_DOUBLE) {
+    int rc = MKS_OK;
+    fx = !fxm_refused([&] { return ws_links_fxm("links", MKS_K_GAUGE, c.auxU, &Ux); }, &rc);
+    MKS_TRY(rc == MKS_ERR_NOMEM ? MKS_OK : rc);
+  }
   timing_begin(MKS_K_GAUGE);
   if (prec == MKS_PREC_DOUBLE) {
     if (fx)
@@ -869,6 +869,7 @@ int gauge_force_dev(double eps, double beta, double u0, int nflavors, int prec) 
   }
   timing_end(MKS_K_GAUGE);
   MKS_CUDA(cudaGetLastError());
+  ws_smear_done();
   return MKS_OK;
 }
 
@@ -877,9 +878,15 @@ int gauge_action_dev(double beta, double u0, int nflavors, double *action) {
   MKS_TRY(upload_paths(nflavors, u0));
   double tot[2];
   const OpGaugeAction f64 = {c.geom, c.auxU};
-  FxMat Ux;
-  if (thin_fxm(&Ux)) MKS_TRY((site_sum<OpGaugeActionFx, 1>(OpGaugeActionFx{f64, Ux}, 2, tot)));
-  else MKS_TRY((site_sum<OpGaugeAction, 1>(f64, 2, tot)));
+  int rc = MKS_OK;
+  if (fxm_refused([&] {
+        FxMat Ux;
+        MKS_TRY(ws_links_fxm("links", MKS_K_GAUGE, c.auxU, &Ux));
+        return site_sum<OpGaugeActionFx, 1>(OpGaugeActionFx{f64, Ux}, 2, tot);
+      }, &rc))
+    rc = site_sum<OpGaugeAction, 1>(f64, 2, tot);
+  ws_smear_done();
+  MKS_TRY(rc);
   *action = beta / 3.0 * (tot[0] + tot[1]);
   return MKS_OK;
 }

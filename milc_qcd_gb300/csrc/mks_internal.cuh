@@ -388,10 +388,11 @@ struct Context {
   // integration), and the one the current fermion links were built with
   int md_prec = MKS_PREC_DOUBLE;
   int links_prec = MKS_PREC_DOUBLE;
-  // integer copies of links: calls in progress that use them, and whether
-  // they had to be given back on this lattice (none are made any more)
+  // integer copies of links: calls in progress that use them, and whether the
+  // slots' had to be given back on this lattice, or the smearing's could not be
+  // had (none are made any more)
   int fx_busy = 0;
-  bool fx_off = false;
+  bool fx_off = false, fxm_off = false;
   // timing
   bool timing = false;
   double kernel_ms[MKS_K_COUNT] = {0};
@@ -425,9 +426,9 @@ int timing_flush();
 
 // Device memory.  An allocation that fails is tried again after mem_release,
 // which gives back what the library holds for speed alone (the links' integer
-// copies); it does nothing while a call that uses them is in progress
-// (FxBusy): such a call ends with MKS_ERR_NOMEM and is repeated without them
-// (with_memory).
+// copies, and scratch kept for the next call); it does nothing while a call
+// that uses them is in progress (FxBusy): such a call ends with MKS_ERR_NOMEM
+// and is repeated without them (with_memory).
 int dev_alloc(void **p, size_t bytes);
 void dev_free(void *p);
 bool mem_release();
@@ -453,6 +454,14 @@ template <class F> inline int with_memory(const F &once) {
 // named workspace buffers kept across calls, until the lattice changes (mks_solvers.cu)
 int ws(const std::string &name, size_t bytes, void **out);
 void ws_free_all();
+// Scratch of the smearing, its reverse and the gauge paths: workspace buffers
+// named "smear_*", which need not outlive a call.  They are kept up to 2^20
+// sites of a parity (9.4 kB per site at most), where an allocation takes a
+// good part of a call; ws_smear_done ends a call.
+bool ws_smear_free();
+inline void ws_smear_done() {
+  if (ctx().Vh > ((size_t)1 << 20)) ws_smear_free();
+}
 
 // reduction scratch sized for `nsum` sums and `blocks` blocks
 int ensure_red(int nsum);

@@ -172,10 +172,10 @@ struct Smear {
     return MKS_OK;
   }
   // load_fatlinks_cpu, ASQ_OPTIMIZED_FATTENING (fermion_links_fn_load_milc.c:
-  // 207-253): nu, rho, sigma = mu + 1, 2, 3 in every order.  F: MatD or FxMat
+  // 207-253): nu, rho, sigma = mu + 1, 2, 3 in every order, nb directions mu a
+  // launch.  F: MatD or FxMat
   template <class F>
-  static int staples(const F &U, const F &S, const F &T, const F &none, const FatCoeffs &cf, MatD<R> fat) {
-    const int nb = staple_batch(ctx().Vh);
+  static int staples(int nb, const F &U, const F &S, const F &T, const F &none, const FatCoeffs &cf, MatD<R> fat) {
     for (int mu0 = 0; mu0 < 4; mu0 += nb)
       for (int kn = 1; kn < 4; kn++) {
         MKS_TRY(staple(mu0, nb, kn, U, U, fat, cf.three_staple, S));
@@ -198,22 +198,27 @@ struct Smear {
     timing_end(MKS_K_LINKS);
     MKS_CUDA(cudaGetLastError());
     if (cf.three_staple == 0.0 && cf.lepage == 0.0 && cf.five_staple == 0.0) return MKS_OK;
-    const int nd = staple_batch(Vh);
+    int nd = staple_batch(Vh), rc = MKS_OK;
     if constexpr (sizeof(R) == 8) {
-      FxMat L, S, T;
-      const FxMat none = {nullptr, nullptr, 0, 0, 1};
-      MKS_TRY(ws_links_fxm("fxm_links", MKS_K_LINKS, links, &L));
-      MKS_TRY(ws_fxm("fxm_s", nd, &S));
-      MKS_TRY(ws_fxm("fxm_t", nd, &T));
-      return staples(L, S, T, none, cf, mat_dirs(fat, Vh));
-    } else {
-      T2 *st[2];
-      for (int k = 0; k < 2; k++)
-        MKS_TRY(ws("staple" + std::to_string(k), (size_t)nd * 18 * Vh * sizeof(T2), (void **)&st[k]));
-      const MatD<R> none = {nullptr, 0, 0};
-      return staples(mat_dirs(links, Vh), mat_dirs(st[0], Vh, nd), mat_dirs(st[1], Vh, nd), none, cf,
-                     mat_dirs(fat, Vh));
+      if (!fxm_refused([&] { return staples_fx(links, nd, cf, fat); }, &rc)) return rc;
     }
+    // in precision R: two matrices per site and direction of a launch
+    T2 *st;
+    auto scratch = [&] { return ws("smear_staples", (size_t)nd * 36 * Vh * sizeof(T2), (void **)&st); };
+    rc = scratch();
+    if (rc == MKS_ERR_NOMEM && nd > 1) { nd = 1; rc = scratch(); }
+    MKS_TRY(rc);
+    const MatD<R> none = {nullptr, 0, 0};
+    return staples(nd, mat_dirs(links, Vh), mat_dirs(st, Vh, nd), mat_dirs(st + (size_t)nd * 18 * Vh, Vh, nd), none, cf,
+                   mat_dirs(fat, Vh));
+  }
+  static int staples_fx(T2 *links, int nd, const FatCoeffs &cf, T2 *fat) {
+    FxMat L, S, T;
+    const FxMat none = {nullptr, nullptr, 0, 0, 1};
+    MKS_TRY(ws_links_fxm("links", MKS_K_LINKS, links, &L));
+    MKS_TRY(ws_fxm("s", nd, &S));
+    MKS_TRY(ws_fxm("t", nd, &T));
+    return staples(nd, L, S, T, none, cf, mat_dirs(fat, ctx().Vh));
   }
 
   static int naik(T2 *W, T2 *lng, double coef) {
@@ -352,6 +357,7 @@ static int build_links(int action, int n_naiks, const double *eps_naik, double u
   cudaStreamSynchronize(c.stream);
   dev_free(nsvd);
   dev_free(scr);
+  ws_smear_done();
   return rc;
 }
 
@@ -463,6 +469,7 @@ int mks_fatlong_links(const double coeffs[6], const double *links, double *fat, 
   if (rc >= 0 && lng) rc = to_host(F, lng, stage);
   cudaStreamSynchronize(c.stream);
   dev_free(stage); dev_free(L); dev_free(F);
+  ws_smear_done();
   return rc;
 }
 
@@ -491,6 +498,7 @@ int mks_hisq_aux_links(const double coeffs1[6], const double *U, double *V, doub
   if (rc >= 0 && W) rc = to_host(c.auxW, W, stage);
   cudaStreamSynchronize(c.stream);
   dev_free(stage); dev_free(nsvd);
+  ws_smear_done();
   return rc;
 }
 

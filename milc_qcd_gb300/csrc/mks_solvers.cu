@@ -56,6 +56,17 @@ void ws_free_all() {
   g_ws.clear();
 }
 
+bool ws_smear_free() {
+  bool any = false;
+  for (auto &kv : g_ws)
+    if (kv.first.compare(0, 6, "smear_") == 0 && kv.second.p) {
+      dev_free(kv.second.p);
+      kv.second = WsBuf();
+      any = true;
+    }
+  return any;
+}
+
 template <typename T> static int wsv(const std::string &name, size_t n, T **out) {
   void *p;
   MKS_TRY(ws(name, n * sizeof(T), &p));

@@ -30,17 +30,34 @@ def solve(n, prec):
     xs = [np.zeros((U.shape[0], 6)) for _ in range(n)]
     m.ks_congrad_block_parity([vec(k, m.EVEN) for k in range(n)], xs, qic(prec), 0.1)
     return xs
-m.load_fn_links(U, U / 24)
+if what in ("hisq", "force", "gauge"):
+    mom = np.zeros((U.shape[0], 4, 10))
+    if what == "hisq":
+        m.load_hisq_links(U, (0.0, -0.1))
+        res += [a for slot in (0, 1) for a in m.get_fn_links(slot)]
+    elif what == "force":
+        for action in ("hisq", "asqtad"):
+            getattr(m, "load_%s_links" % action)(U)
+            mom[:] = 0
+            m.eo_fermion_force_multi(0.1, [1.0, -0.5], [vec(k, m.EVENANDODD) for k in range(2)], mom, action=action)
+            res.append(mom.copy())
+    else:
+        m.gauge_load(U)
+        m.mom_load(mom)
+        m.gauge_force(0.01, 7.4, 0.89, 3)
+        res += [m.mom_get(), np.full_like(mom, m.gauge_action(7.4, 0.89, 3))]
+else:
+    m.load_fn_links(U, U / 24)
 if what == "dslash":
     res.append(np.zeros((U.shape[0], 6)))
     m.dslash_fn_field(vec(1, m.EVENANDODD), res[0], m.EVENANDODD)
-elif what == "multishift":
+if what == "multishift":
     res = [np.zeros((U.shape[0], 6)) for _ in range(4)]
     m.ks_multicg_offset_field(vec(1, m.EVEN), res, [0.04, 0.1, 0.3, 1.0], qic(m.PREC_DOUBLE))
 elif what == "uml":
     res = [np.zeros((U.shape[0], 6))]
     m.mat_invert_uml_field(vec(1, m.EVENANDODD), res[0], qic(m.PREC_SINGLE), 0.1)
-else:
+elif what == "solve":
     res += solve(8, m.PREC_DOUBLE)
     res += solve(8, m.PREC_SINGLE)
 np.save(out, np.stack(res))
@@ -57,10 +74,13 @@ def _run(what, limit, path):
 # the least limits under which the calls passed before there were integer
 # copies (to 16 MiB), and one where the copies fit beside the links but not
 # beside a solve's fields as well.  D: 256 roundings; solutions: residuals of
-# 1e-9 on either side, an operator between 0.04 and 16
+# 1e-9 on either side, an operator between 0.04 and 16; links, force and paths:
+# three levels of 18 roundings, which the projection's derivative multiplies
+# by less than 16
 @pytest.mark.parametrize("what,limits,tol", [
     ("dslash", [416], 256 * 2.0 ** -53), ("multishift", [416, 560], 1e-6), ("uml", [416, 560], 1e-6),
-    ("solve", [576, 640], 1e-6)])
+    ("solve", [576, 640], 1e-6),
+    ("hisq", [992], 1024 * 2.0 ** -53), ("force", [976], 1024 * 2.0 ** -53), ("gauge", [304], 1024 * 2.0 ** -53)])
 def test_limit(gpu, tmp_path, what, limits, tol):
     rc, err, want = _run(what, 0, tmp_path / "a.npy")
     assert rc == 0, err
