@@ -15,7 +15,9 @@
 // bounds these kernels).  The first product of a chain keeps K 2^-64, one add
 // of M's high word; the last K 2^-61.  A matrix of zeros has e = FX_ZERO, one
 // that holds an infinity or a NaN e = FX_SPECIAL and the doubles' bits; a site
-// that meets one is done in plain FP64.
+// that meets one is done in plain FP64.  One exponent per matrix bounds a
+// product's error by its norm, not entry by entry; links with entries far below
+// their largest (FxShape) are left to the FP64 kernels.
 //
 // A staple term is a chain L (M R) of three matrices, its adjoint six chains;
 // the chains run in a loop whose operands are fetched three ahead into shared
@@ -79,8 +81,10 @@ __device__ __forceinline__ void fxm_encode(const double2 (&v)[9], int4 (&u)[9], 
   if (!any) e = FX_ZERO;
 }
 
-// [2][4][9][Vh] doubles -> integers
-static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__restrict__ src, FxMat dst, int Vh) {
+// [2][4][9][Vh] doubles -> integers; *uneven (where given) is set when a matrix
+// has entries that its one exponent does not hold (FxShape)
+static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__restrict__ src, FxMat dst, int Vh,
+                                                            int *uneven) {
   const int h = blockIdx.x * blockDim.x + threadIdx.x, par = blockIdx.y, mu = blockIdx.z;
   if (h >= Vh) return;
   const double2 *s = src + (size_t)(par * 4 + mu) * 9 * Vh + h;
@@ -90,6 +94,12 @@ static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__re
 #pragma unroll
   for (int k = 0; k < 9; k++) v[k] = s[(size_t)k * Vh];
   fxm_encode(v, u, e);
+  if (uneven) {
+    FxShape f;
+#pragma unroll
+    for (int k = 0; k < 9; k++) f.add(v[k]);
+    if (f.uneven()) *uneven = 1;
+  }
   int4 *d = fx_link_dir(dst, mu, Vh).at(par, h);
 #pragma unroll
   for (int k = 0; k < 9; k++) d[32 * k] = u[k];
@@ -97,15 +107,20 @@ static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__re
 }
 
 // Runs `once`, which takes its integer fields from the workspace before it
-// launches anything that changes a result; true when there was no memory for
-// them and the caller is to do without (and is not to ask again on this
-// lattice).  *rc: what `once` returned.
+// launches anything that changes a result; true when the caller is to do
+// without: the links are uneven, or there was no memory (then it is not to ask
+// again on this lattice).  *rc: what `once` returned.
+constexpr int FXM_UNEVEN = 1;
 template <class F> inline bool fxm_refused(const F &once, int *rc) {
   Context &c = ctx();
   if (c.fxm_off) return true;
   {
     FxBusy busy;
     *rc = once();
+  }
+  if (*rc == FXM_UNEVEN) {
+    *rc = MKS_OK;
+    return true;
   }
   if (*rc != MKS_ERR_NOMEM) return false;
   c.fxm_off = true;
@@ -123,15 +138,28 @@ inline int ws_fxm(const char *name, int mats, FxMat *f) {
   return ws(std::string("smear_") + name + "_e", (size_t)mats * 2 * Vh * sizeof(int), (void **)&f->e);
 }
 
-// a link field [2][4][9][Vh] as integers in the workspace
-inline int ws_links_fxm(const char *name, int family, const double2 *links, FxMat *f) {
+// a field of matrices [2][4][9][Vh] as integers in the workspace
+inline int ws_mats_fxm(const char *name, int family, const double2 *mats, FxMat *f, int *uneven = nullptr) {
   Context &c = ctx();
   MKS_TRY(ws_fxm(name, 4, f));
   timing_begin(family);
-  k_links_to_fxm<<<dim3(grid_for(c.Vh, 128), 2, 4), 128, 0, c.stream>>>(links, *f, (int)c.Vh);
+  k_links_to_fxm<<<dim3(grid_for(c.Vh, 128), 2, 4), 128, 0, c.stream>>>(mats, *f, (int)c.Vh, uneven);
   timing_end(family);
   MKS_CUDA(cudaGetLastError());
   return MKS_OK;
+}
+// Links that chains or paths are built of; FXM_UNEVEN when one exponent per
+// matrix does not hold them.  (A field between two links, the outer products
+// of the force, need not be looked at: even links mix its entries.)
+inline int ws_links_fxm(int family, const double2 *links, FxMat *f) {
+  Context &c = ctx();
+  int *flag, uneven = 0;
+  MKS_TRY(ws("fxm_uneven", sizeof(int), (void **)&flag));
+  MKS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), c.stream));
+  MKS_TRY(ws_mats_fxm("links", family, links, f, flag));
+  MKS_CUDA(cudaMemcpyAsync(&uneven, flag, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  MKS_CUDA(cudaStreamSynchronize(c.stream));
+  return uneven ? FXM_UNEVEN : MKS_OK;
 }
 
 // an operand of a chain: a site's matrix, as it is or its adjoint

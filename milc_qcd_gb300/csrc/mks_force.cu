@@ -445,8 +445,9 @@ struct ForceRun {
     MKS_TRY(ws_fxm("t", nd, &S2));
     MKS_TRY(ws_fxm("k1", nd, &fK1));
     MKS_TRY(ws_fxm("k2", nd, &fK2));
-    MKS_TRY(ws_links_fxm("links", MKS_K_FORCE, links, &L));
-    MKS_TRY(ws_links_fxm("kfat", MKS_K_FORCE, Kfat, &K));
+    MKS_TRY(ws_mats_fxm("kfat", MKS_K_FORCE, Kfat, &K));
+    const int rc = ws_links_fxm(MKS_K_FORCE, links, &L);
+    if (rc != MKS_OK) return rc;
     MKS_TRY(staples_adj(nd, L, K, S1, S2, fK2, fK1, none, mat_dirs(Kfat, Vh), mat_dirs(f.mats, Vh, nd),
                         MatD<R>{nullptr, 0, 0}, mat_dirs(f.ka, Vh), mat_dirs(KU, Vh), cf));
     return f.ka == KU ? MKS_OK : axpby(f.ka, KU, 1.0, 1.0, 8 * 9 * Vh);

@@ -20,8 +20,8 @@
 // force and action walk each path link by link (recomputation instead of
 // stored intermediate staple fields): FP32 in floats, FP64 in integer
 // arithmetic on a copy of the links in the workspace, or in plain FP64 when
-// there is no memory for that copy (another 144 bytes per link) or a link is
-// not finite.
+// there is no memory for that copy (another 144 bytes per link), a link is
+// not finite, or a matrix has entries that one exponent does not hold.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -841,13 +841,13 @@ static dim3 link_grid() { return dim3(grid_for(ctx().Vh, 128), 2, 4); }
 int gauge_force_dev(double eps, double beta, double u0, int nflavors, int prec) {
   Context &c = ctx();
   MKS_TRY(upload_paths(nflavors, u0));
-  // the thin links as integers, in the link construction's workspace (the FP64
-  // kernel needs no memory)
+  // the thin links as integers, in the link construction's workspace, unless
+  // that does not hold them (the FP64 kernel needs no memory)
   FxMat Ux;
   bool fx = false;
   if (prec == MKS_PREC_DOUBLE) {
     int rc = MKS_OK;
-    fx = !fxm_refused([&] { return ws_links_fxm("links", MKS_K_GAUGE, c.auxU, &Ux); }, &rc);
+    fx = !fxm_refused([&] { return ws_links_fxm(MKS_K_GAUGE, c.auxU, &Ux); }, &rc);
     MKS_TRY(rc == MKS_ERR_NOMEM ? MKS_OK : rc);
   }
   timing_begin(MKS_K_GAUGE);
@@ -881,7 +881,8 @@ int gauge_action_dev(double beta, double u0, int nflavors, double *action) {
   int rc = MKS_OK;
   if (fxm_refused([&] {
         FxMat Ux;
-        MKS_TRY(ws_links_fxm("links", MKS_K_GAUGE, c.auxU, &Ux));
+        const int uneven = ws_links_fxm(MKS_K_GAUGE, c.auxU, &Ux);
+        if (uneven != MKS_OK) return uneven;
         return site_sum<OpGaugeActionFx, 1>(OpGaugeActionFx{f64, Ux}, 2, tot);
       }, &rc))
     rc = site_sum<OpGaugeAction, 1>(f64, 2, tot);

@@ -215,9 +215,10 @@ struct Smear {
   static int staples_fx(T2 *links, int nd, const FatCoeffs &cf, T2 *fat) {
     FxMat L, S, T;
     const FxMat none = {nullptr, nullptr, 0, 0, 1};
-    MKS_TRY(ws_links_fxm("links", MKS_K_LINKS, links, &L));
     MKS_TRY(ws_fxm("s", nd, &S));
     MKS_TRY(ws_fxm("t", nd, &T));
+    const int rc = ws_links_fxm(MKS_K_LINKS, links, &L);
+    if (rc != MKS_OK) return rc;
     return staples(nd, L, S, T, none, cf, mat_dirs(fat, ctx().Vh));
   }
 
