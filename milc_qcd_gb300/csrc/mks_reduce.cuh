@@ -93,13 +93,18 @@ __device__ __forceinline__ void block_reduce_grouped(T (&v)[NB][NSUM], int G, do
   __syncthreads();
 }
 
-// ---- exact sums over the grid ----
+// ---- sums over the grid ----
 // A sum lives in RED_LIMBS 64-bit integers of global memory: limb k counts
 // units of 2^(32k - 1074), so a double is three signed 32-bit pieces, and
 // blocks add theirs with integer atomics, in any order with the same result
 // (up to 2^31 blocks).  The last limb flags infinities and NaN.  One block
 // that arrives last reads the limbs; rows summed by a tree in two levels of
-// last-to-arrive blocks took 5.3 us more (1296 blocks, three sums).
+// last-to-arrive blocks took 5.3 us more (1296 blocks, three sums).  The limbs
+// hold the sum exactly; what is read is its part down to 2^-63 of the largest
+// block total (limbs are signed, so the highest may cancel), rounded to FP64.
+// Carrying through all limbs first, for the whole of a sum that cancels
+// further, costs every reducing kernel registers (k_site with OpUpdate<float>
+// 32 to 40; 8-source CG on 32^3x64 368.1 to 370.6 ms).
 __device__ __forceinline__ void red_add(unsigned long long *limbs, double x) {
   int f;
   unsigned long long m;
@@ -141,7 +146,8 @@ __device__ __forceinline__ double red_take(unsigned long long *limbs) {
     const long long r = __shfl_sync(0xffffffffu, k >= 64 ? v2 : k >= 32 ? v1 : v0, k & 31);
     w[i] = k >= 0 ? r : 0;
   }
-  // three limbs with the carry of the two below, in units of limb top - 2
+  // three limbs with the carry of the two below, in units of limb top - 2; a
+  // total with a piece in limb `top` is at least 2^64 of them
   const __int128 a = ((((__int128)w[0] << 32) + w[1]) << 32) + w[2] + ((w[3] + (w[4] >> 32)) >> 32);
   const unsigned __int128 u = a < 0 ? -(unsigned __int128)a : (unsigned __int128)a;
   const unsigned long long hi = (unsigned long long)(u >> 64), lo = (unsigned long long)u;
