@@ -905,7 +905,9 @@ static int tune_shape(const LinkT &fat, const LinkT &lng, int nsrc, Shape *best)
 // threads per site, where the lattice admits its tiles.  A trailing ":p"
 // selects the software-pipelined kernel, ":g" the persistent grid, ":a2" or
 // ":a3" the cp.async link buffers (FP32 plain D only).  A leading "d" or "e"
-// limits an entry to the plain D or to the fused-epilogue launches.
+// limits an entry to the plain D or to the fused-epilogue launches.  The FP64
+// D takes its shape by rule (launch_fx): an entry for precision 2 has no
+// effect, which shape_note says once.
 static bool shape_override(int prec, int nsrc, bool epi, Shape *out) {
   const char *e = getenv("MKS_SHAPE");
   if (!e) return false;
@@ -1029,6 +1031,23 @@ static int launch_raw(FxArgs &a, const Fin &fin, int mult, int rows) {
   return MKS_OK;
 }
 
+static void shape_note() {
+  static bool said = false;
+  if (said) return;
+  said = true;
+  const char *e = getenv("MKS_SHAPE");
+  const std::string str = e ? e : "";
+  for (size_t pos = 0; pos < str.size();) {
+    const size_t end = str.find(',', pos) == std::string::npos ? str.size() : str.find(',', pos);
+    const size_t first = str[pos] == 'd' || str[pos] == 'e' ? pos + 1 : pos;
+    if (first + 1 < end && str[first] == '0' + MKS_PREC_DOUBLE && str[first + 1] == ':') {
+      fprintf(stderr, "milc_ks_gb300: MKS_SHAPE entry \"%s\" ignored: the FP64 D takes its shape by rule\n",
+              str.substr(pos, end - pos).c_str());
+    }
+    pos = end + 1;
+  }
+}
+
 // rows = 2: both parities of one source in one launch (in[y], out[y] of
 // output parity y).  One source per thread up to 8 (blocks of one warp per
 // source share their sites' links in L1), two beyond.
@@ -1042,6 +1061,7 @@ static int launch_fx(const LinkSlot &sl, FxArgs &a, const Fin &fin, int rows = 1
   a.lng64 = sl.lng64;
   a.EL = sl.fat_exp;
   a.dE = sl.lng_exp - sl.fat_exp;
+  shape_note();
   const int mult = a.nsrc == 1 ? 4 : a.nsrc == 2 ? 2 : 1;
   if (!sl.fx_made) return launch_raw<OUT, EPI>(a, fin, mult, rows);
   if (a.nsrc <= 8 && c.Vh * a.nsrc * rows < (size_t)c.sm_count * FX_SPLIT_THREADS)
