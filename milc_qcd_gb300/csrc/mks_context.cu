@@ -398,15 +398,16 @@ static void free_slot(LinkSlot &s) {
 }
 
 // Room for the integer copies of a slot's links, 2304 bytes per site of a
-// parity beside the 4032 of its other forms: taken only if an eighth of the
-// memory stays free.  D_eo does without them where there is none.
+// parity beside the 4032 of its other forms: taken only if eight times as much,
+// or an eighth of the memory, stays free for the solves and for other users of
+// the device.  D_eo does without them where there is none.
 static bool alloc_fx(LinkSlot &s) {
-  const size_t bytes = (size_t)8 * 9 * g_ctx.Vh * sizeof(int4);
+  const size_t bytes = (size_t)8 * 9 * g_ctx.Vh * sizeof(int4), both = 2 * bytes;
   if (s.fat_fx && s.lng_fx) return true;
   if (g_ctx.fx_off) return false;
   size_t avail, total;
   mem_info(&avail, &total);
-  if (avail < 2 * bytes + total / 8) return false;
+  if (avail < both + (total / 8 < 8 * both ? total / 8 : 8 * both)) return false;
   if (try_alloc((void **)&s.fat_fx, bytes) == cudaSuccess && try_alloc((void **)&s.lng_fx, bytes) == cudaSuccess)
     return true;
   dev_free(s.fat_fx);
