@@ -273,15 +273,18 @@ __global__ void __launch_bounds__(256, NB == 1 ? 2 : 1) k_dslash_fx(const FxArgs
   dslash_fx_body<SPLIT, false, NB, OUT, EPI, Fin>(a, fin);
 }
 
-// Four threads per site in 102 registers: 20 warps per SM instead of 16, for
+// Four threads per site in 96 registers: 20 warps per SM instead of 16, for
 // launches that 20 hold at once and 16 do not.  On 12^3x24 those left 160 of
 // 2592 warps to a second wave, and the FP64 tail of a warp (24 operations of
 // 64 clocks, 8 when its threads share the colours) is a good part of an
 // epilogue launch: the two D of a multi-shift iteration 55 and 48 us, the
-// FP64 trajectory 143 and 135 ms.  Elsewhere the registers count more
-// (14x10x18x22, 23 warps per SM, D into MILC's layout: 24 and 29 us; 16^3x32,
-// 54 warps per SM: even or slower) and sharing colours costs
-// two exchanges (8^4 CG: 1.43 and 1.49 ms).
+// FP64 trajectory 143 and 135 ms.  On either side it loses: with more warps
+// than 20 the registers count (a whole D call on 14x10x18x22, 23 warps: 34.0
+// and 38.5 us; on 16^3x32, 54 warps: 52.6 and 55.7), and with 16 or fewer
+// sharing colours costs two exchanges (8^4 CG: 1.43 and 1.49 ms).  D into
+// MILC's layout, which has no tail to share, keeps the ordinary kernel; within
+// the window the dense one would take 1.3 to 2 us off a call (12^3x24 30.5 and
+// 29.0 us, 12^3x28 32.4 and 30.4).
 template <int OUT, int EPI, class Fin>
 __global__ void __launch_bounds__(128, 5) k_dslash_fx_dense(const FxArgs a, const Fin fin) {
   dslash_fx_body<4, true, 1, OUT, EPI, Fin>(a, fin);

@@ -5,9 +5,11 @@
 // product of two 57-bit integers built of three such multiply-adds is ten
 // times cheaper than one FP64 fma.  The 3x3 products of D_eo are sums of
 // bounded terms, which a fixed-point sum represents without any rounding of
-// its own: the only errors are the rounding of the operands to a common
-// exponent (2^-57 of the largest component) and the product of the two low
-// halves, which is left out (2^-56 of 2^-56 of the operands' bounds).
+// its own.  Its errors are the links' rounding (2^-57 of the largest of their
+// kind), the vectors' cut to the largest component among a site's 16
+// neighbours (downwards, by up to 2^-56 of it) and the product of the two low
+// halves, which is left out (up to 2^-58 of the operands' bounds): bounds on
+// the norm of a site's terms, not on each component.
 // Measured against a complex128 restatement (which rounds too) on 8^4 ..
 // 32^3x64: 1.8e-16 of the result's norm, where the FP64 sums had 3.8e-16.
 //

@@ -463,7 +463,7 @@ inline void ws_smear_done() {
   if (ctx().Vh > ((size_t)1 << 20)) ws_smear_free();
 }
 
-// reduction scratch sized for `nsum` sums and `blocks` blocks
+// reduction scratch sized for `nsum` sums
 int ensure_red(int nsum);
 
 inline int grid_for(size_t n, int block) { return (int)((n + block - 1) / block); }

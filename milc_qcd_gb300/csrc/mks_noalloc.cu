@@ -9,8 +9,8 @@
 // kernels and the FP64 D_eo with the staging buffers placed in the fixed
 // array below, so it allocates nothing.  It launches the plain one-source
 // D_eo kernel (k_dslash with one source per thread, 256-thread blocks), not
-// the autotuned shape of the allocating entry point: the results agree to
-// rounding, the speed may differ.
+// the integer kernels of the allocating entry point: the results agree to
+// rounding, the speed differs.
 //
 // Limits and sharing: the array holds MKS_NOALLOC_SCRATCH_BYTES (32 MiB),
 // the FP64 input and output staging for lattices of up to 349,525 sites

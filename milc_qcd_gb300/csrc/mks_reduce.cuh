@@ -72,9 +72,7 @@ __device__ __forceinline__ void block_reduce_grouped(T (&v)[NB][NSUM], int G, do
 #pragma unroll
     for (int k = 0; k < NSUM; k++) {
       T x = v[s][k];
-      if (sizeof(T) == 8 && G == 1) x = warp_sum(x);
-      else
-        for (int o = 16; o >= G; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      for (int o = 16; o >= G; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
       v[s][k] = x;
     }
   if (lane < G) {

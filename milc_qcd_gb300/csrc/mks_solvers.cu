@@ -409,8 +409,8 @@ static int launch_site(int family, const Op &op, const Fin &fin, const int *skip
   int Vh = (int)c.Vh;
   int gx = grid_for(Vh, 256);
   // Blocks per SM and source row: about 16 per SM over all rows, 1 to 4 per
-  // row.  Every block ends with a block reduction and a row of partial sums,
-  // so for many sources fewer, longer blocks win (8 sources on 32^3x64: the
+  // row.  Every block ends with a block reduction and its adds to the grid's
+  // sums, so for many sources fewer, longer blocks win (8 sources on 32^3x64: the
   // CG's update and dot kernels 111 ms per solve of 8 with 2 per row, 117
   // with 4, 129 with 8), while one row needs the 4 to fill the chip.
   // MKS_SITE_BLOCKS fixes the count per row.
@@ -997,7 +997,7 @@ static int launch_fx_as(FxArgs &a, const Fin &fin, int mult, int rows) {
   }
   (EPI == EPI_AXPY ? g_shape_epi : g_shape)[MKS_PREC_DOUBLE][a.nsrc] = {a.G * SPLIT, NB, block, 0, 0, 0, 0};
   timing_begin(MKS_K_DSLASH_F64);
-  // warps that the chip holds at once at 20 per SM (102 registers a thread), not at 16
+  // warps that the chip holds at once at 20 per SM (96 registers a thread), not at 16
   const size_t warps = (size_t)grid * rows * (block / 32), sm = c.sm_count;
   bool dense = false;
   if constexpr (SPLIT == 4 && OUT != FX_OUT_AOS) {
@@ -1127,8 +1127,6 @@ static int dslash64(const LinkSlot &sl, int out_par, int nsrc, double2 *const *i
 // ------------------------------------------------------------------
 // per-parity field views inside one contiguous "full" SoA buffer:
 // full field = [2][3][Vh] double2; parity par starts at par*3*Vh
-static inline double2 *par64(double2 *full, int par) { return full + (size_t)par * 3 * ctx().Vh; }
-
 static int parity_index(int parity, int *par) {
   if (parity == MKS_EVEN) *par = 0;
   else if (parity == MKS_ODD) *par = 1;

@@ -40,8 +40,6 @@ __host__ __device__ inline MatT<double> link_dir(double2 *base, int dir, size_t 
 __host__ __device__ inline MatT<float> link_dir(float2 *base, int dir, size_t Vh) {
   return {base + (size_t)dir * 9 * Vh, 36 * Vh};
 }
-__host__ __device__ inline MatT<double> mat_field(double2 *base, size_t Vh) { return {base, 9 * Vh}; }
-__host__ __device__ inline MatT<float> mat_field(float2 *base, size_t Vh) { return {base, 9 * Vh}; }
 
 // a field with one matrix per direction, [par][4][9][Vh], or a scratch field
 // whose one matrix per site every direction uses (ds = 0)
@@ -62,9 +60,12 @@ template <typename T2> inline MatD<typename RealOf<T2>::t> mat_dirs(T2 *p, size_
 // the staples of the four mu do not depend on each other, and with nu, rho and
 // sigma at fixed distances from mu no two of them write to one direction.  One
 // launch for all four on lattices where a launch is short (12x14x10x20 in FP32,
-// links and force: 420 launches and 4.6 ms one by one); beyond a million sites
-// of a parity it gains nothing and its four scratch matrices per site are
-// memory that the largest lattices need.
+// links and force: 420 launches and 4.6 ms one by one).  Its gain falls with
+// the size (kernels of links and force, one direction a launch and four: FP32
+// 24^3x48 27.8 and 25.6 ms, 32^3x64 81.7 and 79.3, 40^3x64 157 and 155; FP64
+// 130 and 125, 393 and 388, 762 and 758), while its four scratch matrices per
+// site are memory that the largest lattices need: the line is at 2^20 sites of
+// a parity (32^3x64).
 inline int staple_batch(size_t Vh) { return Vh <= ((size_t)1 << 20) ? 4 : 1; }
 
 // y = a x + b y, and precision conversions, over n complex numbers
