@@ -270,21 +270,26 @@ __global__ void k_links_soa_to_aos(const double2 *__restrict__ soa, double *__re
 }
 // What the reduced-precision and integer forms need to know of a link field:
 // its largest |component|, the smallest of its matrices that are not zero (by
-// their largest component), and whether one is not finite or uneven
+// their largest component), whether one is not finite, and how many are uneven
 // (mks_fixed.cuh).  All zero before the launch.
 struct LinkStats {
-  unsigned long long max, inv_min, bad, uneven;   // bits of the doubles; inv_min: of the smallest, complemented
+  unsigned long long max, inv_min, bad;   // bits of the doubles; inv_min: of the smallest, complemented
+  FxUneven uneven;
 };
 __global__ void k_links_stats(const double2 *__restrict__ src, int Vh, LinkStats *out) {
   u64 top = 0, low = ~0ull;
   bool bad = false, uneven = false;
+  int ents = 0, parts = 0;
   for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < Vh; h += gridDim.x * blockDim.x) {
     const double2 *s = src + (size_t)blockIdx.y * 9 * Vh + h;   // par*4+dir
-    FxShape f;
+    double2 v[9];
 #pragma unroll
-    for (int k = 0; k < 9; k++) f.add(s[(size_t)k * Vh]);
+    for (int k = 0; k < 9; k++) v[k] = s[(size_t)k * Vh];
+    const FxShape f(v);
     bad = bad || f.bad;
-    uneven = uneven || f.uneven();
+    uneven = uneven || f.uneven;
+    ents += f.ents;
+    parts += f.parts;
     top = f.top > top ? f.top : top;
     low = f.top != 0 && f.top < low ? f.top : low;
   }
@@ -294,12 +299,11 @@ __global__ void k_links_stats(const double2 *__restrict__ src, int Vh, LinkStats
     low = l < low ? l : low;
   }
   bad = __any_sync(0xffffffffu, bad);
-  uneven = __any_sync(0xffffffffu, uneven);
+  fx_uneven_add(&out->uneven, uneven, ents, parts);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(&out->max, top);
     if (top > 0) atomicMax(&out->inv_min, ~low);
     if (bad) atomicMax(&out->bad, 1ull);
-    if (uneven) atomicMax(&out->uneven, 1ull);
   }
 }
 // the FP32, FP16 and, where the slot keeps them, integer forms of a link field
@@ -446,7 +450,7 @@ int links_make_lowprec(LinkSlot &s) {
     memcpy(&top[k], &st[k].max, 8);
     const unsigned long long b = ~st[k].inv_min;
     memcpy(&low[k], &b, 8);
-    if (st[k].bad || st[k].uneven) plain = true;
+    if (st[k].bad || st[k].uneven.any((size_t)8 * Vh)) plain = true;
     if (st[k].bad || !(top[k] > 0)) continue;
     if (ldexp(low[k], FX_SPREAD) < top[k]) plain = true;
     int e = 0;

@@ -156,35 +156,63 @@ constexpr int FX_SPREAD = 4;
 
 // Components of a vector share an exponent, so a component far below the
 // others is as good as a matrix that mixes them makes its part in a result:
-// an entry of size 2^-k leaves 56 - k bits.  A matrix is uneven when it has an
-// entry more than FX_ENTRY bits, or a real or imaginary part more than FX_PART
-// bits, below its largest component: free, diagonal, real or block matrices,
-// which do not mix some components at all.  Fields with an uneven matrix are
-// done in plain FP64.  (Least entry and least part of 262,144 smeared links:
-// 13 and 25 bits below for thin links exp(i 0.3 H), 13 and 29 for random ones,
-// 17.5 and 29 for exp(i 0.05 H); four times the links bring an entry one bit
-// lower, a part two.)
-constexpr int FX_ENTRY = 28, FX_PART = 48;
+// an entry of size 2^-k leaves 56 - k bits.  Links are uneven, and left to
+// FP64, when
+// - a matrix has an entry more than FX_ENTRY bits, or a real or imaginary part
+//   more than FX_PART bits, below its largest component: free, diagonal, real
+//   or block matrices, which do not mix some components at all; or
+// - one entry in 1024 lies more than FX_ENTRIES bits below, or one part more
+//   than FX_PARTS: fields close to such ones, whose typical small entry is
+//   under 2^-7 (a generic field has one such entry in 10^7, one such part in
+//   10^6).
+// Least entry and least part of 262,144 smeared links: 13 and 25 bits below
+// for thin links exp(i 0.3 H), 13 and 29 for random ones, 17.5 and 29 for
+// exp(i 0.05 H); four times the links bring an entry one bit lower, a part two.
+constexpr int FX_ENTRY = 28, FX_PART = 48, FX_ENTRIES = 12, FX_PARTS = 20;
 constexpr u64 FX_INF = 0x7ff0000000000000ull;
 struct FxShape {
-  u64 top, ent, part;   // bits of the largest component, the least entry and the least part
-  bool bad;             // a component is not finite (a NaN does not count as the largest)
-  __device__ __forceinline__ FxShape() : top(0), ent(~0ull), part(~0ull), bad(false) {}
-  __device__ __forceinline__ void add(double2 v) {
-    u64 x = (u64)__double_as_longlong(v.x) & ~(1ull << 63), y = (u64)__double_as_longlong(v.y) & ~(1ull << 63);
-    bad = bad || x >= FX_INF || y >= FX_INF;
-    if (x > FX_INF) x = 0;
-    if (y > FX_INF) y = 0;
-    const u64 e = x > y ? x : y, p = x > y ? y : x;
-    top = e > top ? e : top;
-    ent = e < ent ? e : ent;
-    part = p < part ? p : part;
-  }
-  __device__ __forceinline__ bool uneven() const {
+  u64 top;           // bits of the largest component (a NaN does not count)
+  bool bad, uneven;  // a component is not finite; the first rule
+  int ents, parts;   // entries and parts of the second
+  __device__ __forceinline__ FxShape(const double2 (&v)[9]) : top(0), bad(false), uneven(false), ents(0), parts(0) {
+    int e[9], p[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      u64 x = (u64)__double_as_longlong(v[k].x) & ~(1ull << 63), y = (u64)__double_as_longlong(v[k].y) & ~(1ull << 63);
+      bad = bad || x >= FX_INF || y >= FX_INF;
+      if (x > FX_INF) x = 0;
+      if (y > FX_INF) y = 0;
+      const u64 hi = x > y ? x : y, lo = x > y ? y : x;
+      top = hi > top ? hi : top;
+      e[k] = (int)(hi >> 52);
+      p[k] = (int)(lo >> 52);
+    }
+    if (top == 0) return;
     const int t = (int)(top >> 52);
-    return top != 0 && (t - (int)(ent >> 52) > FX_ENTRY || t - (int)(part >> 52) > FX_PART);
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      uneven = uneven || t - e[k] > FX_ENTRY || t - p[k] > FX_PART;
+      ents += t - e[k] > FX_ENTRIES;
+      parts += t - p[k] > FX_PARTS;
+    }
   }
 };
+// counts of a field's matrices, in global memory and zero at first
+struct FxUneven {
+  unsigned long long uneven, ents, parts;
+  // over `mats` matrices
+  bool any(size_t mats) const { return uneven || 1024 * ents > 9 * mats || 1024 * parts > 9 * mats; }
+};
+// adds a warp's counts (all 32 lanes call)
+__device__ __forceinline__ void fx_uneven_add(FxUneven *u, bool uneven, int ents, int parts) {
+  uneven = __any_sync(0xffffffffu, uneven);
+  ents = __reduce_add_sync(0xffffffffu, ents);
+  parts = __reduce_add_sync(0xffffffffu, parts);
+  if ((threadIdx.x & 31) != 0) return;
+  if (uneven) atomicMax(&u->uneven, 1ull);
+  if (ents) atomicAdd(&u->ents, (unsigned long long)ents);
+  if (parts) atomicAdd(&u->parts, (unsigned long long)parts);
+}
 struct FxLinks {
   const int4 *p;  // [par][dir][9][Vh]
 };

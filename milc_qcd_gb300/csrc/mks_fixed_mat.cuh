@@ -17,7 +17,7 @@
 // that holds an infinity or a NaN e = FX_SPECIAL and the doubles' bits; a site
 // that meets one is done in plain FP64.  One exponent per matrix bounds a
 // product's error by its norm, not entry by entry; links with entries far below
-// their largest (FxShape) are left to the FP64 kernels.
+// their largest (FxUneven) are left to the FP64 kernels.
 //
 // A staple term is a chain L (M R) of three matrices, its adjoint six chains;
 // the chains run in a loop whose operands are fetched three ahead into shared
@@ -81,12 +81,12 @@ __device__ __forceinline__ void fxm_encode(const double2 (&v)[9], int4 (&u)[9], 
   if (!any) e = FX_ZERO;
 }
 
-// [2][4][9][Vh] doubles -> integers; *uneven (where given) is set when a matrix
-// has entries that its one exponent does not hold (FxShape)
+// [2][4][9][Vh] doubles -> integers; *uneven (where given) counts the matrices
+// with entries that one exponent does not hold
 static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__restrict__ src, FxMat dst, int Vh,
-                                                            int *uneven) {
-  const int h = blockIdx.x * blockDim.x + threadIdx.x, par = blockIdx.y, mu = blockIdx.z;
-  if (h >= Vh) return;
+                                                            FxUneven *uneven) {
+  const int h0 = blockIdx.x * blockDim.x + threadIdx.x, par = blockIdx.y, mu = blockIdx.z;
+  const int h = h0 < Vh ? h0 : Vh - 1;   // threads past the last site follow it into the warp's counts
   const double2 *s = src + (size_t)(par * 4 + mu) * 9 * Vh + h;
   double2 v[9];
   int4 u[9];
@@ -95,11 +95,10 @@ static __global__ void __launch_bounds__(128) k_links_to_fxm(const double2 *__re
   for (int k = 0; k < 9; k++) v[k] = s[(size_t)k * Vh];
   fxm_encode(v, u, e);
   if (uneven) {
-    FxShape f;
-#pragma unroll
-    for (int k = 0; k < 9; k++) f.add(v[k]);
-    if (f.uneven()) *uneven = 1;
+    const FxShape f(v);
+    fx_uneven_add(uneven, f.uneven, h0 < Vh ? f.ents : 0, h0 < Vh ? f.parts : 0);
   }
+  if (h0 >= Vh) return;
   int4 *d = fx_link_dir(dst, mu, Vh).at(par, h);
 #pragma unroll
   for (int k = 0; k < 9; k++) d[32 * k] = u[k];
@@ -139,7 +138,7 @@ inline int ws_fxm(const char *name, int mats, FxMat *f) {
 }
 
 // a field of matrices [2][4][9][Vh] as integers in the workspace
-inline int ws_mats_fxm(const char *name, int family, const double2 *mats, FxMat *f, int *uneven = nullptr) {
+inline int ws_mats_fxm(const char *name, int family, const double2 *mats, FxMat *f, FxUneven *uneven = nullptr) {
   Context &c = ctx();
   MKS_TRY(ws_fxm(name, 4, f));
   timing_begin(family);
@@ -153,13 +152,13 @@ inline int ws_mats_fxm(const char *name, int family, const double2 *mats, FxMat 
 // of the force, need not be looked at: even links mix its entries.)
 inline int ws_links_fxm(int family, const double2 *links, FxMat *f) {
   Context &c = ctx();
-  int *flag, uneven = 0;
-  MKS_TRY(ws("fxm_uneven", sizeof(int), (void **)&flag));
-  MKS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), c.stream));
-  MKS_TRY(ws_mats_fxm("links", family, links, f, flag));
-  MKS_CUDA(cudaMemcpyAsync(&uneven, flag, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  FxUneven *count, n;
+  MKS_TRY(ws("fxm_uneven", sizeof n, (void **)&count));
+  MKS_CUDA(cudaMemsetAsync(count, 0, sizeof n, c.stream));
+  MKS_TRY(ws_mats_fxm("links", family, links, f, count));
+  MKS_CUDA(cudaMemcpyAsync(&n, count, sizeof n, cudaMemcpyDeviceToHost, c.stream));
   MKS_CUDA(cudaStreamSynchronize(c.stream));
-  return uneven ? FXM_UNEVEN : MKS_OK;
+  return n.any((size_t)8 * c.Vh) ? FXM_UNEVEN : MKS_OK;
 }
 
 // an operand of a chain: a site's matrix, as it is or its adjoint
